@@ -956,9 +956,9 @@ WaveArgs wave_args(cfdg_grid* G, const Scalars* S) {
   A.tiles_j = G->tiles_j;
   A.tiles_k = G->tiles_k;
   A.flags = G->d_flags;
-  A.uniform = G->uniform ? 1 : 0;
   A.fw = G->d_fw;
   A.sync = G->wave_sync;
+  A.halo = G->wave_halo;
   A.error = G->wave_err;
   A.S = S;
   A.spin_limit = G->wave_spin_limit;
@@ -966,11 +966,53 @@ WaveArgs wave_args(cfdg_grid* G, const Scalars* S) {
   return A;
 }
 
-template <int MODE>
-void launch_wave(cfdg_grid* G, const WaveArgs& A) {
-  cudaMemsetAsync(G->wave_sync, 0, sizeof(int) * (2 + G->tiles_j * G->tiles_k), G->stream);
-  k_wave<MODE><<<G->tiles_j * G->tiles_k, WTJ * WTK, 0, G->stream>>>(A);
+// Tiles of a sweep that may share an SM: as few as keep all of them resident. Left to itself
+// the hardware puts six tiles on one SM while most SMs stay empty (measured: 32 tiles on
+// about five SMs), and the tiles then queue for the FP64 pipe, of which each SM sub-core does
+// one warp operation in 64 cycles. The launch asks for the dynamic shared memory that leaves
+// room for no more (the IC(0) application of 64x64x32: 414 us packed, 371 us spread).
+template <int MODE, bool UNIFORM, bool EXTRA>
+void launch_wave_spread(cfdg_grid* G, const WaveArgs& A) {
+  struct Limits {
+    std::once_flag once;
+    int sms = 1, smem_sm = 0, reserved = 0, fixed = 0, most = 0;
+  };
+  static Limits by_device[64];  // the attribute below holds for one device's context
+  const int dev = G->ctx->device;
+  Limits& L = by_device[dev & 63];
+  std::call_once(L.once, [&L, dev] {
+    cudaDeviceGetAttribute(&L.sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaDeviceGetAttribute(&L.smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
+    cudaDeviceGetAttribute(&L.reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev);
+    int optin = 0;
+    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    cudaFuncAttributes fa{};
+    if (cudaFuncGetAttributes(&fa, k_wave<MODE, UNIFORM, EXTRA>) != cudaSuccess) cudaGetLastError();
+    L.fixed = (int)fa.sharedSizeBytes;
+    L.most = std::max(0, optin - L.fixed);
+    if (cudaFuncSetAttribute(k_wave<MODE, UNIFORM, EXTRA>, cudaFuncAttributeMaxDynamicSharedMemorySize, L.most) !=
+        cudaSuccess) {
+      cudaGetLastError();
+      L.most = 0;
+    }
+  });
+  const int tiles = G->tiles_j * G->tiles_k;
+  const int per = (tiles + L.sms - 1) / L.sms;  // tiles per SM
+  // Just more than the share that per + 1 tiles would have: room for `per`, not for one more.
+  const int want = L.smem_sm / (per + 1) - L.reserved - L.fixed + 1024;
+  const int dyn = std::max(0, std::min(want, std::min(L.most, L.smem_sm / per - L.reserved - L.fixed)));
+  k_wave<MODE, UNIFORM, EXTRA><<<tiles, WTHREADS, dyn, G->stream>>>(A);
   tick(G);
+}
+
+template <int MODE>
+void launch_wave(cfdg_grid* G, const WaveArgs& A, bool extra) {
+  // The weights only serve the Gauss-Seidel sweeps; about half of an IC(0) factor's diagonal
+  // needs the division's extra correction.
+  if constexpr (MODE == IC0_FWD || MODE == IC0_BWD) launch_wave_spread<MODE, true, true>(G, A);
+  else if (!G->uniform) launch_wave_spread<MODE, false, true>(G, A);
+  else if (extra) launch_wave_spread<MODE, true, true>(G, A);
+  else launch_wave_spread<MODE, true, false>(G, A);
 }
 
 void launch_sweep_ic0(cfdg_grid* G, const Scalars* S) {
@@ -978,13 +1020,14 @@ void launch_sweep_ic0(cfdg_grid* G, const Scalars* S) {
   if (G->structured) {
     WaveArgs A = wave_args(G, S);
     A.diag = F.diag;
+    A.rdiag = F.rdiag;
     A.lx = F.lx;
     A.ly = F.ly;
     A.lz = F.lz;
     A.in = G->r;
     A.x = G->z;
-    launch_wave<IC0_FWD>(G, A);
-    launch_wave<IC0_BWD>(G, A);
+    launch_wave<IC0_FWD>(G, A, true);
+    launch_wave<IC0_BWD>(G, A, true);
     return;
   }
   for (size_t l = 0; l + 1 < F.fwd.start.size(); ++l) {
@@ -1003,10 +1046,11 @@ void launch_gs(cfdg_grid* G, DevLevel& L, bool backward, const Scalars* S, bool 
   if (full) {
     WaveArgs A = wave_args(G, S);
     A.diag = L.diag;
+    A.rdiag = L.rdiag;
     A.in = L.rhs;
     A.x = L.x;
-    if (backward) launch_wave<GS_BWD>(G, A);
-    else launch_wave<GS_FWD>(G, A);
+    if (backward) launch_wave<GS_BWD>(G, A, L.rd_extra);
+    else launch_wave<GS_FWD>(G, A, L.rd_extra);
     return;
   }
   const DevSchedule& sc = backward ? L.bwd : L.fwd;
@@ -1209,14 +1253,15 @@ int build_ic0_dev(cfdg_grid* G) {
   auto D = std::make_unique<DevIc0>();
   D->arena.ctx = G->ctx;
   cudaStream_t s = G->stream;
-  if (int e = upload_csr(D->arena, F.lower, D->lower, s)) return e;
-  if (int e = upload_csr(D->arena, F.upper, D->upper, s)) return e;
   if (int e = D->arena.upload(&D->diag, F.diag, s)) return e;
-  if (int e = D->arena.upload(&D->fwd.order, F.fwd.order, s)) return e;
-  if (int e = D->arena.upload(&D->bwd.order, F.bwd.order, s)) return e;
-  D->fwd.start = F.fwd.start;
-  D->bwd.start = F.bwd.start;
-  if (G->structured) {
+  if (!G->structured) {
+    if (int e = upload_csr(D->arena, F.lower, D->lower, s)) return e;
+    if (int e = upload_csr(D->arena, F.upper, D->upper, s)) return e;
+    if (int e = D->arena.upload(&D->fwd.order, F.fwd.order, s)) return e;
+    if (int e = D->arena.upload(&D->bwd.order, F.bwd.order, s)) return e;
+    D->fwd.start = F.fwd.start;
+    D->bwd.start = F.bwd.start;
+  } else {
     // Each row's lower entries are its (k-1), (j-1), (i-1) neighbours (non-periodic 7-point).
     const int64_t N = G->h.cells, nx = G->h.n[0], nxy = (int64_t)G->h.n[0] * G->h.n[1];
     std::vector<double> lx(N, 0.0), ly(N, 0.0), lz(N, 0.0);
@@ -1231,6 +1276,9 @@ int build_ic0_dev(cfdg_grid* G) {
     if (int e = D->arena.upload(&D->lx, lx, s)) return e;
     if (int e = D->arena.upload(&D->ly, ly, s)) return e;
     if (int e = D->arena.upload(&D->lz, lz, s)) return e;
+    if (int e = D->arena.alloc(&D->rdiag, N)) return e;
+    k_recip<<<grid_blocks(N), BLOCK, 0, s>>>(D->diag, D->rdiag, N, G->wave_err + 1); tick(G);
+    CU(cudaGetLastError());
   }
   CU(cudaStreamSynchronize(s));
   G->ic0 = std::move(D);
@@ -1361,6 +1409,15 @@ int build_mg_dev(cfdg_grid* G, const Poller& poll) {
     L.n = M.n;
     if (int e = upload_csr(D->arena, M.a, L.a, s)) return e;
     if (int e = D->arena.upload(&L.diag, M.diag, s)) return e;
+    if (l == 0 && D->full0) {
+      if (int e = D->arena.alloc(&L.rdiag, L.n)) return e;
+      CU(cudaMemsetAsync(G->wave_err + 1, 0, sizeof(int), s));
+      k_recip<<<grid_blocks(L.n), BLOCK, 0, s>>>(L.diag, L.rdiag, L.n, G->wave_err + 1); tick(G);
+      int extra = 1;
+      CU(cudaMemcpyAsync(&extra, G->wave_err + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
+      CU(cudaStreamSynchronize(s));
+      L.rd_extra = extra != 0;
+    }
     if (int e = D->arena.upload(&L.fwd.order, M.fwd.order, s)) return e;
     if (int e = D->arena.upload(&L.bwd.order, M.bwd.order, s)) return e;
     L.fwd.start = M.fwd.start;
@@ -1535,8 +1592,21 @@ int prepare_mg_impl(cfdg_grid* G, const Poller& poll, cfdg_info* info) {
   return 0;
 }
 
+// The hand-off entries of the wavefront sweeps (no epoch is 0, so zeroed entries are unset).
+int ensure_wave(cfdg_grid* G) {
+  if (!G->structured || G->wave_halo) return 0;
+  const size_t n = (size_t)G->tiles_j * G->tiles_k * G->h.n[0] * WHALO;
+  ulonglong2* p = nullptr;
+  if (int e = G->arena.alloc(&p, n)) return e;
+  CU(cudaMemsetAsync(p, 0, n * sizeof(ulonglong2), G->stream));
+  CU(cudaStreamSynchronize(G->stream));
+  G->wave_halo = p;
+  return 0;
+}
+
 // pressure.rs:55-97: the cached factor, or the hierarchy checked against its signature.
 int prepare_preconditioner(cfdg_grid* G, const Poller& poll, cfdg_info* info) {
+  if (int e = ensure_wave(G)) return e;
   if (G->preconditioner == CFDG_PRECOND_MULTIGRID) return prepare_mg_impl(G, poll, info);
   if (!G->ic0) {
     reset_chunk(G);
@@ -2520,7 +2590,8 @@ int cfdg_grid_open(cfdg_context* ctx, const cfdg_grid_desc* d, cfdg_grid** out) 
   G->structured = !h.periodic[0] && !h.periodic[1] && !h.periodic[2] && h.n[0] >= 2 && h.n[1] >= 2 && h.n[2] >= 2;
   G->tiles_j = (h.n[1] + WTJ - 1) / WTJ;
   G->tiles_k = (h.n[2] + WTK - 1) / WTK;
-  if ((e = A.alloc(&G->wave_sync, 2 + (size_t)G->tiles_j * G->tiles_k)) || (e = A.alloc(&G->wave_err, 1))) return e;
+  if ((e = A.alloc(&G->wave_sync, 2)) || (e = A.alloc(&G->wave_err, 2))) return e;
+  CU(cudaMemsetAsync(G->wave_sync, 0, 2 * sizeof(unsigned long long), s));
   CU(cudaMemsetAsync(G->wave_err, 0, sizeof(int), s));
   if ((e = refresh_weights(G.get()))) return e;
   CU(cudaStreamSynchronize(s));

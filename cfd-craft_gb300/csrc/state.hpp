@@ -111,7 +111,9 @@ struct DevIc0 {
   ~DevIc0() { arena.release(); }
   DevCsr lower, upper;
   double* diag = nullptr;
-  double *lx = nullptr, *ly = nullptr, *lz = nullptr;  // structured grids: per-cell lower coefficients
+  // Structured grids: the reciprocal diagonal (wave.cuh recip_of) and per-cell lower
+  // coefficients; other grids: the factor's rows and columns above.
+  double *rdiag = nullptr, *lx = nullptr, *ly = nullptr, *lz = nullptr;
   DevSchedule fwd, bwd;
 };
 
@@ -119,6 +121,10 @@ struct DevLevel {
   int n = 0;
   DevCsr a;
   double* diag = nullptr;
+  // Level 0 in full-grid layout: reciprocals of diag (wave.cuh recip_of), and whether some
+  // of them need the division's extra correction.
+  double* rdiag = nullptr;
+  bool rd_extra = true;
   DevSchedule fwd, bwd;
   DevCsr groups, prolong, restrict_;
   int ngroups = 0;
@@ -194,8 +200,11 @@ struct cfdg_grid {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   bool structured = false;  // no periodic axis: pipelined wavefront sweeps on the fine level
   int tiles_j = 0, tiles_k = 0;
-  int* wave_sync = nullptr;  // ticket, abort, per-tile progress of one sweep
-  int* wave_err = nullptr;   // set when a wavefront wait gave up
+  // Wavefront sweeps (wave.cuh): tickets taken and the last epoch that gave up; the boundary
+  // values handed from tile to tile, allocated by the first plain preconditioner.
+  unsigned long long* wave_sync = nullptr;
+  ulonglong2* wave_halo = nullptr;
+  int* wave_err = nullptr;   // [0] set when a wavefront wait gave up, [1] scratch of k_recip
   long long wave_spin_limit = WAVE_SPIN_LIMIT;  // cfdg_debug_wave_stall
   int wave_hold_tile = -1;
   std::shared_ptr<cfdg::Hierarchy> host_mg;  // the hierarchy as uploaded (level 0 re-indexed when full0)

@@ -3,16 +3,31 @@
 // A lexicographic sweep over the 7-point pattern in natural cell order (IC(0)
 // forward/backward substitution, pressure.rs:225-240; Gauss-Seidel,
 // multigrid.rs:272-281 / masked.rs:158-172) updates cell (i,j,k) after (i-1,j,k),
-// (i,j-1,k) and (i,j,k-1). Each CTA owns a TJ x TK tile of x-pencils; thread (tj,tk)
-// walks its pencil and handles cell i at local step s = i + tj + tk, so the cells of
-// one step lie on a hyperplane of the tile. Values of the previous step come from
-// shared memory (one barrier per step), the pencil's own predecessor from a register.
-// Tiles depend on their (J-1,K) and (J,K-1) neighbours only through the boundary
-// pencils: a tile publishes how many steps it has completed (release store, one step
-// behind so that a single barrier per step orders it after the steps' stores) and a
-// consumer at step s waits for s + TJ (resp. s + TK) of its producer (acquire load,
-// bounded spin). Tiles are taken in a topological order from an atomic ticket, so a
-// CTA only ever waits for tiles already held by running CTAs.
+// (i,j-1,k) and (i,j,k-1). Each CTA owns a TJ x TK tile of x-pencils; compute thread
+// (tj,tk) walks its pencil and handles cell i at local step s = i + tj + tk, so the cells
+// of one step lie on a hyperplane of the tile. Values of the previous step come from
+// shared memory (one barrier of the two compute warps per step), the pencil's own
+// predecessor from a register. Tiles depend on their (J-1,K) and (J,K-1) neighbours only
+// through the boundary pencils: a boundary thread stores each new value together with the
+// launch's epoch in one 16-byte store, and a receiver warp of the consuming tile polls
+// those entries (four per lane and round trip, bounded) into a shared ring, so the compute
+// threads never wait on global memory but for data not produced yet. Tiles are taken in a
+// topological order from an atomic ticket, so a CTA only ever waits for tiles already held
+// by running CTAs; the ticket counts on from launch to launch and gives the epoch, so
+// nothing is cleared between launches.
+//
+// Bound: the instructions of one warp's step, nx + ny + nz of them in a row plus a hand-off
+// of about a microsecond per tile on the way. A warp's FP64 operation takes 64 cycles on
+// this part (31 ns, measured; independent ones of the same warp do not overlap), so a
+// Gauss-Seidel step's fifteen (six sums, six products, three of the division) cost at least
+// 0.46 us. What else a step does is kept off that chain and free of branches: the operands
+// that do not depend on the sweep (right-hand side, flags, diagonal, the neighbours not
+// updated yet) are loaded WPF steps ahead into registers, absent faces are selected to a
+// neutral zero, and the correctly rounded division by the diagonal uses its precomputed
+// reciprocal (div_pre: three or five operations instead of 272 ns). One Gauss-Seidel sweep
+// of 128x128x64 takes 275 us, of 64x64x32 136 us; with a flag poll, a fence, unprefetched
+// loads, branches and a division per step the former took 1295 us. An IC(0) application
+// (both sweeps) of 64x64x32 takes 242 us (954 us). Tiles of one warp (8 x 4) gave 310 us.
 //
 // Every cell is computed with the same operations in the same order as the
 // reference's natural-order loop, so the result is bit-identical to it. Backward
@@ -22,7 +37,12 @@
 
 namespace cfdg {
 
-constexpr int WTJ = 8, WTK = 8;  // tile of pencils per CTA
+constexpr int WTJ = 8, WTK = 8;       // tile of pencils per CTA
+constexpr int WCT = WTJ * WTK;        // compute threads (two warps)
+constexpr int WTHREADS = WCT + 32;    // and the receiver warp
+constexpr int WRING = 256;            // received values per boundary pencil held in shared memory
+constexpr int WPF = 4;                // steps of operands in flight per compute thread
+constexpr int WHALO = WTJ + WTK;      // boundary pencils of a tile that its consumers read
 
 enum WaveMode { IC0_FWD = 0, IC0_BWD = 1, GS_FWD = 2, GS_BWD = 3 };
 
@@ -33,184 +53,323 @@ struct WaveArgs {
   const double* in;       // r (IC0_FWD) or rhs (GS_*)
   double* x;              // z (IC0_*; IC0_BWD in place) or x (GS_*, in place)
   const double* diag;     // IC(0) factor diagonal, or the level-0 matrix diagonal
+  const double* rdiag;    // its reciprocals as div_pre takes them (k_recip)
   const double* lx;       // IC(0): lower coefficient of each row towards (i-1), (j-1), (k-1)
   const double* ly;
   const double* lz;
   // Gauss-Seidel weights: uniform per axis, or per face.
-  int uniform;
   double w_in[3];
   const double* fw;
   long long face_off[3];
   int fdim[3][3];
-  int* sync;        // [0] ticket, [1] abort, [2 ..] progress per tile
-  int* error;       // persistent: set to 1 when a wait gave up
+  unsigned long long* sync;  // [0] tickets taken so far, [1] epoch of the last launch that gave up
+  ulonglong2* halo;          // [tile][step along x][WHALO]: a boundary value's bits and its epoch
+  int* error;                // persistent: set to 1 when a wait gave up
   const Scalars* S;
   long long spin_limit;  // polls before a wait gives up (WAVE_SPIN_LIMIT)
   int hold_tile;         // -1; a test of the bounded waits names a tile that never publishes
 };
 
-__device__ __forceinline__ int ld_acquire(const int* p) {
-  int v;
-  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+// One 16-byte access each way (PTX b128): the value and its epoch arrive together.
+__device__ __forceinline__ void st_halo(ulonglong2* p, double v, unsigned long long epoch, bool on) {
+  asm volatile(
+      "{\n\t.reg .b128 t;\n\t.reg .pred p;\n\tsetp.ne.u32 p, %3, 0;\n\tmov.b128 t, {%1, %2};\n\t"
+      "@p st.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(p),
+      "l"((unsigned long long)__double_as_longlong(v)), "l"(epoch), "r"((unsigned)on)
+      : "memory");
+}
+__device__ __forceinline__ ulonglong2 ld_halo(const ulonglong2* p) {
+  ulonglong2 v;
+  asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
+               : "=l"(v.x), "=l"(v.y)
+               : "l"(p)
+               : "memory");
   return v;
 }
-__device__ __forceinline__ void st_release(int* p, int v) {
-  asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+__device__ __forceinline__ unsigned long long ld_relaxed(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(WTJ* WTK) k_wave(WaveArgs A) {
+// The division by a known divisor. rd is recip_of(d): r = RN(1/d), negative where the first
+// quotient below may be more than one ulp off, 0 where d lies outside [2^-60, 2^60].
+__device__ __forceinline__ double recip_of(double d) {
+  if (!(d >= 0x1p-60 && d <= 0x1p60)) return 0.0;
+  const double r = __drcp_rn(d);
+  return fabs(__fma_rn(r, d, -1.0)) <= 0x1p-54 ? r : -r;
+}
+__device__ __noinline__ double div_rare(double v, double d) { return __ddiv_rn(v, d); }
+
+// v / d, correctly rounded, by Markstein's correction step (P. Markstein, IBM J. Res. Dev.
+// 34(1), 1990): from r = RN(1/d) and q within one ulp of v/d, the remainder v - q d is
+// exact under one FMA and RN(q + rem r) is RN(v/d). q = RN(v r) is within one ulp when
+// |r d - 1| <= 2^-54: with significands v, d in [1, 2) its error is at most v |r - 1/d|
+// plus half an ulp of q, v |r - 1/d| <= 2^-54 v/d, and v/d < 1 halves the ulp, so both
+// cases stay within one ulp. Otherwise (rd < 0) one more correction first makes it so.
+// Zeros, subnormals, NaN, infinities and v outside [2^-900, 2^900] (where a product or
+// remainder could leave the normal range) take the division. The tests are on the bits: a
+// comparison of doubles would queue for the FP64 pipe. on: whether the result is used;
+// EXTRA: whether some rd is negative (a warp's FP64 operations take 64 cycles each, also
+// where no lane needs them).
+template <bool EXTRA>
+__device__ __forceinline__ double div_pre(double v, double d, double rd, bool on) {
+  const int hi = __double2hiint(rd);
+  const double r = fabs(rd);
+  double q = __dmul_rn(v, r);
+  double rem = __fma_rn(-q, d, v);
+  q = __fma_rn(rem, r, q);
+  if (EXTRA && hi < 0) {
+    rem = __fma_rn(-q, d, v);
+    q = __fma_rn(rem, r, q);
+  }
+  const unsigned e = ((unsigned)__double2hiint(v) >> 20) & 0x7ffu;
+  if (on && (e - 123u > 1800u || hi == 0)) q = div_rare(v, d);
+  return q;
+}
+
+// rd = recip_of(d) for n divisors; *extra is set when one of them is negative.
+__global__ void k_recip(const double* __restrict__ d, double* __restrict__ rd, long long n, int* extra) {
+  bool neg = false;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    const double r = recip_of(d[i]);
+    rd[i] = r;
+    neg |= r < 0.0;
+  }
+  if (neg) *extra = 1;
+}
+
+// The operands of one cell that do not depend on the sweep.
+template <int MODE, bool UNIFORM>
+struct WaveCell {
+  unsigned fl;
+  double in, d, rd;
+  double o[3];                                     // GS: the neighbours not updated yet; IC(0): the coefficients
+  double w[(MODE >= GS_FWD && !UNIFORM) ? 6 : 1];  // GS on non-uniform grids: the face weights
+};
+
+template <int MODE, bool UNIFORM, bool EXTRA>
+__global__ void __launch_bounds__(WTHREADS) k_wave(WaveArgs A) {
   constexpr bool BWD = (MODE == IC0_BWD || MODE == GS_BWD);
-  __shared__ double sh[2][WTK][WTJ];
-  __shared__ int tile_s, bail_s;
-  __shared__ int seen_j, seen_k;
+  constexpr bool GS = MODE >= GS_FWD;
+  // The last two steps' values, [step & 1][thread], then the received values, [pencil][WRING].
+  __shared__ double sh[2 * WCT + WHALO * WRING];
+  double* const ring = sh + 2 * WCT;
+  __shared__ volatile int seen[WHALO];  // values received per boundary pencil
+  __shared__ volatile int passed;       // steps whose barrier the compute warps have passed
+  __shared__ volatile int bail;
+  __shared__ unsigned long long ticket;
   if (A.S && A.S->done) return;
   const int nx = A.n[0], ny = A.n[1], nz = A.n[2];
-  const long long sx = 1, sy = nx, sz = (long long)nx * ny;
-  const int tj = threadIdx.x % WTJ, tk = threadIdx.x / WTJ;
   if (threadIdx.x == 0) {
-    tile_s = atomicAdd(&A.sync[0], 1);
-    bail_s = 0;
-    seen_j = 0;
-    seen_k = 0;
+    ticket = atomicAdd(&A.sync[0], 1ull);
+    passed = 0;
+    bail = 0;
   }
+  if (threadIdx.x < WHALO) seen[threadIdx.x] = 0;
   __syncthreads();
-  const int t = tile_s;
+  const unsigned ntiles = gridDim.x;  // every block of every launch takes one ticket
+  const unsigned long long epoch = ticket / ntiles + 1;
+  const int t = (int)(ticket % ntiles);
   int J = t % A.tiles_j, K = t / A.tiles_j;  // row-major tiles: producers have smaller tickets
   if (BWD) {
     J = A.tiles_j - 1 - J;
     K = A.tiles_k - 1 - K;
   }
+  if (threadIdx.x >= WCT) {
+    // Receiver warp: lane p < WTJ + WTK follows one boundary pencil of the tile before this
+    // one along j (lanes 0 .. WTK-1: its last pencil column, one per k) or along k. All lanes
+    // take every turn of the loop together, so one round trip serves them all.
+    const int lane = threadIdx.x - WCT;
+    const bool along_j = lane < WTK;
+    const int p = along_j ? lane : lane - WTK;
+    bool open = lane < WHALO && (along_j ? (BWD ? J + 1 < A.tiles_j : J > 0) && K * WTK + p < nz
+                                         : (BWD ? K + 1 < A.tiles_k : K > 0) && J * WTJ + p < ny);
+    const int back = along_j ? 1 : A.tiles_j;  // the producer's ticket is t - back
+    const ulonglong2* src = A.halo + (long long)(open ? t - back : t) * nx * WHALO + (open ? lane : 0);
+    // The pencil's first cell is used at step `late`: entries below passed - late are free.
+    const int late = BWD ? (along_j ? WTK : WTJ) - 1 - p : p;
+    int got = 0;
+    long long polls = 0;
+    for (unsigned turn = 1; __any_sync(0xffffffffu, open); ++turn) {
+      const bool room = open && got + 4 <= passed - late + WRING;
+      int m = 0;
+      if (room) {
+        ulonglong2 v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[q] = ld_halo(src + (long long)min(got + q, nx - 1) * WHALO);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (m == q && got + q < nx && v[q].y == epoch) {
+            ring[lane * WRING + ((got + q) & (WRING - 1))] = __longlong_as_double((long long)v[q].x);
+            m = q + 1;
+          }
+        if (m) {
+          got += m;
+          __threadfence_block();
+          seen[lane] = got;
+          open = got < nx;
+        }
+        polls = m ? 0 : polls + 1;
+      }
+      const bool late_launch = (turn & 63u) == 0 && ld_relaxed(&A.sync[1]) == epoch;
+      if (__any_sync(0xffffffffu, polls > A.spin_limit || late_launch)) {
+        // Give up: flag the launch and let the compute warps run out without waiting; the
+        // host discards the result.
+        if (lane == 0) {
+          atomicExch(&A.sync[1], epoch);
+          atomicExch(A.error, 1);
+          bail = 1;
+        }
+        return;
+      }
+    }
+    return;
+  }
+  const int tj = threadIdx.x % WTJ, tk = threadIdx.x / WTJ;
   const int j = J * WTJ + tj, k = K * WTK + tk;
   const bool lane_ok = j < ny && k < nz;
-  // Distance of this pencil from the tile's first pencil in sweep order.
-  const int dj = BWD ? WTJ - 1 - tj : tj;
-  const int dk = BWD ? WTK - 1 - tk : tk;
+  const int len = lane_ok ? nx : 0;  // cells of this thread's pencil
+  // Distance of this pencil from the tile's first pencil in sweep order, the way along it and
+  // (structured grids have fewer than 2^31 cells) the offsets of the neighbours.
+  const int dj = BWD ? WTJ - 1 - tj : tj, dk = BWD ? WTK - 1 - tk : tk;
+  constexpr int dir = BWD ? -1 : 1;
   const int nsteps = nx + WTJ + WTK - 2;
-  // Producers: the tiles before this one in sweep order along j and along k.
-  const int pj = BWD ? (J + 1 < A.tiles_j ? t - 1 : -1) : (J > 0 ? t - 1 : -1);
-  const int pk = BWD ? (K + 1 < A.tiles_k ? t - A.tiles_j : -1) : (K > 0 ? t - A.tiles_j : -1);
-  int* progress = A.sync + 2;
-  double prev = 0.0;  // this pencil's value at the previous cell in sweep order
-  for (int s = 0; s < nsteps; ++s) {
-    if (threadIdx.x == 0) {
-      // Every thread passed the barrier of step s - 1, so steps 0 .. s - 2 are stored.
-      if (s > 1 && t != A.hold_tile) {
-        __threadfence();
-        st_release(&progress[t], s - 1);
-      }
-      // Boundary pencils at step s need step s + TJ - 1 (s + TK - 1) of the producers.
-      const int need_j = min(s + WTJ, nsteps), need_k = min(s + WTK, nsteps);
-      long long spins = 0;
-      if (pj >= 0 && seen_j < need_j) {
-        int v;
-        while ((v = ld_acquire(&progress[pj])) < need_j) {
-          if (++spins > A.spin_limit || ld_acquire(&A.sync[1])) {
-            bail_s = 1;
-            break;
-          }
+  const bool has_ny = BWD ? j + 1 < ny : j > 0, has_nz = BWD ? k + 1 < nz : k > 0;
+  const bool edge_y = lane_ok && dj == 0 && has_ny, edge_z = lane_ok && dk == 0 && has_nz;
+  // The neighbours along j and k: IC(0) backward reads their rows' coefficients, Gauss-Seidel
+  // the values not updated yet. Where there is none the cell's own entry stands in, unused.
+  const bool has_oy = MODE == IC0_BWD ? has_ny : (BWD ? j > 0 : j + 1 < ny);
+  const bool has_oz = MODE == IC0_BWD ? has_nz : (BWD ? k > 0 : k + 1 < nz);
+  const int oy = has_oy ? (MODE == IC0_BWD ? nx : dir * nx) : 0, oz = has_oz ? (MODE == IC0_BWD ? nx * ny : dir * nx * ny) : 0;
+  // Where a new value along j or k is read: the tile's previous step, or the ring.
+  const int near_y = has_ny && !edge_y ? (int)threadIdx.x - dir : (int)threadIdx.x;
+  const int near_z = has_nz && !edge_z ? (int)threadIdx.x - dir * WTJ : (int)threadIdx.x;
+  const int ring_y = 2 * WCT + tk * WRING, ring_z = 2 * WCT + (WTK + tj) * WRING;
+  const bool pub_y = lane_ok && dj == WTJ - 1 && (BWD ? J > 0 : J + 1 < A.tiles_j) && t != A.hold_tile;
+  const bool pub_z = lane_ok && dk == WTK - 1 && (BWD ? K > 0 : K + 1 < A.tiles_k) && t != A.hold_tile;
+  ulonglong2* pub = A.halo + (long long)t * nx * WHALO;
+  // A thread without a pencil goes through the motions on the first one; its values are not
+  // stored, published or read by any other cell.
+  const int row = lane_ok ? (k * ny + j) * nx : 0;
+  using Cell = WaveCell<MODE, UNIFORM>;
+  Cell cell[WPF];
+  int fat = -dj - dk;  // the cell (in sweep order) fetched next
+  // No branch: outside the pencil its end cell is fetched again, unused.
+  auto fetch = [&](Cell& C) {
+    const int at = min(max(fat, 0), nx - 1);
+    const int c = row + (BWD ? nx - 1 - at : at);
+    C.fl = A.flags[c];
+    C.d = A.diag[c];
+    C.rd = A.rdiag[c];
+    if (MODE == IC0_FWD) {
+      C.in = A.in[c];
+      C.o[0] = A.lx[c], C.o[1] = A.ly[c], C.o[2] = A.lz[c];
+    } else if (MODE == IC0_BWD) {
+      // Rows (k+1), (j+1), (i+1), each with its coefficient towards this cell.
+      C.in = A.x[c];
+      C.o[0] = A.lx[at > 0 ? c + 1 : c];
+      C.o[1] = A.ly[c + oy];
+      C.o[2] = A.lz[c + oz];
+    } else {
+      C.in = A.in[c];
+      C.o[0] = A.x[at + 1 < nx ? c + dir : c];
+      C.o[1] = A.x[c + oy];
+      C.o[2] = A.x[c + oz];
+      if (!UNIFORM) {
+        const int q[3] = {BWD ? nx - 1 - at : at, lane_ok ? j : 0, lane_ok ? k : 0};
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          int f[3] = {q[0], q[1], q[2]};
+          C.w[2 * a] = A.fw[A.face_off[a] + ((long long)f[2] * A.fdim[a][1] + f[1]) * A.fdim[a][0] + f[0]];
+          f[a] += 1;
+          C.w[2 * a + 1] = A.fw[A.face_off[a] + ((long long)f[2] * A.fdim[a][1] + f[1]) * A.fdim[a][0] + f[0]];
         }
-        seen_j = v;
       }
-      if (!bail_s && pk >= 0 && seen_k < need_k) {
-        int v;
-        while ((v = ld_acquire(&progress[pk])) < need_k) {
-          if (++spins > A.spin_limit || ld_acquire(&A.sync[1])) {
-            bail_s = 1;
-            break;
-          }
-        }
-        seen_k = v;
-      }
-      if (bail_s) {
-        atomicExch(&A.sync[1], 1);
-        atomicExch(A.error, 1);
-      }
-      __threadfence();
     }
-    __syncthreads();
-    if (bail_s) return;
-    const int step_i = s - dj - dk;
-    const double* cur_prev = &sh[(s + 1) & 1][0][0];
-    double* cur = &sh[s & 1][0][0];
-    if (lane_ok && step_i >= 0 && step_i < nx) {
-      const int i = BWD ? nx - 1 - step_i : step_i;
-      const long long c = ((long long)k * ny + j) * nx + i;
-      const unsigned fl = A.flags[c];
-      // Neighbour values already updated in this sweep ("new") along x, y, z.
-      const bool has_ny = BWD ? j + 1 < ny : j > 0;
-      const bool has_nz = BWD ? k + 1 < nz : k > 0;
-      const bool in_tile_y = BWD ? tj + 1 < WTJ : tj > 0;
-      const bool in_tile_z = BWD ? tk + 1 < WTK : tk > 0;
-      const long long cy = BWD ? c + sy : c - sy, cz = BWD ? c + sz : c - sz;
-      double newx = prev;
-      double newy = 0.0, newz = 0.0;
-      if (has_ny) newy = in_tile_y ? cur_prev[tk * WTJ + (BWD ? tj + 1 : tj - 1)] : __ldcg(&A.x[cy]);
-      if (has_nz) newz = in_tile_z ? cur_prev[(BWD ? tk + 1 : tk - 1) * WTJ + tj] : __ldcg(&A.x[cz]);
-      double v;
+    ++fat;
+  };
+  // Face f of the cell, where it is in the operator: its weight (GS).
+  const double w0 = A.w_in[0], w1 = A.w_in[1], w2 = A.w_in[2];
+  auto weight = [&](const Cell& C, int f) {
+    return UNIFORM ? (f < 2 ? w0 : f < 4 ? w1 : w2) : C.w[GS && !UNIFORM ? f : 0];
+  };
+  // A term of a row, or the zero whose sum (GS) or difference (IC(0)) leaves every number's
+  // bits alone: -0.0 added, +0.0 subtracted. Selected, not branched around.
+  auto term = [&](const Cell& C, int f, double w, double x) {
+    const double p = w * x;
+    return (C.fl & (1u << f)) ? p : (GS ? -0.0 : 0.0);
+  };
+  double old[3];  // GS: the terms of the neighbours not updated yet, of the step to come
+  auto old_terms = [&](const Cell& C) {
+    if (GS) {
+#pragma unroll
+      for (int a = 0; a < 3; ++a) old[a] = term(C, 2 * a + (BWD ? 0 : 1), weight(C, 2 * a + (BWD ? 0 : 1)), C.o[a]);
+    }
+  };
+  double prev = 0.0;  // this pencil's value at the previous cell in sweep order
+  int have_y = edge_y ? 0 : nx, have_z = edge_z ? 0 : nx;  // received values as last seen
+#pragma unroll
+  for (int m = 0; m < WPF; ++m) fetch(cell[m]);
+  old_terms(cell[0]);
+  int at = -dj - dk, c = row + (BWD ? nx - 1 : 0) + dir * at;
+  for (int s0 = 0; s0 < nsteps; s0 += WPF) {  // steps past nsteps - 1 find no cell in range
+#pragma unroll
+    for (int m = 0; m < WPF; ++m, ++at, c += dir) {
+      Cell& C = cell[m];
+      const bool on = (unsigned)at < (unsigned)len;
+      while (__any_sync(0xffffffffu, on && (have_y <= at || have_z <= at))) {
+        if (edge_y) have_y = seen[tk];
+        if (edge_z) have_z = seen[WTK + tj];
+        if (bail) have_y = have_z = nx;
+      }
+      asm volatile("bar.sync 1, %0;" ::"n"(WCT) : "memory");  // the step before is in sh
+      if (m == 0 && threadIdx.x == 0) passed = s0;
+      const int before = ((m + 1) & 1) * WCT;  // WPF is even: step parity is m's
+      const int slot = at & (WRING - 1);
+      const double newy = sh[edge_y ? ring_y + slot : before + near_y];
+      const double newz = sh[edge_z ? ring_z + slot : before + near_z];
+      double v = C.in;
       if (MODE == IC0_FWD) {
         // Ascending columns: (k-1), (j-1), (i-1).
-        v = A.in[c];
-        if (fl & (1u << 4)) v = v - A.lz[c] * newz;
-        if (fl & (1u << 2)) v = v - A.ly[c] * newy;
-        if (fl & (1u << 0)) v = v - A.lx[c] * newx;
-        v = v / A.diag[c];
+        v = v - term(C, 4, C.o[2], newz);
+        v = v - term(C, 2, C.o[1], newy);
+        v = v - term(C, 0, C.o[0], prev);
+        v = div_pre<EXTRA>(v, C.d, C.rd, on);
       } else if (MODE == IC0_BWD) {
-        // Rows (k+1), (j+1), (i+1) in descending order, each with its coefficient
-        // towards this cell.
-        v = __ldcg(&A.x[c]);
-        if (fl & (1u << 5)) v = v - A.lz[c + sz] * newz;
-        if (fl & (1u << 3)) v = v - A.ly[c + sy] * newy;
-        if (fl & (1u << 1)) v = v - A.lx[c + sx] * newx;
-        v = v / A.diag[c];
+        // Rows (k+1), (j+1), (i+1) in descending order.
+        v = v - term(C, 5, C.o[2], newz);
+        v = v - term(C, 3, C.o[1], newy);
+        v = v - term(C, 1, C.o[0], prev);
+        v = div_pre<EXTRA>(v, C.d, C.rd, on);
       } else {
-        const double d = A.diag[c];
-        if (d == 0.0) {
-          v = 0.0;  // a cell with no faces in the operator: a sealed singleton, or a solid cell
-        } else {
-          // Row order x-lo, x-hi, y-lo, y-hi, z-lo, z-hi; entries are -w, and
-          // v - (-w) x == v + w x exactly.
-          double w[6];
-          if (A.uniform) {
-#pragma unroll
-            for (int a = 0; a < 3; ++a) w[2 * a] = w[2 * a + 1] = A.w_in[a];
-          } else {
-            const int q[3] = {i, j, k};
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-              int p[3] = {q[0], q[1], q[2]};
-              w[2 * a] = A.fw[A.face_off[a] + ((long long)p[2] * A.fdim[a][1] + p[1]) * A.fdim[a][0] + p[0]];
-              p[a] += 1;
-              w[2 * a + 1] = A.fw[A.face_off[a] + ((long long)p[2] * A.fdim[a][1] + p[1]) * A.fdim[a][0] + p[0]];
-            }
-          }
-          // Lower neighbours are "new" in a forward sweep, upper ones in a backward sweep.
-          const double xlo = BWD ? (i > 0 ? __ldcg(&A.x[c - sx]) : 0.0) : newx;
-          const double xhi = BWD ? newx : (i + 1 < nx ? __ldcg(&A.x[c + sx]) : 0.0);
-          const double ylo = BWD ? (j > 0 ? __ldcg(&A.x[c - sy]) : 0.0) : newy;
-          const double yhi = BWD ? newy : (j + 1 < ny ? __ldcg(&A.x[c + sy]) : 0.0);
-          const double zlo = BWD ? (k > 0 ? __ldcg(&A.x[c - sz]) : 0.0) : newz;
-          const double zhi = BWD ? newz : (k + 1 < nz ? __ldcg(&A.x[c + sz]) : 0.0);
-          v = A.in[c];
-          if (fl & (1u << 0)) v = v + w[0] * xlo;
-          if (fl & (1u << 1)) v = v + w[1] * xhi;
-          if (fl & (1u << 2)) v = v + w[2] * ylo;
-          if (fl & (1u << 3)) v = v + w[3] * yhi;
-          if (fl & (1u << 4)) v = v + w[4] * zlo;
-          if (fl & (1u << 5)) v = v + w[5] * zhi;
-          v = v / d;
-        }
+        // Row order x-lo, x-hi, y-lo, y-hi, z-lo, z-hi; entries are -w, and v - (-w) x == v + w x
+        // exactly.
+        const double nx_ = term(C, BWD ? 1 : 0, weight(C, BWD ? 1 : 0), prev);
+        const double ny_ = term(C, BWD ? 3 : 2, weight(C, BWD ? 3 : 2), newy);
+        const double nz_ = term(C, BWD ? 5 : 4, weight(C, BWD ? 5 : 4), newz);
+        v = v + (BWD ? old[0] : nx_);
+        v = v + (BWD ? nx_ : old[0]);
+        v = v + (BWD ? old[1] : ny_);
+        v = v + (BWD ? ny_ : old[1]);
+        v = v + (BWD ? old[2] : nz_);
+        v = v + (BWD ? nz_ : old[2]);
+        // d = 0: a cell with no faces in the operator (a sealed singleton, or a solid cell).
+        const bool some = ((unsigned)__double2hiint(C.d) << 1 | (unsigned)__double2loint(C.d)) != 0;
+        v = div_pre<EXTRA>(v, C.d, C.rd, on && some);
+        if (!some) v = 0.0;
       }
-      A.x[c] = v;
-      cur[tk * WTJ + tj] = v;
+      sh[(m & 1) * WCT + threadIdx.x] = v;
       prev = v;
+      st_halo(pub + at * WHALO + tk, v, epoch, on && pub_y);
+      st_halo(pub + at * WHALO + WTK + tj, v, epoch, on && pub_z);
+      if (on) A.x[c] = v;
+      old_terms(cell[(m + 1) % WPF]);
+      fetch(C);
     }
   }
-  __syncthreads();
-  if (threadIdx.x == 0 && t != A.hold_tile) {
-    __threadfence();
-    st_release(&progress[t], nsteps);
-  }
 }
+
+static_assert(WPF % 2 == 0, "the step's buffer is chosen by its place in the unrolled group");
 
 }  // namespace cfdg

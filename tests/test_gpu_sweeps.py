@@ -1,0 +1,40 @@
+"""The wavefront sweeps of the plain form at the edges of their tiles: IC(0) and the
+multigrid cycle, bit for bit the oracle's natural-order loops (8x8 tiles of x-pencils:
+remainders in y and z, pencils shorter than the tile's skew and longer than the ring of
+received values, per-face weights, right-hand sides outside the range of the division from
+precomputed reciprocals)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def bits(a):
+    return np.ascontiguousarray(a, np.float64).view(np.uint64)
+
+
+@pytest.mark.parametrize("scale", [1.0, 1e-290])
+@pytest.mark.parametrize("faces", ["uniform", "perturbed"])
+@pytest.mark.parametrize("cells", [(2, 9, 7), (3, 8, 8), (17, 17, 9), (300, 5, 3), (21, 24, 16)])
+def test_sweeps_bitwise_at_tile_edges(pkg, O, cells, faces, scale):
+    boxes = [((3.0, 3.0, 0.0), (7.5, 7.5, 4.5))] if min(cells) > 8 else []
+    case = pkg.synth.case(cells, 1.5, inflow=5.0, boxes=boxes)
+    g = pkg.grid.Grid.build(case)
+    og = O.Grid(case)
+    dg = pkg.pressure.DeviceGrid(g, preconditioner="ic0")
+    if faces == "perturbed":
+        area = g.face_area * (1.0 + (np.arange(g.n_faces) % 7) * 0.025)
+        og.set_faces(area=area)
+        dg.update_faces(area=area)
+    rng = np.random.default_rng(sum(cells))
+    r = np.where(g.fluid == 1, rng.uniform(-1.0, 1.0, g.count), 0.0)
+    r[rng.integers(0, g.count, g.count // 8)] = 0.0
+    r *= scale
+    for _ in range(2):  # a second sweep over the same hand-off entries
+        assert np.array_equal(bits(dg.precondition(r)), bits(og.ic0_apply(r)))
+    dg.configure("multigrid")
+    og.set_preconditioner("multigrid")
+    oz, _ = og.mg_apply(r)
+    for _ in range(2):
+        assert np.array_equal(bits(dg.precondition(r)), bits(oz))
+    dg.close()
