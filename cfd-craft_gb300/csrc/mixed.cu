@@ -195,91 +195,53 @@ __device__ __forceinline__ double bsum(double v, double* sh) {
   return s;
 }
 
-// Reductions of the fine-level kernels. A tile's warps leave their sums in shared memory and
-// the first warp adds them in a fixed tree into the tile's one partial; a block counts a
-// case's tiles once per run of consecutive tiles of that case, and the block that completes
-// a case sums the partials in slot order (the same bits whatever the grid size) and applies
-// the case's scalar update. One partial per tile instead of one per warp: the last block's
-// sum is a chain of FP64 additions (64 cycles per warp and sub-core), 8 us of them for the
-// 32,768 warps' partials of 8.4 M cells.
-constexpr int PG = 4;  // tiles of a group (tile_run)
-struct TileSums {
-  double d[2][PG][TILE / 32];  // two buffers: one barrier per group of tiles
-  float2 f[2][PG][TILE / 32];
-};
-
-// The warp's part of a tile's FP64 sum, and the partials of a group of tiles from them (as
-// tile_pair and group_partials below).
-__device__ __forceinline__ void tile_sum(double v, TileSums& ts, int buf, int m) {
+// Reductions of the fine-level kernels. Every warp stores its sum in the case's partials
+// (slot = tile * RT + warp, no block barrier); a block counts a case's tiles once per run
+// of consecutive tiles of that case, and the block that completes a case sums the
+// partials in slot order (the same bits whatever the grid size) and applies the case's
+// scalar update.
+__device__ __forceinline__ void tile_partial(double v, const FineCase& F, int lt, double* sh, int& seg_n) {
+  (void)sh;
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  if ((threadIdx.x & 31) == 0) ts.d[buf][m][threadIdx.x >> 5] = v;
-}
-__device__ __forceinline__ void group_sums(const FineCase& F, int lt, int n, TileSums& ts, int buf, int& seg_n) {
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    const int m = threadIdx.x / (TILE / 32), w = threadIdx.x % (TILE / 32);
-    double v = m < n ? ts.d[buf][m][w] : 0.0;
-#pragma unroll
-    for (int o = TILE / 64; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o, TILE / 32);
-    if (w == 0 && m < n) F.partials[lt + m] = v;
-  }
-  seg_n += n;
+  if ((threadIdx.x & 31) == 0) F.partials[lt * (TILE / 32) + (threadIdx.x >> 5)] = v;
+  ++seg_n;
 }
 
-// (hi, lo) += (h2, l2) for compensated FP32 pairs (TwoSum).
-__device__ __forceinline__ void pair_add(float& hi, float& lo, float h2, float l2) {
-  const float s = hi + h2, bb = s - hi;
-  lo += l2 + ((hi - (s - bb)) + (h2 - bb));
-  hi = s;
-}
-// The warp's part of a tile's sum of compensated FP32 pairs, one pair per thread: the pairs
-// stay in FP32 and become one FP64 number per tile (the FP64 pipe is narrow). m: the tile's
-// place in its group, buf: the group's buffer.
-__device__ __forceinline__ void tile_pair(float hi, float lo, TileSums& ts, int buf, int m) {
-  for (int o = 16; o > 0; o >>= 1)
-    pair_add(hi, lo, __shfl_down_sync(0xffffffffu, hi, o), __shfl_down_sync(0xffffffffu, lo, o));
-  if ((threadIdx.x & 31) == 0) ts.f[buf][m][threadIdx.x >> 5] = make_float2(hi, lo);
-}
-// The partials of the n tiles lt .. lt + n - 1 from their warps' pairs. Every thread of the
-// block calls it once per group; the buffers alternate from group to group.
-__device__ __forceinline__ void group_partials(const FineCase& F, int lt, int n, TileSums& ts, int buf, int& seg_n) {
-  static_assert(PG * (TILE / 32) == 32, "one lane per tile of the group and warp");
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    const int m = threadIdx.x / (TILE / 32), w = threadIdx.x % (TILE / 32);
-    const float2 v = m < n ? ts.f[buf][m][w] : make_float2(0.0f, 0.0f);
-    float hi = v.x, lo = v.y;
-#pragma unroll
-    for (int o = TILE / 64; o > 0; o >>= 1)
-      pair_add(hi, lo, __shfl_down_sync(0xffffffffu, hi, o, TILE / 32), __shfl_down_sync(0xffffffffu, lo, o, TILE / 32));
-    if (w == 0 && m < n) F.partials[lt + m] = (double)hi + (double)lo;
+// The same from a compensated FP32 pair per thread (hi, lo): the warp's pairs are summed
+// with TwoSum in FP32 and converted to FP64 once per warp (the FP64 pipe is narrow).
+__device__ __forceinline__ void tile_partial2(float hi, float lo, const FineCase& F, int lt, int& seg_n) {
+  for (int o = 16; o > 0; o >>= 1) {
+    const float h2 = __shfl_down_sync(0xffffffffu, hi, o), l2 = __shfl_down_sync(0xffffffffu, lo, o);
+    const float s = hi + h2, bb = s - hi;
+    lo += l2 + ((hi - (s - bb)) + (h2 - bb));
+    hi = s;
   }
-  seg_n += n;
+  if ((threadIdx.x & 31) == 0) F.partials[lt * (TILE / 32) + (threadIdx.x >> 5)] = (double)hi + (double)lo;
+  ++seg_n;
 }
 
 struct Seg {
   int ci = -1, n = 0;  // case of the current run of tiles, tiles with a stored partial
-  int buf = 0;         // buffer of the next group's sums
 };
 
 template <class Fin>
 __device__ __forceinline__ void close_seg(const FineCase* FC, MState* ST, Seg& g, double* sh, Fin fin) {
   if (g.n == 0) return;
   __shared__ bool last;
-  __syncthreads();  // the partials of the run are stored (by the first warp)
+  __syncthreads();  // every warp's partials of the run are stored
   if (threadIdx.x == 0) {
-    __threadfence();  // cumulative over the barrier: the stores of the block's first warp
+    __threadfence();
     last = atomicAdd(&ST[g.ci].counter, (unsigned)g.n) + (unsigned)g.n == (unsigned)FC[g.ci].ntiles;
   }
   __syncthreads();
   g.n = 0;
   if (!last) return;
   __threadfence();
-  const int nt = FC[g.ci].ntiles;
+  const int nt = FC[g.ci].ntiles * (TILE / 32);
   const double* part = FC[g.ci].partials;
   // One block reads every partial of the case while the others have finished: eight loads in
   // flight per thread, added in slot order (the sums start at +0, so the zeros past the end
-  // change nothing). One load at a time, the round trips of 32,768 partials took 48 us.
+  // change nothing). One load at a time took 48 us for the 32,768 partials of 8.4 M cells.
   double a = 0.0;
   for (int k = threadIdx.x; k < nt; k += 8 * TILE) {
     double v[8];
@@ -319,6 +281,7 @@ __device__ __forceinline__ void close_seg(const FineCase* FC, MState* ST, Seg& g
 // state and descriptor) is paid once per group and a warp's loads of several rows are in
 // flight together. tile_run: the length of the run of consecutive tiles of t's case that
 // starts at list entry ti (at most PG, inside the block's range).
+constexpr int PG = 4;
 __device__ __forceinline__ int tile_run(const int2* tiles, int ti, int t1, int2 t) {
   int2 u[PG - 1];
 #pragma unroll
@@ -617,79 +580,69 @@ struct FinOp {
   }
 };
 
-// A: q = A32 p, alpha = rz / (p.q) (E032 when not positive), over the n tiles lt .. lt+n-1.
-__device__ __forceinline__ void b_op(const FineCase* FC, MState* ST, const int2 t, int n, int& cached_, TileSums& ts,
-                                    Seg& g) {
+// A: q = A32 p, alpha = rz / (p.q) (E032 when not positive).
+__device__ __forceinline__ void b_op(const FineCase* FC, MState* ST, const int2 t, int& cached_, double* sh,
+                                    int& seg_n) {
   FINE_PROLOGUE(S.state == RUN)
-  for (int m = 0; m < n; ++m) {
-    float hi = 0.0f, lo = 0.0f;
-    int j, k, rb;
-    if (warp_row(F, lt + m, warp, j, k, rb) && F.uniform && !(nxh_ & 1)) {
-      const int r = (lt + m) * RT + warp, sy = 2 * nxh_, sz = sy * F.n[1];
-      const bool hy0 = j > 0, hy1 = j + 1 < F.n[1], hz0 = k > 0, hz1 = k + 1 < F.n[2];
-      for (int col = 0; col < 2; ++col) {
-        const int par = (j + k + col) & 1;
-        const int own = lay(r, col, nxh_, 0), oth = lay(r, col ^ 1, nxh_, 0);
-        for (int s2 = 2 * lane; s2 < nxh_; s2 += 64) {
-          const float2 pc = *reinterpret_cast<const float2*>(F.p + own + s2);
-          const unsigned fl2 = *reinterpret_cast<const unsigned*>(F.flags0 + own + s2);
-          Pair P;
-          P.load(F.p, oth, s2, par, nxh_, sy, sz, hy0, hy1, hz0, hz1);
-          float nb[6];
-          float2 y = make_float2(0.0f, 0.0f);
-          // Interior faces in face order, each through a selected weight (0 where the face
-          // is not interior) instead of a branch; the rare outlet faces after them.
-          P.of(0, par, nb);
+  float hi = 0.0f, lo = 0.0f;
+  int j, k, rb;
+  if (warp_row(F, lt, warp, j, k, rb) && F.uniform && !(nxh_ & 1)) {
+    const int r = lt * RT + warp, sy = 2 * nxh_, sz = sy * F.n[1];
+    const bool hy0 = j > 0, hy1 = j + 1 < F.n[1], hz0 = k > 0, hz1 = k + 1 < F.n[2];
+    for (int col = 0; col < 2; ++col) {
+      const int par = (j + k + col) & 1;
+      const int own = lay(r, col, nxh_, 0), oth = lay(r, col ^ 1, nxh_, 0);
+      for (int s2 = 2 * lane; s2 < nxh_; s2 += 64) {
+        const float2 pc = *reinterpret_cast<const float2*>(F.p + own + s2);
+        const unsigned fl2 = *reinterpret_cast<const unsigned*>(F.flags0 + own + s2);
+        Pair P;
+        P.load(F.p, oth, s2, par, nxh_, sy, sz, hy0, hy1, hz0, hz1);
+        float nb[6];
+        float2 y = make_float2(0.0f, 0.0f);
+        // Interior faces in face order, each through a selected weight (0 where the face
+        // is not interior) instead of a branch; the rare outlet faces after them.
+        P.of(0, par, nb);
 #pragma unroll
-          for (int f = 0; f < 6; ++f) y.x = fmaf((fl2 & (1u << f)) ? F.w32[f >> 1] : 0.0f, pc.x - nb[f], y.x);
-          if (fl2 & 0xfc0u) y.x = fmaf(outlet_sum(F, fl2 >> 6), pc.x, y.x);
-          P.of(1, par, nb);
+        for (int f = 0; f < 6; ++f) y.x = fmaf((fl2 & (1u << f)) ? F.w32[f >> 1] : 0.0f, pc.x - nb[f], y.x);
+        if (fl2 & 0xfc0u) y.x = fmaf(outlet_sum(F, fl2 >> 6), pc.x, y.x);
+        P.of(1, par, nb);
 #pragma unroll
-          for (int f = 0; f < 6; ++f) y.y = fmaf((fl2 & (1u << (16 + f))) ? F.w32[f >> 1] : 0.0f, pc.y - nb[f], y.y);
-          if (fl2 & 0xfc00000u) y.y = fmaf(outlet_sum(F, fl2 >> 22), pc.y, y.y);
-          *reinterpret_cast<float2*>(F.q + own + s2) = y;
-          // p.q: the pair's two products in one FMA, then a compensated running sum.
-          dd_add(fmaf(pc.x, y.x, pc.y * y.y), hi, lo);
-        }
-      }
-    } else if (warp_row(F, lt + m, warp, j, k, rb)) {
-      const int r = (lt + m) * RT + warp, sy = 2 * nxh_, sz = sy * F.n[1];
-      for (int col = 0; col < 2; ++col) {
-        const int par = (j + k + col) & 1;
-        const int own = lay(r, col, nxh_, 0), oth = lay(r, col ^ 1, nxh_, 0);
-        for (int s = lane; s < nxh_; s += 32) {
-          const int i = 2 * s + par;
-          if (i >= nx_) break;
-          const float v = op32s(F, F.p, own + s, Nbr(oth, i, s, sy, sz), i, j, k, F.flags0[own + s]);
-          F.q[own + s] = v;
-          dd_add_prod(F.p[own + s], v, hi, lo);
-        }
+        for (int f = 0; f < 6; ++f) y.y = fmaf((fl2 & (1u << (16 + f))) ? F.w32[f >> 1] : 0.0f, pc.y - nb[f], y.y);
+        if (fl2 & 0xfc00000u) y.y = fmaf(outlet_sum(F, fl2 >> 22), pc.y, y.y);
+        *reinterpret_cast<float2*>(F.q + own + s2) = y;
+        // p.q: the pair's two products in one FMA, then a compensated running sum.
+        dd_add(fmaf(pc.x, y.x, pc.y * y.y), hi, lo);
       }
     }
-    tile_pair(hi, lo, ts, g.buf, m);
+  } else if (warp_row(F, lt, warp, j, k, rb)) {
+    const int r = lt * RT + warp, sy = 2 * nxh_, sz = sy * F.n[1];
+    for (int col = 0; col < 2; ++col) {
+      const int par = (j + k + col) & 1;
+      const int own = lay(r, col, nxh_, 0), oth = lay(r, col ^ 1, nxh_, 0);
+      for (int s = lane; s < nxh_; s += 32) {
+        const int i = 2 * s + par;
+        if (i >= nx_) break;
+        const float v = op32s(F, F.p, own + s, Nbr(oth, i, s, sy, sz), i, j, k, F.flags0[own + s]);
+        F.q[own + s] = v;
+        dd_add_prod(F.p[own + s], v, hi, lo);
+      }
+    }
   }
-  group_partials(F, lt, n, ts, g.buf, g.n);
-  g.buf ^= 1;
+  tile_partial2(hi, lo, F, lt, seg_n);
 }
 __global__ void __launch_bounds__(TILE, 5) k_op(const FineCase* FC, MState* ST, const int2* tiles, const int* count) {
   __shared__ double sh[32];
-  __shared__ TileSums ts;
   TILE_RANGE
   int cached_ = -1;  // case whose descriptor is in shared memory
   Seg g;
-  for (int ti = t0_; ti < t1_;) {
+  for (int ti = t0_; ti < t1_; ++ti) {
     const int2 t = tiles[ti];
-    if (ST[t.x].state != RUN) {  // the rest of this case's tiles in the range
-      ti += FC[t.x].ntiles - t.y;
-      continue;
-    }
+    SKIP_CASE(t, S_.state == RUN)
     if (t.x != g.ci) {
       close_seg(FC, ST, g, sh, FinOp());
       g.ci = t.x;
     }
-    const int n = tile_run(tiles, ti, t1_, t);
-    b_op(FC, ST, t, n, cached_, ts, g);
-    ti += n;
+    b_op(FC, ST, t, cached_, sh, g.n);
   }
   close_seg(FC, ST, g, sh, FinOp());
 }
@@ -715,7 +668,7 @@ __device__ __forceinline__ bool group4(const FineCase& F, int sb, int nxh) {
 // B: e += alpha p, r -= alpha q; |r| decides the end of the inner solve. One reduction
 // partial per tile, as in the one-tile path, so the bits do not depend on the grouping.
 __device__ __forceinline__ void b_update(const FineCase* FC, MState* ST, const int2 t, int n, int& cached_,
-                                         TileSums& ts, Seg& g) {
+                                         int& seg_n) {
   FINE_PROLOGUE(S.state == RUN)
   const float alpha = (float)S.alpha;
   const int T = RT * 2 * nxh_;
@@ -744,10 +697,8 @@ __device__ __forceinline__ void b_update(const FineCase* FC, MState* ST, const i
         st4(F.r32 + c, rv);
         dd_add(fmaf(rv.x, rv.x, fmaf(rv.y, rv.y, fmaf(rv.z, rv.z, rv.w * rv.w))), hi, lo);
       }
-      tile_pair(hi, lo, ts, g.buf, m);
+      tile_partial2(hi, lo, F, lt + m, seg_n);
     }
-    group_partials(F, lt, n, ts, g.buf, g.n);
-    g.buf ^= 1;
     return;
   }
   for (int m = 0; m < n; ++m) {
@@ -773,14 +724,11 @@ __device__ __forceinline__ void b_update(const FineCase* FC, MState* ST, const i
         dd_add_prod(r, r, hi, lo);
       }
     }
-    tile_pair(hi, lo, ts, g.buf, m);
+    tile_partial2(hi, lo, F, lt + m, seg_n);
   }
-  group_partials(F, lt, n, ts, g.buf, g.n);
-  g.buf ^= 1;
 }
 __global__ void __launch_bounds__(TILE) k_update(const FineCase* FC, MState* ST, const int2* tiles, const int* count) {
   __shared__ double sh[32];
-  __shared__ TileSums ts;
   TILE_RANGE
   int cached_ = -1;  // case whose descriptor is in shared memory
   Seg g;
@@ -795,7 +743,7 @@ __global__ void __launch_bounds__(TILE) k_update(const FineCase* FC, MState* ST,
       g.ci = t.x;
     }
     const int n = tile_run(tiles, ti, t1_, t);
-    b_update(FC, ST, t, n, cached_, ts, g);
+    b_update(FC, ST, t, n, cached_, g.n);
     ti += n;
   }
   close_seg(FC, ST, g, sh, FinUpdate());
@@ -839,86 +787,76 @@ struct FinOuterResid {
   }
 };
 
-// r = b_c - A x in FP64; the true residual decides convergence. The n tiles lt .. lt+n-1.
-__device__ __forceinline__ void b_outer_resid(const FineCase* FC, MState* ST, const int2 t, int n, int& cached_,
-                                              TileSums& ts, Seg& g) {
+// r = b_c - A x in FP64; the true residual decides convergence.
+__device__ __forceinline__ void b_outer_resid(const FineCase* FC, MState* ST, const int2 t, int& cached_, double* sh,
+                                    int& seg_n) {
   FINE_PROLOGUE(S.state == OUTER)
-  for (int m = 0; m < n; ++m) {
-    double acc = 0.0;
-    int j, k, rb;
-    if (!S.has_e) {
-      // First outer step: x = 0 exactly, so A x = 0 and r = b_c bit for bit.
-      for (int c = cb + m * RT * nx_ + threadIdx.x; c < min(F.N, cb + (m + 1) * RT * nx_); c += TILE) {
-        const double v = F.bc[c];
-        F.r64[c] = v;
+  double acc = 0.0;
+  int j, k, rb;
+  if (!S.has_e) {
+    // First outer step: x = 0 exactly, so A x = 0 and r = b_c bit for bit.
+    for (int c = cb + threadIdx.x; c < ce; c += TILE) {
+      const double v = F.bc[c];
+      F.r64[c] = v;
+      acc = __fma_rn(v, v, acc);
+    }
+  } else if (warp_row(F, lt, warp, j, k, rb)) {
+    // One warp per row, several cells per lane: the cells' FP64 chains are independent.
+    const double* __restrict__ x = F.x64;
+    const double* __restrict__ bc = F.bc;
+    const uint16_t* __restrict__ fl = F.flags;
+    double* __restrict__ r = F.r64;
+    if (F.uniform) {
+      // A x as diag x minus the interior neighbours through one FMA each (nine FP64
+      // operations per cell against the fourteen of the reference's rounding order): on
+      // this part the FP64 pipe bounds the kernel. The rounding differs from
+      // pressure::apply's by a few ulps of diag |x|, far below the 1e-8 test.
+      const int sy = F.n[0], sz = F.n[0] * F.n[1];
+      const double mw[3] = {-F.w64[0], -F.w64[1], -F.w64[2]};
+      const double* __restrict__ d64 = F.diag64;
+#pragma unroll 4
+      for (int i = lane; i < nx_; i += 32) {
+        const int c = rb + i;
+        const unsigned f = fl[c];
+        double y = 0.0;
+        if (f & 0x0fffu) {
+          y = d64[c] * x[c];
+          if (f & 1u) y = __fma_rn(mw[0], x[c - 1], y);
+          if (f & 2u) y = __fma_rn(mw[0], x[c + 1], y);
+          if (f & 4u) y = __fma_rn(mw[1], x[c - sy], y);
+          if (f & 8u) y = __fma_rn(mw[1], x[c + sy], y);
+          if (f & 16u) y = __fma_rn(mw[2], x[c - sz], y);
+          if (f & 32u) y = __fma_rn(mw[2], x[c + sz], y);
+        }
+        const double v = __dsub_rn(bc[c], y);
+        r[c] = v;
         acc = __fma_rn(v, v, acc);
       }
-    } else if (warp_row(F, lt + m, warp, j, k, rb)) {
-      // One warp per row, several cells per lane: the cells' FP64 chains are independent.
-      const double* __restrict__ x = F.x64;
-      const double* __restrict__ bc = F.bc;
-      const uint16_t* __restrict__ fl = F.flags;
-      double* __restrict__ r = F.r64;
-      if (F.uniform) {
-        // A x as diag x minus the interior neighbours through one FMA each (nine FP64
-        // operations per cell against the fourteen of the reference's rounding order): on
-        // this part the FP64 pipe bounds the kernel. The rounding differs from
-        // pressure::apply's by a few ulps of diag |x|, far below the 1e-8 test.
-        const int sy = F.n[0], sz = F.n[0] * F.n[1];
-        const double mw[3] = {-F.w64[0], -F.w64[1], -F.w64[2]};
-        const double* __restrict__ d64 = F.diag64;
+    } else {
 #pragma unroll 4
-        for (int i = lane; i < nx_; i += 32) {
-          const int c = rb + i;
-          const unsigned f = fl[c];
-          double y = 0.0;
-          if (f & 0x0fffu) {
-            y = d64[c] * x[c];
-            if (f & 1u) y = __fma_rn(mw[0], x[c - 1], y);
-            if (f & 2u) y = __fma_rn(mw[0], x[c + 1], y);
-            if (f & 4u) y = __fma_rn(mw[1], x[c - sy], y);
-            if (f & 8u) y = __fma_rn(mw[1], x[c + sy], y);
-            if (f & 16u) y = __fma_rn(mw[2], x[c - sz], y);
-            if (f & 32u) y = __fma_rn(mw[2], x[c + sz], y);
-          }
-          const double v = __dsub_rn(bc[c], y);
-          r[c] = v;
-          acc = __fma_rn(v, v, acc);
-        }
-      } else {
-#pragma unroll 4
-        for (int i = lane; i < nx_; i += 32) {
-          const int c = rb + i;
-          const double v = __dsub_rn(bc[c], op64r(F, x, c, i, j, k, fl[c]));
-          r[c] = v;
-          acc = __fma_rn(v, v, acc);
-        }
+      for (int i = lane; i < nx_; i += 32) {
+        const int c = rb + i;
+        const double v = __dsub_rn(bc[c], op64r(F, x, c, i, j, k, fl[c]));
+        r[c] = v;
+        acc = __fma_rn(v, v, acc);
       }
     }
-    tile_sum(acc, ts, g.buf, m);
   }
-  group_sums(F, lt, n, ts, g.buf, g.n);
-  g.buf ^= 1;
+  tile_partial(acc, F, lt, sh, seg_n);
 }
 __global__ void __launch_bounds__(TILE) k_outer_resid(const FineCase* FC, MState* ST, const int2* tiles, const int* count) {
   __shared__ double sh[32];
-  __shared__ TileSums ts;
   TILE_RANGE
   int cached_ = -1;  // case whose descriptor is in shared memory
   Seg g;
-  for (int ti = t0_; ti < t1_;) {
+  for (int ti = t0_; ti < t1_; ++ti) {
     const int2 t = tiles[ti];
-    if (ST[t.x].state != OUTER) {  // the rest of this case's tiles in the range
-      ti += FC[t.x].ntiles - t.y;
-      continue;
-    }
+    SKIP_CASE(t, S_.state == OUTER)
     if (t.x != g.ci) {
       close_seg(FC, ST, g, sh, FinOuterResid());
       g.ci = t.x;
     }
-    const int n = tile_run(tiles, ti, t1_, t);
-    b_outer_resid(FC, ST, t, n, cached_, ts, g);
-    ti += n;
+    b_outer_resid(FC, ST, t, cached_, sh, g.n);
   }
   close_seg(FC, ST, g, sh, FinOuterResid());
 }
@@ -971,8 +909,7 @@ struct FinRz {
 };
 
 // F: rz' = r.z; START: rz = rz', p = z (beta = 0) -> RUN; RUN: beta = rz'/rz.
-__device__ __forceinline__ void b_rz(const FineCase* FC, MState* ST, const int2 t, int n, int& cached_, TileSums& ts,
-                                     Seg& g) {
+__device__ __forceinline__ void b_rz(const FineCase* FC, MState* ST, const int2 t, int n, int& cached_, int& seg_n) {
   FINE_PROLOGUE(S.state == RUN || S.state == START)
   const int T = RT * 2 * nxh_;
   if (group4(F, sb, nxh_)) {
@@ -989,10 +926,8 @@ __device__ __forceinline__ void b_rz(const FineCase* FC, MState* ST, const int2 
       if (m >= n) break;
       float hi = 0.0f, lo = 0.0f;
       if (ok[m]) dd_add(fmaf(r[m].x, z[m].x, fmaf(r[m].y, z[m].y, fmaf(r[m].z, z[m].z, r[m].w * z[m].w))), hi, lo);
-      tile_pair(hi, lo, ts, g.buf, m);
+      tile_partial2(hi, lo, F, lt + m, seg_n);
     }
-    group_partials(F, lt, n, ts, g.buf, g.n);
-    g.buf ^= 1;
     return;
   }
   for (int m = 0; m < n; ++m) {
@@ -1006,14 +941,11 @@ __device__ __forceinline__ void b_rz(const FineCase* FC, MState* ST, const int2 
     } else {
       for (int c = b0 + threadIdx.x; c < b1; c += TILE) dd_add_prod(F.r32[c], F.x0[c], hi, lo);
     }
-    tile_pair(hi, lo, ts, g.buf, m);
+    tile_partial2(hi, lo, F, lt + m, seg_n);
   }
-  group_partials(F, lt, n, ts, g.buf, g.n);
-  g.buf ^= 1;
 }
 __global__ void __launch_bounds__(TILE) k_rz(const FineCase* FC, MState* ST, const int2* tiles, const int* count) {
   __shared__ double sh[32];
-  __shared__ TileSums ts;
   TILE_RANGE
   int cached_ = -1;  // case whose descriptor is in shared memory
   Seg g;
@@ -1028,7 +960,7 @@ __global__ void __launch_bounds__(TILE) k_rz(const FineCase* FC, MState* ST, con
       g.ci = t.x;
     }
     const int n = tile_run(tiles, ti, t1_, t);
-    b_rz(FC, ST, t, n, cached_, ts, g);
+    b_rz(FC, ST, t, n, cached_, g.n);
     ti += n;
   }
   close_seg(FC, ST, g, sh, FinRz());
@@ -2437,8 +2369,8 @@ struct FinNorm {
 };
 
 // |b_c| (after the host-side gauge of closed components); x = 0.
-__device__ __forceinline__ void b_norm(const FineCase* FC, MState* ST, const int2 t, int& cached_, TileSums& ts,
-                                       Seg& g) {
+__device__ __forceinline__ void b_norm(const FineCase* FC, MState* ST, const int2 t, int& cached_, double* sh,
+                                    int& seg_n) {
   FINE_PROLOGUE(S.state == IDLE)
   double acc = 0.0;
   for (int c = cb + threadIdx.x; c < ce; c += TILE) {
@@ -2447,13 +2379,10 @@ __device__ __forceinline__ void b_norm(const FineCase* FC, MState* ST, const int
     F.x64[c] = 0.0;
   }
   for (int c = sb + threadIdx.x; c < se; c += TILE) F.e[c] = 0.0f;
-  tile_sum(acc, ts, g.buf, 0);
-  group_sums(F, lt, 1, ts, g.buf, g.n);
-  g.buf ^= 1;
+  tile_partial(acc, F, lt, sh, seg_n);
 }
 __global__ void __launch_bounds__(TILE) k_norm(const FineCase* FC, MState* ST, const int2* tiles, const int* count) {
   __shared__ double sh[32];
-  __shared__ TileSums ts;
   TILE_RANGE
   int cached_ = -1;  // case whose descriptor is in shared memory
   Seg g;
@@ -2464,7 +2393,7 @@ __global__ void __launch_bounds__(TILE) k_norm(const FineCase* FC, MState* ST, c
       close_seg(FC, ST, g, sh, FinNorm());
       g.ci = t.x;
     }
-    b_norm(FC, ST, t, cached_, ts, g);
+    b_norm(FC, ST, t, cached_, sh, g.n);
   }
   close_seg(FC, ST, g, sh, FinNorm());
 }
@@ -2754,7 +2683,7 @@ int build_case(cfdg_grid* G, CaseState& cs) {
     }
   }
   F.ntiles = (h.n[1] * h.n[2] + RT - 1) / RT;  // row tiles (one reduction partial each)
-  if (int e = A.alloc(&F.partials, (size_t)F.ntiles)) return e;
+  if (int e = A.alloc(&F.partials, (size_t)F.ntiles * (TILE / 32))) return e;
   cs.ngroups0 = M0.groups.rows();
   F.ngroups = cs.ngroups0;
   F.wbc = G->ncomp_groups == 0 ? 1 : 0;
