@@ -683,5 +683,5 @@ def autotune(device_grids, u_ptrs, p_ptrs, reset, dts, tol=1e-8, max_iter=10000,
     def key(c):
         return ",".join(str(v) for v in c)
 
-    return {"choice": list(choice), "ms": {key(c): round(1e3 * t, 2) for c, t in timing.items()},
+    return {"choice": list(choice), "ms": {key(c): round(1e3 * t, 4) for c, t in timing.items()},
             "iterations": {key(c): round(v, 2) for c, v in iters.items()}, "sweep_tile": tile}
