@@ -2123,6 +2123,8 @@ __device__ __forceinline__ void terminal_block(const CLev& L, int bk, int ln) {
   if (ln < n) L.x[ix[ln]] = (float)((a0 + a1) + (a2 + a3));
 }
 
+#include "coarse_cluster.cuh"
+
 // Levels l0 .. of case C, down to the terminal level and back up to l0.
 __device__ void blk_cycle(const CCase& C, int l0, int nu, double* sh) {
   int l = l0;
@@ -2183,6 +2185,9 @@ __device__ void blk_cycle(const CCase& C, int l0, int nu, double* sh) {
   }
 }
 
+// PART 0: the whole cycle of the cases in the table. PART 1 and 2: the way down and the way up
+// over the levels above the first one that k_coarse_cluster runs (the table holds no others).
+template <int PART>
 __global__ void __launch_bounds__(512, 2) k_coarse_all(const CCase* cases, const MState* ST, const CoarseTab* Tp) {
   const CoarseTab T = *Tp;
   __shared__ double sh[32];
@@ -2198,11 +2203,11 @@ __global__ void __launch_bounds__(512, 2) k_coarse_all(const CCase* cases, const
   if (threadIdx.x == 0) some = 0;
   __syncthreads();
   for (int ci = threadIdx.x; ci < nc; ci += blockDim.x)
-    if (active(ST, ci)) some = 1;
+    if (active(ST, ci) && __ldg(&T.rows[ci + 1]) > __ldg(&T.rows[ci])) some = 1;
   __syncthreads();
   if (!some) return;
   const int gl = min(T.nlev, T.lb);  // levels 0 .. gl-1 grid-wide
-  for (int l = 0; l < gl; ++l) {
+  for (int l = 0; PART != 2 && l < gl; ++l) {
     load_levels(cases, nc, l, MAXL, sl);
     if (T.anyg[l]) g_center(sl, ST, T, l, 0, sh, grid);
     {
@@ -2284,14 +2289,15 @@ __global__ void __launch_bounds__(512, 2) k_coarse_all(const CCase* cases, const
     }
     grid.sync();
   }
-  if (gl < T.nlev) {
+  if (PART == 0 && gl < T.nlev) {
     // The remaining levels of every case inside one block each.
     for (int ci = blockIdx.x; ci < nc; ci += gridDim.x)
-      if (active(ST, ci) && cases[ci].nl > gl) blk_cycle(cases[ci], gl, T.nu, sh);
+      if (active(ST, ci) && cases[ci].nl > gl && __ldg(&T.rows[ci + 1]) > __ldg(&T.rows[ci]))  // in the table
+        blk_cycle(cases[ci], gl, T.nu, sh);
     __threadfence();
     grid.sync();
   }
-  for (int l = min(T.nlev - 2, gl - 1); l >= 0; --l) {
+  for (int l = PART == 0 ? min(T.nlev - 2, gl - 1) : PART == 2 ? gl - 1 : -1; l >= 0; --l) {
     load_levels(cases, nc, l, MAXL, sl);
     {
       const int* off = T.live + l * (nc + 1);
@@ -2487,6 +2493,7 @@ struct CaseState {
   Arena arena;
   FineCase F{};
   CCase C{};
+  ClCase cl{};  // on: the coarse levels from cl.lc run on a cluster of their own
   std::vector<std::vector<int32_t>> colors;  // per coarse level: colour offsets (host copy)
   struct LevelStats {
     long long rows, nnz, ell, groups, blocks;
@@ -2519,6 +2526,18 @@ Csr permute_csr(const Csr& a, const std::vector<int32_t>& prow, const std::vecto
     }
   }
   return out;
+}
+
+// The direction 0..5 (x-lo, x-hi, y-lo, y-hi, z-lo, z-hi) from bin a to a face neighbour b, or -1.
+int bin_dir(const std::array<int32_t, 3>& a, const std::array<int32_t, 3>& b) {
+  int dir = -1, steps = 0;
+  for (int q = 0; q < 3; ++q) {
+    const int d = b[q] - a[q];
+    steps += std::abs(d);
+    if (d == -1) dir = 2 * q;
+    if (d == 1) dir = 2 * q + 1;
+  }
+  return steps == 1 ? dir : -1;
 }
 
 // cuTensorMapEncodeTiled, fetched from the driver (the library links only the runtime).
@@ -2554,6 +2573,99 @@ bool encode_split(CUtensorMap& m, const void* base, bool u16, int nxh, int rows,
   return enc(&m, u16 ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(base), dims,
              strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// A bin level of the hierarchy for plan_cluster: its bins per axis and the types of its rows
+// (coarse_cluster.cuh ClRow), one per row of the bin layout.
+struct BinMatrix {
+  int nb[3] = {0, 0, 0}, nbh = 0, h = 0;
+  std::vector<uint16_t> type;                  // [2h]
+  std::vector<std::array<uint32_t, 12>> tab;
+};
+constexpr int CL_TYPES = 2048;  // more types than this: the level is not planned as a bin level
+
+// Plans k_coarse_cluster for a case whose coarse levels allow it (aggregation levels of at
+// most two colours without closed groups) and uploads what it needs; bins[l] holds the bin
+// levels among levels 1.. (h == 0: not a bin level). Levels are split over the cluster's
+// blocks while their layers fill at least three quarters of them and a split phase beats one
+// block's (about 1,200 rows), or while one block would be slow (above 2,500 rows); levels
+// without a bin layout are split above 1,500 rows. The cluster starts at the first level
+// whose slabs fit the blocks' registers and shared memory; a level split by rows is taken up
+// to 32,768 of them (four a thread).
+int plan_cluster(Arena& A, cudaStream_t s, const CCase& C, const std::vector<int>& jacobi, const std::vector<BinMatrix>& bins,
+                 float alpha, ClCase& K) {
+  K = ClCase{};
+  for (int l = 1; l <= C.nl; ++l)
+    if (C.lv[l - 1].ngroups || jacobi[l] || C.lv[l - 1].ncolors > 2) return 0;
+  for (int lc = 1; lc <= C.nl; ++lc) {
+    ClCase T{};
+    T.lc = lc - 1;
+    T.alpha = alpha;
+    while (T.nb < CLB && lc + T.nb < C.nl && bins[lc + T.nb].h > 0) ++T.nb;
+    T.ng = C.nl - lc + 1 - T.nb;
+    for (int t = 0; t < T.nb; ++t) {
+      const BinMatrix& M = bins[lc + t];
+      if ((M.nb[2] >= 3 * CLS / 4 && 2 * M.h > 1200) || 2 * M.h > 2500) T.nd = t + 1;
+    }
+    if (T.nd > 0)
+      for (int r = 0; r <= CLS; ++r) T.slab[r] = r * bins[lc + T.nd - 1].nb[2] / CLS;
+    size_t at = 0;
+    auto take = [&](size_t bytes) {
+      const size_t o = at;
+      at += (bytes + 15) / 16 * 16;
+      return (int)o;
+    };
+    bool ok = true;
+    for (int t = 0; t < T.nb && ok; ++t) {
+      const BinMatrix& M = bins[lc + t];
+      ClBin& B = T.b[t];
+      B.nby = M.nb[1], B.nbz = M.nb[2], B.nbh = M.nbh, B.h = M.h, B.plane = M.nb[1] * M.nbh;
+      auto magic = [](int d) { return (unsigned)((((uint64_t)1 << 32) + d - 1) / d); };
+      B.mh = magic(B.nbh), B.my = magic(B.nby);
+      B.layers = B.nbz;
+      if (t < T.nd) {
+        B.layers = 0;
+        for (int r = 0; r < CLS; ++r) {
+          const int sh = T.nd - 1 - t;
+          B.layers = std::max(B.layers, std::min(T.slab[r + 1] << sh, B.nbz) - std::min(T.slab[r] << sh, B.nbz));
+        }
+      }
+      const size_t rows = (size_t)B.layers * B.plane;
+      ok = (uint64_t)rows * B.nbh < ((uint64_t)1 << 32);  // cl_div
+      B.x = take(2 * (rows + 2 * B.plane) * 4);
+      B.ntypes = (int)M.tab.size();
+      B.tab = take(48 * M.tab.size());
+      B.rhs = B.type = -1;
+      if (t > 0 || T.nd == 0 || rows > (size_t)CLR * CLT) B.rhs = take(2 * rows * 4), B.type = take(2 * rows * 2);
+      const CLev& L = C.lv[lc + t - 1];
+      B.grhs = L.rhs, B.gx = L.x, B.gres = L.res;
+    }
+    for (int t = T.nb; t < T.nb + T.ng && ok; ++t) {
+      const CLev& L = C.lv[lc + t - 1];
+      if (T.nb == T.nd && t == T.nb + T.ndl && !L.terminal && L.n > 1500) {
+        ok = L.n <= 32768;
+        ++T.ndl;
+        continue;
+      }
+      ok = t < MAXL && L.n <= 4096;
+      T.gx[t] = take((size_t)L.n * 4), T.grhs[t] = take((size_t)L.n * 4);
+    }
+    if (!ok || at > (size_t)CL_SMEM) continue;
+    T.smem = (int)at;
+    T.on = 1;
+    for (int t = 0; t < T.nb; ++t) {
+      ClBin& B = T.b[t];
+      unsigned short* dt;
+      std::array<uint32_t, 12>* dr;
+      if (int e = A.upload(&dt, bins[lc + t].type, s)) return e;
+      if (int e = A.upload(&dr, bins[lc + t].tab, s)) return e;
+      B.gtype = dt;
+      B.gtab = reinterpret_cast<const float4*>(dr);
+    }
+    K = T;
+    return 0;
+  }
+  return 0;
 }
 
 // Builds the FP32 device copy of a grid's hierarchy for the mixed form (cached on the grid).
@@ -2750,7 +2862,7 @@ int build_case(cfdg_grid* G, CaseState& cs) {
     B.on = ok;
     if (!ok) B.slot.clear(), B.bin.clear();
   };
-  if (G->mx_bins && H.masked && M0.groups.rows() == 0 && F.uniform && !(F.nxh & 1) && H.levels.size() >= 3) {
+  if (G->mx_bins && H.masked && M0.groups.rows() == 0 && F.uniform && H.levels.size() >= 3) {
     bool ok = (int64_t)M0.prolong.rows() == (int64_t)F.N;
     for (int c = 0; c < F.N && ok; ++c) {
       const int n = M0.prolong.off[c + 1] - M0.prolong.off[c];
@@ -3096,6 +3208,75 @@ int build_case(cfdg_grid* G, CaseState& cs) {
     }
   }
   if (int e = A.alloc(&C.gpart, (size_t)maxg * CS)) return e;
+  {
+    std::vector<BinMatrix> bins(C.nl + 1);
+    for (int l = 1; l < C.nl && binl[l].on; ++l) {
+      const BinLevel& B = binl[l];
+      BinMatrix& M = bins[l];
+      const size_t n = 2 * (size_t)B.h;
+      const int plane = B.nb[1] * B.nbh;
+      if (plane > 32767) break;  // offsets are 16-bit
+      const MgLevel& src = H.levels[l];
+      const MgLevel& fine = H.levels[l - 1];
+      std::map<std::array<uint32_t, 12>, int> index;
+      std::vector<int> agg(n, -1);
+      for (int a = 0; a < src.n; ++a) agg[B.slot[a]] = a;
+      auto word = [](float f) {
+        uint32_t w;
+        std::memcpy(&w, &f, 4);
+        return w;
+      };
+      bool ok = true;
+      M.type.assign(n, 0);
+      for (size_t row = 0; row < n && ok; ++row) {
+        std::array<uint32_t, 12> r{};
+        int16_t off[6] = {0, 0, 0, 0, 0, 0};
+        unsigned order = 0xe4;  // children 0, 1, 2, 3
+        if (const int a = agg[row]; a >= 0) {
+          const auto& bin = B.bin[a];
+          const int par = bin[0] & 1;
+          const int offs[6] = {par - 1, par, -B.nbh, B.nbh, -plane, plane};
+          int m = 0;
+          for (int k = src.a.off[a]; k < src.a.off[a + 1] && ok; ++k, ++m) {
+            const int dir = bin_dir(bin, B.bin[src.a.col[k]]);
+            ok = m < 6 && dir >= 0;
+            if (!ok) break;
+            r[m] = word((float)src.a.val[k]);
+            off[m] = (int16_t)offs[dir];
+          }
+          r[6] = word((float)src.diag[a]);
+          r[7] = word(src.diag[a] == 0.0 ? 0.0f : 1.0f / (float)src.diag[a]);
+          if (l > 1 && ok) {
+            // The colour-0 children (of the bins of the level below) in the restriction's order,
+            // then those that are empty.
+            unsigned seen = 0;
+            int at = 0;
+            order = 0;
+            for (int k = fine.restrict.off[a]; k < fine.restrict.off[a + 1]; ++k) {
+              const auto& cb = binl[l - 1].bin[fine.restrict.col[k]];
+              if ((cb[0] + cb[1] + cb[2]) & 1) continue;
+              const unsigned pos = 2 * (cb[2] & 1) + (cb[1] & 1);
+              order |= pos << (2 * at++);
+              seen |= 1u << pos;
+            }
+            for (unsigned pos = 0; pos < 4; ++pos)
+              if (!(seen >> pos & 1u)) order |= pos << (2 * at++);
+          }
+        }
+        for (int m = 0; m < 3; ++m)
+          r[8 + m] = (uint32_t)(uint16_t)off[2 * m] | (uint32_t)(uint16_t)off[2 * m + 1] << 16;
+        r[11] = order;
+        const auto it = index.emplace(r, (int)M.tab.size());
+        if (it.second) M.tab.push_back(r);
+        M.type[row] = (uint16_t)it.first->second;
+        ok = ok && M.tab.size() <= CL_TYPES;
+      }
+      if (!ok) break;
+      for (int a = 0; a < 3; ++a) M.nb[a] = B.nb[a];
+      M.nbh = B.nbh, M.h = B.h;
+    }
+    if (int e = plan_cluster(A, s, C, ljacobi, bins, alpha, cs.cl)) return e;
+  }
   F.n1 = C.lv[0].n;
   F.rhs1 = C.lv[0].rhs;
   F.x1 = C.lv[0].x;
@@ -3159,9 +3340,17 @@ struct cfdg_batch {
   bool any_groups = false;
   bool any_bin1 = false;  // some case has its level 1 as the bin grid
   // Coarse-level phase tables (device), refilled for each active set.
-  CoarseTab h_tab{};
-  CoarseTab* d_tab = nullptr;
-  int* tab_buf = nullptr;
+  // [0] the cases whose coarse levels all run in the grid-wide phases, [1] the levels above
+  // the first cluster level of the others.
+  CoarseTab h_tab[2]{};
+  CoarseTab* d_tab[2] = {nullptr, nullptr};
+  int* tab_buf[2] = {nullptr, nullptr};
+  bool any_tab[2] = {false, false};
+  // The cluster kernel's cases, and the shared memory the largest of them asks for.
+  ClCase* d_cl = nullptr;
+  std::vector<char> clustered;
+  bool any_cl = false;
+  int cl_smem = 0;
   int nlev_all = 0;
   int coop_blocks = 0;
   bool coop = true;
@@ -3294,10 +3483,12 @@ int fill_lists(cfdg_batch* B, WorkLists& W, const std::vector<char>& on, cudaStr
   return 0;
 }
 
-// Coarse phase tables for the active cases (inactive ones contribute no rows).
-int fill_tab(cfdg_batch* B, const std::vector<char>& on, cudaStream_t s) {
+// Coarse phase tables of the cases in `on` (the others contribute no rows). which 0: all their
+// levels; 1: those above the first cluster level.
+int fill_tab(cfdg_batch* B, int which, const std::vector<char>& on, cudaStream_t s) {
   const int nc = (int)B->cases.size(), nlev = B->nlev_all, w = nc + 1;
-  CoarseTab& T = B->h_tab;
+  CoarseTab& T = B->h_tab[which];
+  auto depth = [&](int i) { return which ? B->cases[i]->cl.lc : B->cases[i]->C.nl; };
   static thread_local std::vector<int32_t> buf;
   const size_t words = (size_t)nlev * w * (6 + 2 * MAXC);
   buf.assign(words, 0);
@@ -3316,17 +3507,17 @@ int fill_tab(cfdg_batch* B, const std::vector<char>& on, cudaStream_t s) {
   for (int l = nlev - 1; l >= 0; --l) {
     long long most = 0;
     for (int i = 0; i < nc; ++i)
-      if (on[i] && l < B->cases[i]->C.nl) {
+      if (on[i] && l < depth(i)) {
         const auto& st = B->cases[i]->stats[l];
         most = std::max(most, st.rows + st.ell);
       }
-    if (most > BLK_WORK) break;
+    if (most > BLK_WORK || which) break;
     T.lb = l;
   }
   for (int l = 0; l < nlev; ++l) {
     int maxc = 0, anyg = 0;
     auto lev = [&](int i) -> const CLev* {
-      return on[i] && l < B->cases[i]->C.nl ? &B->cases[i]->C.lv[l] : nullptr;
+      return on[i] && l < depth(i) ? &B->cases[i]->C.lv[l] : nullptr;
     };
     for (int i = 0; i < nc; ++i)
       if (const CLev* L = lev(i)) {
@@ -3363,7 +3554,7 @@ int fill_tab(cfdg_batch* B, const std::vector<char>& on, cudaStream_t s) {
       }
     }
   }
-  T.rows = B->tab_buf;
+  T.rows = B->tab_buf[which];
   T.term = T.rows + nlev * w;
   T.next = T.term + nlev * w;
   T.live = T.next + nlev * w;
@@ -3371,42 +3562,75 @@ int fill_tab(cfdg_batch* B, const std::vector<char>& on, cudaStream_t s) {
   T.res = T.grp + nlev * w;
   T.fwd = T.res + nlev * w;
   T.bwd = T.fwd + (size_t)nlev * MAXC * w;
-  if (int e = staged_h2d(B, B->tab_buf, buf.data(), words * sizeof(int32_t), s)) return e;
-  return staged_h2d(B, B->d_tab, &T, sizeof(CoarseTab), s);
+  if (int e = staged_h2d(B, B->tab_buf[which], buf.data(), words * sizeof(int32_t), s)) return e;
+  return staged_h2d(B, B->d_tab[which], &T, sizeof(CoarseTab), s);
 }
 
 // The graph's lists and tables cover the cases marked in B->active.
 int set_active(cfdg_batch* B, cudaStream_t s) {
   if (int e = fill_lists(B, B->run, B->active, s)) return e;
-  return fill_tab(B, B->active, s);
+  for (int which = 0; which < 2; ++which) {
+    if (!B->any_tab[which]) continue;
+    std::vector<char> on(B->active);
+    for (size_t i = 0; i < on.size(); ++i)
+      on[i] = on[i] && (which ? B->clustered[i] && B->cases[i]->cl.lc > 0 : !B->clustered[i]);
+    if (int e = fill_tab(B, which, on, s)) return e;
+  }
+  return 0;
 }
 
-void launch_coarse(cfdg_batch* B, cudaStream_t s) {
-  if (B->coop) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)B->coop_blocks, 1, 1);
-    cfg.blockDim = dim3(512, 1, 1);
-    cfg.dynamicSmemBytes = 2 * B->cases.size() * sizeof(CLev);
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k_coarse_all, (const CCase*)B->d_cc, (const MState*)B->d_st, (const CoarseTab*)B->d_tab);
-    return;
-  }
+// A cooperative launch of the grid-wide phases over table `which`.
+template <int PART>
+void launch_phases(cfdg_batch* B, int which, cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(B->cases.size() * B->csize), 1, 1);
-  cfg.blockDim = dim3(CT, 1, 1);
+  cfg.gridDim = dim3((unsigned)B->coop_blocks, 1, 1);
+  cfg.blockDim = dim3(512, 1, 1);
+  cfg.dynamicSmemBytes = 2 * B->cases.size() * sizeof(CLev);
   cfg.stream = s;
   cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, k_coarse_all<PART>, (const CCase*)B->d_cc, (const MState*)B->d_st,
+                     (const CoarseTab*)B->d_tab[which]);
+}
+
+// A launch of clusters of `size` blocks, one cluster per case.
+void cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, unsigned cases, unsigned size, unsigned threads,
+                    size_t smem, cudaStream_t s) {
+  cfg = {};
+  cfg.gridDim = dim3(cases * size, 1, 1);
+  cfg.blockDim = dim3(threads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
   at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = (unsigned)B->csize;
+  at[0].val.clusterDim.x = size;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
+}
+
+// The coarse levels of every case: one cluster per case where its levels allow it
+// (k_coarse_cluster), the grid-wide phases for the levels above it and for the other cases.
+void launch_coarse(cfdg_batch* B, cudaStream_t s) {
+  const unsigned nc = (unsigned)B->cases.size();
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute at[1];
+  if (B->any_tab[1]) launch_phases<1>(B, 1, s);
+  if (B->any_cl) {
+    cluster_config(cfg, at, nc, CLS, CLT, B->cl_smem, s);
+    cudaLaunchKernelEx(&cfg, k_coarse_cluster, (const ClCase*)B->d_cl, (const CCase*)B->d_cc, (const MState*)B->d_st,
+                       B->nuc);
+  }
+  if (B->any_tab[1]) launch_phases<2>(B, 1, s);
+  if (!B->any_tab[0]) return;
+  if (B->coop) {
+    launch_phases<0>(B, 0, s);
+    return;
+  }
+  cluster_config(cfg, at, nc, B->csize, CT, 0, s);
   cudaLaunchKernelEx(&cfg, k_coarse, (const CCase*)B->d_cc, (const MState*)B->d_st, B->nuc);
 }
 
@@ -3672,24 +3896,62 @@ int cfdg_mixed_pack(cfdg_batch* B) {
   CU(cudaMemcpyAsync(B->d_st, idle.data(), sizeof(MState) * nc, cudaMemcpyHostToDevice, s));
   if (B->h_st) cudaFreeHost(B->h_st);
   CU(cudaMallocHost((void**)&B->h_st, sizeof(MState) * nc));
-  if (int e = A.alloc(&B->tab_buf, (size_t)B->nlev_all * (nc + 1) * (6 + 2 * MAXC) + 1)) return e;
-  if (int e = A.alloc(&B->d_tab, 1)) return e;
-  B->active.assign(nc, 1);
-  if (int e = set_active(B, s)) return e;
   // Grid of the cooperative coarse-level kernel: all blocks co-resident.
   {
     int dev = 0, sms = 0, per = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const size_t dsm = 2 * (size_t)nc * sizeof(CLev);
-    if (dsm > 48 * 1024) cudaFuncSetAttribute(k_coarse_all, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsm);
     B->coop = true;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_coarse_all, 512, dsm) != cudaSuccess || per < 1) {
-      cudaGetLastError();
-      B->coop = false;
+    for (const void* fn : {(const void*)k_coarse_all<0>, (const void*)k_coarse_all<1>, (const void*)k_coarse_all<2>}) {
+      if (dsm > 48 * 1024) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsm);
+      int one = 0;
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&one, fn, 512, dsm) != cudaSuccess || one < 1) {
+        cudaGetLastError();
+        B->coop = false;
+      }
+      per = per ? std::min(per, one) : one;
     }
     B->coop_blocks = sms * std::max(1, std::min(per, 4));
   }
+  // Which cases run their coarse levels on clusters: all that have a plan, when such a cluster
+  // fits the device (and, for those with levels above it, the cooperative launch).
+  {
+    std::vector<ClCase> cl(nc);
+    B->cl_smem = 0;
+    for (int i = 0; i < nc; ++i) {
+      const ClCase& K = B->cases[i]->cl;
+      if (K.on && (K.lc == 0 || B->coop)) cl[i] = K;
+      B->cl_smem = std::max(B->cl_smem, cl[i].smem);
+    }
+    int clusters = 0;
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute at[1];
+    cluster_config(cfg, at, 1, CLS, CLT, B->cl_smem, s);
+    if (cudaFuncSetAttribute(k_coarse_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaFuncSetAttribute(k_coarse_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, CL_SMEM) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&clusters, k_coarse_cluster, &cfg) != cudaSuccess || clusters < 1) {
+      cudaGetLastError();
+      for (ClCase& K : cl) K = ClCase{};
+    }
+    B->clustered.assign(nc, 0);
+    B->any_cl = B->any_tab[0] = B->any_tab[1] = false;
+    for (int i = 0; i < nc; ++i) {
+      B->clustered[i] = cl[i].on != 0;
+      B->any_cl |= cl[i].on != 0;
+      B->any_tab[0] |= !cl[i].on;
+      B->any_tab[1] |= cl[i].on && cl[i].lc > 0;
+    }
+    if (int e = A.upload(&B->d_cl, cl, s)) return e;
+    CU(cudaStreamSynchronize(s));
+  }
+  for (int which = 0; which < 2; ++which) {
+    if (!B->any_tab[which]) continue;
+    if (int e = A.alloc(&B->tab_buf[which], (size_t)B->nlev_all * (nc + 1) * (6 + 2 * MAXC) + 1)) return e;
+    if (int e = A.alloc(&B->d_tab[which], 1)) return e;
+  }
+  B->active.assign(nc, 1);
+  if (int e = set_active(B, s)) return e;
   if (!B->coop) {
     // One cluster per case: 16 CTAs when that non-portable size is allowed, else 8.
     B->csize = CS;
@@ -4040,7 +4302,8 @@ int64_t cfdg_batch_stats_json(cfdg_batch* B, char* buf, int64_t cap) {
   snprintf(tmp, sizeof tmp,
            "{\"coarse_kernel\": \"%s\", \"coarse_blocks\": %d, \"staged_sweeps\": %s, \"sweep_blocks\": %d, "
            "\"sweep_rows\": %d, \"sweep_stages\": %d, \"cases\": [",
-           B->coop ? "cooperative" : "cluster", B->coop ? B->coop_blocks : (int)B->cases.size() * B->csize,
+           !B->any_tab[0] || !B->coop ? "cluster" : "cooperative",
+           !B->any_tab[0] ? (int)B->cases.size() * CLS : B->coop ? B->coop_blocks : (int)B->cases.size() * B->csize,
            B->rb_tma ? "true" : "false", B->rb_tma ? B->rb_grid : B->g_fine, B->rb_tma ? B->rb_sr : RT,
            B->rb_tma ? B->rb_ns : 0);
   std::string out = tmp;

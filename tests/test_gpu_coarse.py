@@ -1,0 +1,66 @@
+"""The coarse levels of the mixed form on one thread-block cluster per case, against the
+grid-wide phases over index lists (cfdg_grid_set_coarse_layout 0): the same projected bits
+and iterations, alone and in a batch. Shapes at the edges of the split: layers that do not
+divide among the blocks, a split over fewer layers than blocks, levels of one block only,
+odd bin rows, sweep counts other than two, a first level too large for a cluster, and a
+grid whose weights are not powers of two."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def bits(a):
+    return np.ascontiguousarray(a, np.float64).view(np.uint64)
+
+
+def solve(pkg, grids, us, bins, cycle):
+    dgs = [pkg.pressure.DeviceGrid(g, preconditioner="multigrid", precision="mixed") for g in grids]
+    for d in dgs:
+        d.set_coarse_layout(bins)
+        d.set_cycle(*cycle)
+    alone = []
+    for d, g, u in zip(dgs, grids, us):
+        uu, pp = u.copy(), np.zeros(g.count)
+        info = d.project(uu, pp, 0.1, 1e-8, 10000)
+        alone.append((uu, pp, info.iterations))
+    batch = pkg.pressure.Batch(dgs)
+    kernel = batch.stats()["coarse_kernel"]
+    bu, bp = [u.copy() for u in us], [np.zeros(g.count) for g in grids]
+    res = batch.project(bu, bp, [0.1] * len(grids), 1e-8, 10000)
+    batch.close()
+    for d in dgs:
+        d.close()
+    for (uu, pp, it), u, p, (code, info) in zip(alone, bu, bp, res):
+        assert code == 0 and info.iterations == it
+        assert np.array_equal(bits(uu), bits(u)) and np.array_equal(bits(pp), bits(p))
+    return alone, kernel
+
+
+SHAPES = {
+    "uneven layers": [((64, 48, 50), 2.0, 5), ((40, 36, 27), 2.0, 2)],
+    "odd rows": [((37, 29, 33), 1.5, 3), ((50, 42, 26), 2.5, 3)],
+    "one block": [((24, 20, 16), 2.0, 1), ((12, 10, 8), 2.0, 0)],
+    "thin": [((96, 80, 10), 2.0, 4), ((30, 8, 60), 2.0, 0)],
+    "three levels split": [((128, 96, 64), 2.0, 12)],
+    "grid-wide first level": [((176, 160, 80), 2.0, 10), ((48, 48, 48), 2.0, 3)],
+}
+
+
+@pytest.mark.parametrize("cycle", [(2, 2), (1, 3)])
+@pytest.mark.parametrize("name", list(SHAPES))
+def test_cluster_levels_give_the_grid_wide_bits(pkg, name, cycle):
+    if cycle != (2, 2) and name == "grid-wide first level":
+        pytest.skip("one cycle is enough at this size")
+    rng = np.random.default_rng(len(name))
+    cases = [pkg.synth.case(n, dx, inflow=5.0, preconditioner="multigrid",
+                            boxes=pkg.synth.random_boxes(rng, nb, [dx * v for v in n], side=(6.0, 20.0), dx=dx))
+             for n, dx, nb in SHAPES[name]]
+    grids = [pkg.grid.Grid.build(c) for c in cases]
+    us = [pkg.synth.random_velocity(g, 70 + i) for i, g in enumerate(grids)]
+    lists, _ = solve(pkg, grids, us, False, cycle)
+    bins, kernel = solve(pkg, grids, us, True, cycle)
+    assert kernel == "cluster"
+    for a, b in zip(lists, bins):
+        assert a[2] == b[2]
+        assert np.array_equal(bits(a[0]), bits(b[0])) and np.array_equal(bits(a[1]), bits(b[1]))
