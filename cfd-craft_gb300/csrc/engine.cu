@@ -630,7 +630,11 @@ struct GridBarrier {
 struct ClusterBarrier {
   __device__ void sync() { cg::this_cluster().sync(); }
 };
-constexpr int PC_CLUSTER = 8;  // blocks of the plain coarse-level cluster (portable size)
+constexpr int PC_CLUSTER = 8;  // blocks of that cluster (portable size)
+
+}  // namespace
+#include "plain_cluster.cuh"
+namespace {
 
 // The banded forward and backward substitutions of one block (multigrid/line.rs:172-185)
 // for a half-bandwidth BW: the last BW results stay in registers and the factor entries of
@@ -1061,6 +1065,24 @@ void launch_gs(cfdg_grid* G, DevLevel& L, bool backward, const Scalars* S, bool 
   }
 }
 
+// A launch of the coarse-level cluster over the plan of H (plain_cluster.cuh).
+void launch_plain_cluster(cfdg_grid* G, const DevHierarchy& H, int from, int what, const Scalars* S) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(PCS, 1, 1);
+  cfg.blockDim = dim3(PCT, 1, 1);
+  cfg.dynamicSmemBytes = (size_t)H.pc_smem;
+  cfg.stream = G->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = PCS;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, k_plain_cluster, (const PcPlan*)H.d_pc, from - 1, what, S);
+  tick(G);
+}
+
 // One symmetric V(2,2) cycle, z = M^-1 r (multigrid.rs:656-726, masked.rs:292-342).
 void launch_vcycle(cfdg_grid* G, const double* r, double* z, const Scalars* S) {
   DevHierarchy& H = *G->mg;
@@ -1076,13 +1098,17 @@ void launch_vcycle(cfdg_grid* G, const double* r, double* z, const Scalars* S) {
   }
   const int nl = (int)H.levels.size();
   // Levels 1 .. L-1 in one cooperative launch when available, else level by level.
-  const bool coop = (H.coop_blocks > 0 || H.cluster) && nl > 1;
-  const int first = H.coop0 ? 0 : 1;  // the first level of the cooperative launch
+  const bool coop = (H.coop_blocks > 0 || H.cluster || H.pc_rest > 0) && nl > 1;
+  // The first level of the cooperative launch, or of the cluster plan's whole cycle.
+  const int first = H.pc_rest > 0 ? H.pc_rest : H.coop0 ? 0 : 1;
   for (int l = 0; l < (coop ? first : nl); ++l) {
     DevLevel& L = H.levels[l];
     const bool full = l == 0 && H.full0;
+    const bool planned = l > 0 && H.pc_rest > 0;  // no groups, not terminal
     launch_center(G, L.groups, L.ngroups, L.rhs, S);
-    k_fill<<<grid_blocks(L.n), BLOCK, 0, s>>>(L.x, 0.0, L.n, S); tick(G);
+    if (!planned) {
+      k_fill<<<grid_blocks(L.n), BLOCK, 0, s>>>(L.x, 0.0, L.n, S); tick(G);
+    }
     if (L.terminal) {
       if (L.nblocks > 0) {
         k_direct<<<(L.nblocks + 63) / 64, 64, 0, s>>>(L.nblocks, L.d_ioff, L.d_idx, L.d_foff, L.d_fac, L.rhs, L.x, S); tick(G);
@@ -1090,8 +1116,12 @@ void launch_vcycle(cfdg_grid* G, const double* r, double* z, const Scalars* S) {
       launch_center(G, L.groups, L.ngroups, L.x, S);
       break;
     }
-    launch_gs(G, L, false, S, full);
-    launch_gs(G, L, false, S, full);
+    if (planned) {
+      launch_plain_cluster(G, H, l, 0, S);
+    } else {
+      launch_gs(G, L, false, S, full);
+      launch_gs(G, L, false, S, full);
+    }
     launch_center(G, L.groups, L.ngroups, L.x, S);
     if (full) {
       if (G->uniform) k_residual_struct<true><<<grid_blocks(L.n), BLOCK, 0, s>>>(G->g, L.diag, L.rhs, L.x, L.res, L.n, S);
@@ -1105,9 +1135,12 @@ void launch_vcycle(cfdg_grid* G, const double* r, double* z, const Scalars* S) {
     k_restrict<<<grid_blocks(C.n), BLOCK, 0, s>>>(C.n, L.restrict_.off, L.restrict_.col, L.restrict_.val, L.res,
                                                   C.rhs, S); tick(G);
   }
-  if (coop) {
-    // One cluster of PC_CLUSTER blocks (cluster barriers, about 0.3 us a phase), or the
-    // cooperative grid where clusters cannot be launched.
+  if (H.pc_rest > 0) {
+    launch_plain_cluster(G, H, H.pc_rest, 2, S);
+  } else if (coop) {
+    // Block-smoothed hierarchies and levels with closed groups: one cluster of PC_CLUSTER
+    // blocks (cluster barriers, about 0.3 us a phase), or the cooperative grid where clusters
+    // cannot be launched.
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(BLOCK, 1, 1);
     cfg.stream = s;
@@ -1136,8 +1169,12 @@ void launch_vcycle(cfdg_grid* G, const double* r, double* z, const Scalars* S) {
     DevLevel& C = H.levels[l + 1];
     const bool full = l == 0 && H.full0;
     k_prolong<<<grid_blocks(L.n), BLOCK, 0, s>>>(L.n, L.prolong.off, L.prolong.col, L.prolong.val, C.x, L.x, S); tick(G);
-    launch_gs(G, L, true, S, full);
-    launch_gs(G, L, true, S, full);
+    if (l > 0 && H.pc_rest > 0) {
+      launch_plain_cluster(G, H, l, 1, S);
+    } else {
+      launch_gs(G, L, true, S, full);
+      launch_gs(G, L, true, S, full);
+    }
     launch_center(G, L.groups, L.ngroups, L.x, S);
   }
   if (H.masked && !H.full0) {
@@ -1380,6 +1417,182 @@ int mixed_host_hierarchy_impl(cfdg_grid* G, std::shared_ptr<Hierarchy>& out) {
   return 0;
 }
 
+// recip_of on the host (the same bits: both reciprocals are correctly rounded).
+double host_recip(double d) {
+  if (!(d >= 0x1p-60 && d <= 0x1p60)) return 0.0;
+  const double r = 1.0 / d;
+  return std::fabs(std::fma(r, d, -1.0)) <= 0x1p-54 ? r : -r;
+}
+
+// The cluster plan of levels 1.. (plain_cluster.cuh), where no level has closed groups or
+// block smoothing and their iterates fit a cluster's shared memory; else H keeps none.
+int plan_plain_cluster(DevHierarchy& D, const Hierarchy& H, cudaStream_t s) {
+  const int nl = (int)H.levels.size() - 1;
+  if (nl < 1 || nl > PC_MAXLEV) return 0;
+  PcPlan P{};
+  P.nl = nl;
+  int ndep = 0, rest = 0;
+  for (int l = 1; l <= nl; ++l) {
+    const MgLevel& M = H.levels[l];
+    if (M.groups.rows() || !M.lines.empty()) return 0;
+    if (D.levels[l].terminal != (l == nl)) return 0;
+    PcLev& L = P.lv[l - 1];
+    L.n = M.n;
+    L.terminal = l == nl;
+    if (!L.terminal) {
+      L.ndep = M.fwd.levels();
+      ndep = std::max(ndep, L.ndep);
+      L.solo = L.ndep > 0 && M.n <= PC_SOLO_ROWS * L.ndep;
+      for (int i = 0; i < M.n; ++i) L.w = std::max(L.w, M.a.off[i + 1] - M.a.off[i]);
+      if (L.w > 255) return 0;
+    } else {
+      L.solo = 1;
+    }
+    L.chunk = L.solo ? M.n : (M.n + PCS - 1) / PCS;
+    if (!L.solo && M.n > PC_GRID_ROWS && rest == l - 1) rest = l;  // levels 1 .. rest: transfers grid-wide
+  }
+  const int base = ((ndep + 1) * 4 + 15) / 16 * 16;
+  int at = base, most = base;
+  for (int l = 1; l <= nl; ++l) {
+    PcLev& L = P.lv[l - 1];
+    int& o = l <= rest ? most : at;
+    if (l <= rest) {  // alone in its launches
+      L.x = base;
+      L.rhs = base + 8 * (L.chunk + 1);
+      most = std::max(most, L.rhs + 8 * L.chunk);
+    } else {
+      if (L.chunk >= (PC_SMEM - o) / 16) return 0;
+      L.x = o;
+      L.rhs = o + 8 * (L.chunk + 1);
+      o = (L.rhs + 8 * L.chunk + 15) / 16 * 16;
+    }
+    if (most > PC_SMEM || at > PC_SMEM) return 0;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(PCS, 1, 1);
+  cfg.blockDim = dim3(PCT, 1, 1);
+  cfg.dynamicSmemBytes = (size_t)std::max(at, most);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = PCS;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int clusters = 0;
+  if (cudaFuncSetAttribute(k_plain_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+      cudaFuncSetAttribute(k_plain_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, PC_SMEM) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&clusters, k_plain_cluster, &cfg) != cudaSuccess || clusters < 1) {
+    cudaGetLastError();
+    return 0;
+  }
+  for (int l = 1; l <= nl; ++l) {
+    const MgLevel& M = H.levels[l];
+    const DevLevel& V = D.levels[l];
+    PcLev& L = P.lv[l - 1];
+    L.grhs = V.rhs, L.gx = V.x, L.gres = V.res;
+    if (L.terminal) {
+      L.nblocks = V.nblocks;
+      L.ioff = V.d_ioff, L.idx = V.d_idx, L.foff = V.d_foff, L.fac = V.d_fac;
+      std::vector<double> rd(M.direct_idx.col.size());
+      for (int b = 0; b < L.nblocks; ++b) {
+        const int n = M.direct_idx.off[b + 1] - M.direct_idx.off[b];
+        for (int i = 0; i < n; ++i)
+          rd[M.direct_idx.off[b] + i] = host_recip(M.direct_factor[M.direct_off[b] + (size_t)i * n + i]);
+      }
+      double* d;
+      if (int e = D.arena.upload(&d, rd, s)) return e;
+      L.frd = d;
+      CU(cudaStreamSynchronize(s));
+      continue;
+    }
+    L.roff = V.restrict_.off, L.rcol = V.restrict_.col, L.rval = V.restrict_.val;
+    L.poff = V.prolong.off, L.pcol = V.prolong.col, L.pval = V.prolong.val;
+    const int owners = L.solo ? 1 : PCS;
+    const size_t slots = (size_t)PCS * L.chunk;
+    std::vector<int> ls((size_t)PCS * (L.ndep + 1), 0), gid(slots, 0), pos(M.n), fill(PCS, 0);
+    // Positions: per owner (a contiguous range of rows) by dependency level, rows ascending.
+    for (int dep = 0; dep < L.ndep; ++dep) {
+      for (int o = 0; o < owners; ++o) ls[(size_t)o * (L.ndep + 1) + dep] = fill[o];
+      for (int q = M.fwd.start[dep]; q < M.fwd.start[dep + 1]; ++q) {
+        const int i = M.fwd.order[q], o = i / L.chunk;
+        pos[i] = fill[o];
+        gid[(size_t)o * L.chunk + fill[o]++] = i;
+      }
+    }
+    for (int o = 0; o < owners; ++o) ls[(size_t)o * (L.ndep + 1) + L.ndep] = fill[o];
+    const bool narrow = L.w <= PCW;
+    std::vector<PcRec> rec(narrow ? slots : 0);
+    const size_t wide = narrow ? 0 : slots;
+    std::vector<unsigned> col((size_t)L.w * wide, 0);
+    std::vector<double> val((size_t)L.w * wide, 0.0), diag(wide, 0.0), rd(wide, 0.0);
+    std::vector<unsigned short> cnt(wide, 0);
+    for (int i = 0; i < M.n; ++i) {
+      const int o = i / L.chunk;
+      const size_t at_i = (size_t)o * L.chunk + pos[i];
+      int low = 0;
+      const int b = M.a.off[i], n = M.a.off[i + 1] - b;
+      for (int a = 0; a < n; ++a) {
+        if (M.a.col[b + a] < i && a != low) return 0;  // lower neighbours come first in a row
+        low += M.a.col[b + a] < i;
+      }
+      const bool irregular = low > 3 || n - low > 3;
+      if (narrow) {
+        PcRec& r = rec[at_i];
+        r = PcRec{};
+        r.d = M.diag[i];
+        r.rd = host_recip(M.diag[i]);
+        r.irregular = irregular;
+        for (int a = 0; a < PCW; ++a) r.col[a] = (unsigned)o << 24 | (unsigned)(L.x + 8 * L.chunk);
+      } else {
+        diag[at_i] = M.diag[i];
+        rd[at_i] = host_recip(M.diag[i]);
+        cnt[at_i] = (unsigned short)n;
+      }
+      for (int a = 0; a < n; ++a) {
+        const int j = M.a.col[b + a];
+        const unsigned c = (unsigned)(j / L.chunk) << 24 | (unsigned)(L.x + 8 * pos[j]);
+        if (narrow) {
+          const int at_a = irregular || a < low ? a : 3 + a - low;
+          rec[at_i].col[at_a] = c;
+          rec[at_i].val[at_a] = M.a.val[b + a];
+        } else {
+          col[(size_t)a * slots + at_i] = c;
+          val[(size_t)a * slots + at_i] = M.a.val[b + a];
+        }
+      }
+    }
+    int *dls, *dgid;
+    if (int e = D.arena.upload(&dls, ls, s)) return e;
+    if (int e = D.arena.upload(&dgid, gid, s)) return e;
+    L.ls = dls, L.gid = dgid;
+    if (narrow) {
+      PcRec* dr;
+      if (int e = D.arena.upload(&dr, rec, s)) return e;
+      L.rec = dr;
+    } else {
+      unsigned* dcol;
+      double *dval, *ddiag, *drd;
+      unsigned short* dcnt;
+      if (int e = D.arena.upload(&dcol, col, s)) return e;
+      if (int e = D.arena.upload(&dval, val, s)) return e;
+      if (int e = D.arena.upload(&ddiag, diag, s)) return e;
+      if (int e = D.arena.upload(&drd, rd, s)) return e;
+      if (int e = D.arena.upload(&dcnt, cnt, s)) return e;
+      L.col = dcol, L.val = dval, L.diag = ddiag, L.rd = drd, L.cnt = dcnt;
+    }
+    CU(cudaStreamSynchronize(s));
+  }
+  PcPlan* dp = nullptr;
+  std::vector<PcPlan> one(1, P);
+  if (int e = D.arena.upload(&dp, one, s)) return e;
+  CU(cudaStreamSynchronize(s));
+  D.d_pc = dp;
+  D.pc_rest = rest + 1;
+  D.pc_smem = std::max(at, most);
+  return 0;
+}
+
 int build_mg_dev(cfdg_grid* G, const Poller& poll) {
   Hierarchy H;
   if (int e = build_hierarchy(G->h, poll, H)) {
@@ -1536,6 +1749,7 @@ int build_mg_dev(cfdg_grid* G, const Poller& poll) {
       }
       D->cluster = clusters > 0;
     }
+    if (int e = plan_plain_cluster(*D, H, s)) return e;
     if (D->coop0 && D->coop_blocks == 0 && !D->cluster)
       return fail(CFDG_ERR_UNSUPPORTED, "block-smoothed multigrid needs a co-resident cooperative launch");
   }

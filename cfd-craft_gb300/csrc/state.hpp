@@ -157,6 +157,11 @@ struct DevHierarchy {
   void* d_plev = nullptr;
   int coop_blocks = 0;
   bool cluster = false;  // the coarse kernel runs as one thread-block cluster (engine.cu)
+  // Levels 1.. on one cluster with their iterates in shared memory (plain_cluster.cuh): the
+  // plan, the first level whose whole cycle it runs (0: no plan; levels 1 .. pc_rest - 1 only
+  // sweep there) and the dynamic shared memory of a launch.
+  void* d_pc = nullptr;
+  int pc_rest = 0, pc_smem = 0;
   // Block-smoothed (anisotropic) hierarchies: d_plev starts at level 0 and the whole cycle
   // is the cooperative launch.
   bool coop0 = false;

@@ -38,3 +38,21 @@ def test_sweeps_bitwise_at_tile_edges(pkg, O, cells, faces, scale):
     for _ in range(2):
         assert np.array_equal(bits(dg.precondition(r)), bits(oz))
     dg.close()
+
+
+@pytest.mark.parametrize("cells, boxes", [((100, 92, 50), 6), ((60, 44, 24), 0), ((75, 61, 37), 4), ((34, 30, 18), 2)])
+def test_coarse_cluster_cycle_bitwise(pkg, O, cells, boxes):
+    """The plain cycle's coarse levels on one thread-block cluster: a first coarse level whose
+    transfers are grid-wide, the 27-point levels of a grid without solid cells, levels split
+    over the blocks and levels of one block, each cycle the oracle's bits."""
+    rng = np.random.default_rng(cells[0])
+    case = pkg.synth.case(cells, 2.0, inflow=5.0, preconditioner="multigrid",
+                          boxes=pkg.synth.random_boxes(rng, boxes, [2.0 * v for v in cells], side=(8.0, 24.0), dx=2.0))
+    g = pkg.grid.Grid.build(case)
+    og = O.Grid(case)
+    dg = pkg.pressure.DeviceGrid(g, preconditioner="multigrid")
+    for seed in range(2):
+        r = np.where(g.fluid == 1, np.random.default_rng(seed).uniform(-1.0, 1.0, g.count), 0.0)
+        oz, _ = og.mg_apply(r)
+        assert np.array_equal(bits(dg.precondition(r)), bits(oz))
+    dg.close()
