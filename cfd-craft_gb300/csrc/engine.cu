@@ -17,8 +17,7 @@
 // Also here, on device arrays: laminar SSPRK2 time stepping (momentum right-hand side
 // and stage update, cfdg_step_device), linear-upwind scalar transport (k_scalar_pass,
 // cfdg_scalar_step_device), receptor sampling (cfdg_receptors_sample), and the
-// line/plane block smoothers of anisotropic multigrid hierarchies (line_block, in the
-// cooperative V-cycle k_plain_coarse). All of it follows the reference's operation order
+// line/plane block smoothers of anisotropic multigrid hierarchies (line_cluster.cuh). All of it follows the reference's operation order
 // (bit-identical results) under -fmad=false.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -371,6 +370,48 @@ __global__ void k_center(const int* __restrict__ off, const int* __restrict__ me
   for (int k = b + threadIdx.x; k < e; k += blockDim.x) x[members[k]] = x[members[k]] - m;
 }
 
+// The same for groups of many members, in two launches: the warps of k_center's block on SMs of
+// their own, with their loads in flight together (a single block waits 523 us for the loads and
+// FP64 sums of 110,592 members), then the differences by the whole grid. The sums keep
+// k_center's order.
+constexpr int CENTER_WARPS = BLOCK / 32;
+__global__ void __launch_bounds__(32) k_center_sums(const int* __restrict__ off, const int* __restrict__ members,
+                                                    const double* __restrict__ x, double* part, const Scalars* S) {
+  if (S && S->done) return;
+  const int b = off[blockIdx.y], e = off[blockIdx.y + 1];
+  constexpr int AHEAD = 32;
+  double acc = 0.0;
+  int m[AHEAD];
+  const auto fetch = [&](int k) {
+#pragma unroll
+    for (int q = 0; q < AHEAD; ++q) m[q] = k + q * BLOCK < e ? members[k + q * BLOCK] : 0;
+  };
+  int k = b + blockIdx.x * 32 + threadIdx.x;
+  fetch(k);
+  for (; k < e; k += AHEAD * BLOCK) {
+    double v[AHEAD];
+#pragma unroll
+    for (int q = 0; q < AHEAD; ++q) v[q] = k + q * BLOCK < e ? x[m[q]] : 0.0;
+    fetch(k + AHEAD * BLOCK);
+#pragma unroll
+    for (int q = 0; q < AHEAD; ++q)
+      if (k + q * BLOCK < e) acc += v[q];
+  }
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+  if (threadIdx.x == 0) part[blockIdx.y * CENTER_WARPS + blockIdx.x] = acc;
+}
+__global__ void k_center_apply(const int* __restrict__ off, const int* __restrict__ members, double* __restrict__ x,
+                               const double* __restrict__ part, const Scalars* S) {
+  if (S && S->done) return;
+  const int b = off[blockIdx.y], e = off[blockIdx.y + 1], lane = threadIdx.x & 31;
+  const int k0 = b + blockIdx.x * blockDim.x + threadIdx.x;
+  if (k0 - (int)threadIdx.x >= e) return;
+  double s = lane < CENTER_WARPS ? part[blockIdx.y * CENTER_WARPS + lane] : 0.0;
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  const double m = __shfl_sync(0xffffffffu, s / (double)(e - b), 0);
+  for (int k = k0; k < e; k += gridDim.x * blockDim.x) x[members[k]] = x[members[k]] - m;
+}
+
 // Compatibility of the closed components (pressure.rs:351-362): one block per group.
 __global__ void k_compat(const int* __restrict__ off, const int* __restrict__ members, const double* __restrict__ b,
                          const double* __restrict__ terms, int use_terms, Scalars* S) {
@@ -564,28 +605,6 @@ __global__ void k_prolong(int n, const int* __restrict__ off, const int* __restr
   }
 }
 
-// Dense Cholesky solves of the terminal level, one thread per block (masked.rs:52-69).
-__global__ void k_direct(int nblocks, const int* __restrict__ ioff, const int* __restrict__ idx,
-                         const long long* __restrict__ foff, const double* __restrict__ L,
-                         const double* __restrict__ rhs, double* __restrict__ x, const Scalars* S) {
-  if (S && S->done) return;
-  int bk = blockIdx.x * blockDim.x + threadIdx.x;
-  if (bk >= nblocks) return;
-  const int* ix = idx + ioff[bk];
-  const int n = ioff[bk + 1] - ioff[bk];
-  const double* f = L + foff[bk];
-  for (int i = 0; i < n; ++i) {
-    double v = rhs[ix[i]];
-    for (int j = 0; j < i; ++j) v = v - f[i * n + j] * x[ix[j]];
-    x[ix[i]] = v / f[i * n + i];
-  }
-  for (int i = n - 1; i >= 0; --i) {
-    double v = x[ix[i]];
-    for (int j = i + 1; j < n; ++j) v = v - f[j * n + i] * x[ix[j]];
-    x[ix[i]] = v / f[i * n + i];
-  }
-}
-
 // ----------------------------------------------------------------- coarse levels, one launch
 // Levels 1 .. L-1 of the V-cycle in one cooperative kernel: each dependency level of a
 // lexicographic sweep, the residual, the restriction, the prolongation and the gauges is
@@ -608,13 +627,6 @@ struct PLev {
   const int *ioff, *idx;
   const long long* foff;
   const double* fac;
-  // Sweeps each way (2, or 1 with block smoothing) and the block smoother, if any.
-  int nsweep, lines, llen, lbw;
-  int lnfwd, lnbwd, lblocal, pad2_;
-  const int *lnodes, *looff, *locol;
-  const double *loval, *lfac;
-  double* lscr;
-  const int *lfo, *lfs, *lbo, *lbs;
 };
 
 namespace cg = cooperative_groups;
@@ -633,93 +645,18 @@ struct ClusterBarrier {
 constexpr int PC_CLUSTER = 8;  // blocks of that cluster (portable size)
 
 }  // namespace
+#include "line_cluster.cuh"
 #include "plain_cluster.cuh"
 namespace {
 
-// The banded forward and backward substitutions of one block (multigrid/line.rs:172-185)
-// for a half-bandwidth BW: the last BW results stay in registers and the factor entries of
-// a row are independent of the chain, so only the multiply-subtract chain is serial. The
-// operations and their order are the reference's (bit-identical).
-template <int BW>
-__device__ __forceinline__ void line_subst(double* s, const double* __restrict__ fac, long long base, int len) {
-  constexpr int stride = BW + 1;
-  double w[BW + 1];  // w[d]: the result d rows back (forward) or ahead (backward)
-#pragma unroll
-  for (int d = 0; d <= BW; ++d) w[d] = 0.0;
-  for (int i = 0; i < len; ++i) {
-    const double* f = fac + base + (long long)i * stride;
-    double v = s[i];
-#pragma unroll
-    for (int d = BW; d >= 1; --d)  // columns i-BW .. i-1, ascending
-      if (i - d >= 0) v = v - f[d] * w[d];
-    v = v * f[0];
-    s[i] = v;
-#pragma unroll
-    for (int d = BW; d >= 2; --d) w[d] = w[d - 1];
-    w[1] = v;
-  }
-#pragma unroll
-  for (int d = 0; d <= BW; ++d) w[d] = 0.0;
-  for (int i = len - 1; i >= 0; --i) {
-    double v = s[i];
-#pragma unroll
-    for (int d = 1; d <= BW; ++d)  // columns i+1 .. i+BW, ascending
-      if (i + d < len) v = v - fac[base + (long long)(i + d) * stride + d] * w[d];
-    v = v * fac[base + (long long)i * stride];
-    s[i] = v;
-#pragma unroll
-    for (int d = BW; d >= 2; --d) w[d] = w[d - 1];
-    w[1] = v;
-  }
-}
-
-// Any half-bandwidth, as line.rs:172-185 writes it.
-__device__ __noinline__ void line_subst_any(double* s, const double* __restrict__ fac, long long base, int len, int bw) {
-  const long long stride = bw + 1;
-  for (int i = 0; i < len; ++i) {
-    const long long row = base + i * stride;
-    double v = s[i];
-    for (int j = max(0, i - bw); j < i; ++j) v = v - fac[row + i - j] * s[j];
-    s[i] = v * fac[row];
-  }
-  for (int i = len - 1; i >= 0; --i) {
-    double v = s[i];
-    for (int j = i + 1; j < min(len, i + bw + 1); ++j) v = v - fac[base + j * stride + j - i] * s[j];
-    s[i] = v * fac[base + i * stride];
-  }
-}
-
-constexpr int LSCR = 256;  // block lengths up to this keep their scratch in shared memory
-
-// multigrid/line.rs:155-190, one block, by one warp: the lanes gather the right-hand side
-// less the outside entries for the block's nodes (each node's entries in the reference's
-// order), lane 0 runs the substitutions, the lanes write the block's values to x.
-// Bit-identical to the sequential sweep. x and rhs come through L2 (other blocks of the
-// launch write them); the scratch is the warp's shared row or the block's global slice.
-__device__ __forceinline__ void line_block(int b, const PLev& L, const double* rhs, double* x, int lane,
-                                           double* wsh) {
-  const int len = L.llen, bw = L.lbw;
-  const int start = b * len;
-  const long long base = (long long)start * (bw + 1);
-  double* scr = len <= LSCR ? wsh : L.lscr + start;
-  for (int i = lane; i < len; i += 32) {
-    double v = __ldcg(&rhs[L.lnodes[start + i]]);
-    for (int e = L.looff[start + i]; e < L.looff[start + i + 1]; ++e) v = v - L.loval[e] * __ldcg(&x[L.locol[e]]);
-    scr[i] = v;
-  }
-  __syncwarp();
-  if (lane == 0) {
-    switch (bw) {
-      case 1: line_subst<1>(scr, L.lfac, base, len); break;
-      case 2: line_subst<2>(scr, L.lfac, base, len); break;
-      case 3: line_subst<3>(scr, L.lfac, base, len); break;
-      case 4: line_subst<4>(scr, L.lfac, base, len); break;
-      default: line_subst_any(scr, L.lfac, base, len, bw); break;
-    }
-  }
-  __syncwarp();
-  for (int i = lane; i < len; i += 32) x[L.lnodes[start + i]] = scr[i];
-  __syncwarp();  // the row is reused by the warp's next block
+// Dense Cholesky solves of the terminal level, one warp per block.
+__global__ void k_direct(int nblocks, const int* __restrict__ ioff, const int* __restrict__ idx,
+                         const long long* __restrict__ foff, const double* __restrict__ f,
+                         const double* __restrict__ frd, const double* rhs, double* x, const Scalars* S) {
+  if (S && S->done) return;
+  const int bk = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (bk >= nblocks) return;
+  pc_direct(idx + ioff[bk], ioff[bk + 1] - ioff[bk], f + foff[bk], frd + ioff[bk], rhs, x);
 }
 
 template <class Bar>
@@ -730,40 +667,8 @@ __device__ void pc_center(const PLev& L, double* v, double* sh, double* mean, Ba
   grid.sync();
 }
 
-// A block Gauss-Seidel sweep over the block dependency levels (blocks of one level share
-// no entry, so they run in parallel; the reference's block order is kept where it matters).
 template <class Bar>
-__device__ void pc_lines(const PLev& L, bool backward, Bar& grid, double* lsh) {
-  const int* order = backward ? L.lbo : L.lfo;
-  const int* start = backward ? L.lbs : L.lfs;
-  const int nlev = backward ? L.lnbwd : L.lnfwd;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
-  double* wsh = lsh + warp * LSCR;
-  if (L.lblocal) {
-    if (blockIdx.x == 0)
-      for (int dl = 0; dl < nlev; ++dl) {
-        for (int t = start[dl] + warp; t < start[dl + 1]; t += wpb) line_block(order[t], L, L.rhs, L.x, lane, wsh);
-        __threadfence();
-        __syncthreads();
-      }
-    __threadfence();
-    grid.sync();
-    return;
-  }
-  const int gw = blockIdx.x * wpb + warp, nw = gridDim.x * wpb;
-  for (int dl = 0; dl < nlev; ++dl) {
-    for (int t = start[dl] + gw; t < start[dl + 1]; t += nw) line_block(order[t], L, L.rhs, L.x, lane, wsh);
-    __threadfence();
-    grid.sync();
-  }
-}
-
-template <class Bar>
-__device__ void pc_sweep(const PLev& L, bool backward, Bar& grid, double* lsh) {
-  if (L.lines) {
-    pc_lines(L, backward, grid, lsh);
-    return;
-  }
+__device__ void pc_sweep(const PLev& L, bool backward, Bar& grid) {
   const int* order = backward ? L.bo : L.fo;
   const int* start = backward ? L.bs : L.fs;
   const int nlev = backward ? L.nbwd : L.nfwd;
@@ -792,7 +697,6 @@ __device__ void plain_coarse(const PLev* lv, int nl, const Scalars* S, Bar& grid
   if (S && S->done) return;  // read once; nothing in this kernel changes it
   __shared__ double sh[32];
   __shared__ double mean;
-  __shared__ double lsh[(BLOCK / 32) * LSCR];  // one scratch row per warp (block smoothers)
   const int gt = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
   int l = 0;
   for (; l < nl; ++l) {
@@ -808,7 +712,7 @@ __device__ void plain_coarse(const PLev* lv, int nl, const Scalars* S, Bar& grid
       pc_center(L, L.x, sh, &mean, grid);
       break;
     }
-    for (int sw = 0; sw < L.nsweep; ++sw) pc_sweep(L, false, grid, lsh);
+    for (int sw = 0; sw < 2; ++sw) pc_sweep(L, false, grid);
     pc_center(L, L.x, sh, &mean, grid);
     for (int i = gt; i < L.n; i += nth) residual_row(i, L.off, L.col, L.val, L.diag, L.rhs, L.x, L.res);
     __threadfence();
@@ -825,7 +729,7 @@ __device__ void plain_coarse(const PLev* lv, int nl, const Scalars* S, Bar& grid
     for (int i = gt; i < L.n; i += nth) prolong_row(i, L.poff, L.pcol, L.pval, N.x, L.x);
     __threadfence();
     grid.sync();
-    for (int sw = 0; sw < L.nsweep; ++sw) pc_sweep(L, true, grid, lsh);
+    for (int sw = 0; sw < 2; ++sw) pc_sweep(L, true, grid);
     pc_center(L, L.x, sh, &mean, grid);
   }
 }
@@ -943,8 +847,19 @@ inline void tick(cfdg_grid* G) {
   if (!G->capturing) count();
 }
 
+// Members from which a group is centred in two launches. One against two, us: 110,592 members
+// 523 / 54, 13,824 57 / 15, 4,608 21 / 12, 1,152 9 / 11.
+constexpr int CENTER_SPLIT = 2048;
+
 int launch_center(cfdg_grid* G, const DevCsr& groups, int ngroups, double* x, const Scalars* S) {
   if (ngroups == 0) return 0;
+  if (groups.most >= CENTER_SPLIT && ngroups * CENTER_WARPS <= MAX_BLOCKS) {
+    // G->partials is free between the reductions of the stream's kernels.
+    k_center_sums<<<dim3(CENTER_WARPS, ngroups), 32, 0, G->stream>>>(groups.off, groups.col, x, G->partials, S); tick(G);
+    k_center_apply<<<dim3(grid_blocks(groups.most), ngroups), BLOCK, 0, G->stream>>>(groups.off, groups.col, x,
+                                                                                     G->partials, S); tick(G);
+    return 0;
+  }
   k_center<<<ngroups, BLOCK, 0, G->stream>>>(groups.off, groups.col, x, S); tick(G);
   return 0;
 }
@@ -1083,6 +998,24 @@ void launch_plain_cluster(cfdg_grid* G, const DevHierarchy& H, int from, int wha
   tick(G);
 }
 
+// A block Gauss-Seidel sweep of an anisotropic level (line_cluster.cuh).
+void launch_lines(cfdg_grid* G, const DevLevel& L, bool backward, const Scalars* S) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(L.ll.nb, 1, 1);
+  cfg.blockDim = dim3(LCT, 1, 1);
+  cfg.dynamicSmemBytes = (size_t)L.lsmem;
+  cfg.stream = G->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = L.ll.nb;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, line_kernel(backward, L.lshx), L.ll, S);
+  tick(G);
+}
+
 // One symmetric V(2,2) cycle, z = M^-1 r (multigrid.rs:656-726, masked.rs:292-342).
 void launch_vcycle(cfdg_grid* G, const double* r, double* z, const Scalars* S) {
   DevHierarchy& H = *G->mg;
@@ -1098,26 +1031,29 @@ void launch_vcycle(cfdg_grid* G, const double* r, double* z, const Scalars* S) {
   }
   const int nl = (int)H.levels.size();
   // Levels 1 .. L-1 in one cooperative launch when available, else level by level.
-  const bool coop = (H.coop_blocks > 0 || H.cluster || H.pc_rest > 0) && nl > 1;
+  const bool coop = !H.lines && (H.coop_blocks > 0 || H.cluster || H.pc_rest > 0) && nl > 1;
   // The first level of the cooperative launch, or of the cluster plan's whole cycle.
-  const int first = H.pc_rest > 0 ? H.pc_rest : H.coop0 ? 0 : 1;
+  const int first = H.pc_rest > 0 ? H.pc_rest : 1;
   for (int l = 0; l < (coop ? first : nl); ++l) {
     DevLevel& L = H.levels[l];
     const bool full = l == 0 && H.full0;
     const bool planned = l > 0 && H.pc_rest > 0;  // no groups, not terminal
     launch_center(G, L.groups, L.ngroups, L.rhs, S);
-    if (!planned) {
+    if (!planned && !L.lshx) {
       k_fill<<<grid_blocks(L.n), BLOCK, 0, s>>>(L.x, 0.0, L.n, S); tick(G);
     }
     if (L.terminal) {
       if (L.nblocks > 0) {
-        k_direct<<<(L.nblocks + 63) / 64, 64, 0, s>>>(L.nblocks, L.d_ioff, L.d_idx, L.d_foff, L.d_fac, L.rhs, L.x, S); tick(G);
+        k_direct<<<(L.nblocks + 1) / 2, 64, 0, s>>>(L.nblocks, L.d_ioff, L.d_idx, L.d_foff, L.d_fac, L.d_frd, L.rhs,
+                                                    L.x, S); tick(G);
       }
       launch_center(G, L.groups, L.ngroups, L.x, S);
       break;
     }
     if (planned) {
       launch_plain_cluster(G, H, l, 0, S);
+    } else if (L.lines) {
+      launch_lines(G, L, false, S);
     } else {
       launch_gs(G, L, false, S, full);
       launch_gs(G, L, false, S, full);
@@ -1138,7 +1074,7 @@ void launch_vcycle(cfdg_grid* G, const double* r, double* z, const Scalars* S) {
   if (H.pc_rest > 0) {
     launch_plain_cluster(G, H, H.pc_rest, 2, S);
   } else if (coop) {
-    // Block-smoothed hierarchies and levels with closed groups: one cluster of PC_CLUSTER
+    // Levels with closed groups or beyond the shared memory: one cluster of PC_CLUSTER
     // blocks (cluster barriers, about 0.3 us a phase), or the cooperative grid where clusters
     // cannot be launched.
     cudaLaunchConfig_t cfg = {};
@@ -1171,6 +1107,8 @@ void launch_vcycle(cfdg_grid* G, const double* r, double* z, const Scalars* S) {
     k_prolong<<<grid_blocks(L.n), BLOCK, 0, s>>>(L.n, L.prolong.off, L.prolong.col, L.prolong.val, C.x, L.x, S); tick(G);
     if (l > 0 && H.pc_rest > 0) {
       launch_plain_cluster(G, H, l, 1, S);
+    } else if (L.lines) {
+      launch_lines(G, L, true, S);
     } else {
       launch_gs(G, L, true, S, full);
       launch_gs(G, L, true, S, full);
@@ -1322,14 +1260,6 @@ int build_ic0_dev(cfdg_grid* G) {
   return 0;
 }
 
-// Device bytes of one level's block smoother as uploaded (nodes, outside rows, banded
-// factor, scratch, the two dependency orders).
-uint64_t line_device_bytes(const LineBlocks& B) {
-  return 4 * (B.nodes.size() + B.outside.off.size() + B.outside.col.size() + B.fwd.order.size() +
-              B.fwd.start.size() + B.bwd.order.size() + B.bwd.start.size()) +
-         8 * (B.outside.val.size() + B.factor.size() + B.nodes.size());
-}
-
 // MultigridStats (multigrid.rs:55-72) as JSON, fields in the reference's order; the empty
 // level_dimensions and block_smoothers are omitted as serde skips them. allocated_bytes
 // counts the device arrays the hierarchy holds (the storage this engine retains).
@@ -1354,7 +1284,7 @@ std::string stats_json_of(const DevHierarchy& D, const Hierarchy& H) {
       for (size_t a = 0; a < B.axes.size(); ++a) blocks += (a ? "," : "") + std::to_string(B.axes[a]);
       blocks += "],\"block_unknowns\":" + std::to_string(B.length) + ",\"block_count\":" +
                 std::to_string(B.count()) + ",\"half_bandwidth\":" + std::to_string(B.bandwidth) +
-                ",\"allocated_bytes\":" + std::to_string(line_device_bytes(B)) + "}";
+                ",\"allocated_bytes\":" + std::to_string(D.levels[l].lbytes) + "}";
     }
   if (!blocks.empty()) s += ",\"block_smoothers\":[" + blocks + "]";
   return s + "}";
@@ -1422,6 +1352,126 @@ double host_recip(double d) {
   if (!(d >= 0x1p-60 && d <= 0x1p60)) return 0.0;
   const double r = 1.0 / d;
   return std::fabs(std::fma(r, d, -1.0)) <= 0x1p-54 ? r : -r;
+}
+
+// Reciprocals of a terminal level's factor diagonals, by solved row.
+std::vector<double> direct_recip(const MgLevel& M) {
+  std::vector<double> rd(M.direct_idx.col.size());
+  for (int b = 0; b < M.direct_idx.rows(); ++b) {
+    const int n = M.direct_idx.off[b + 1] - M.direct_idx.off[b];
+    for (int i = 0; i < n; ++i)
+      rd[M.direct_idx.off[b] + i] = host_recip(M.direct_factor[M.direct_off[b] + (size_t)i * n + i]);
+  }
+  return rd;
+}
+
+// The sweeps of an anisotropic level (line_cluster.cuh): a cluster of 16 blocks (8 where the
+// device does not schedule the non-portable size), the iterate in its shared memory and the
+// records copied ahead where both fit, else only the copies, else neither.
+int plan_lines(DevHierarchy& D, DevLevel& L, const MgLevel& M, const LineBlocks& B, cudaStream_t s) {
+  L.lines = true;
+  LineLev& P = L.ll;
+  P.n = M.n, P.len = B.length, P.bw = B.bandwidth, P.count = B.count(), P.ndep = B.fwd.levels();
+  const int len = P.len, W = P.bw + 1;
+  std::vector<int> most(P.count, 0), where(P.count), block(M.n), place(M.n);
+  int wide = 0;
+  for (int q = 0; q < P.count; ++q) {
+    where[B.fwd.order[q]] = q;
+    for (int at = q * len; at < (q + 1) * len; ++at) {
+      block[B.nodes[at]] = q, place[B.nodes[at]] = at - q * len;
+      most[q] = std::max(most[q], B.outside.off[at + 1] - B.outside.off[at]);
+    }
+    wide = std::max(wide, most[q]);
+  }
+  P.wide = wide;
+  P.val_at = 16 + (len + P.bw) * W * 8;
+  P.col_at = P.val_at + wide * len * 8;
+  P.place_at = P.col_at + wide * len * 4;
+  P.row_at = P.place_at + wide * len * 4;
+  P.rec = (P.row_at + len * 4 + 15) / 16 * 16;
+  const long long starts = ((P.ndep + 1) * 4 + 15) / 16 * 16, bufs = 2LL * LCW * P.rec;
+  P.x_at = (int)starts;
+  for (P.nb = 16;; P.nb = 8) {
+    const long long xs = (8LL * ((P.count + P.nb - 1) / P.nb * len + 1) + 15) / 16 * 16;
+    P.scr_len = wide * len;
+    L.lshx = starts + xs + bufs + 8LL * LCW * P.scr_len <= LC_SMEM;
+    if (!L.lshx) P.scr_len += len;
+    P.staged = L.lshx || starts + bufs + 8LL * LCW * P.scr_len <= LC_SMEM;
+    P.buf_at = (int)(starts + (L.lshx ? xs : 0));
+    P.scr_at = P.staged ? (int)(P.buf_at + bufs) : 0;
+    L.lsmem = (int)(P.staged ? P.scr_at + 8LL * LCW * P.scr_len : starts);
+    int clusters = 0;
+    for (int way = 0; way < 2; ++way) {
+      const auto k = line_kernel(way == 1, L.lshx);
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(P.nb, 1, 1);
+      cfg.blockDim = dim3(LCT, 1, 1);
+      cfg.dynamicSmemBytes = (size_t)L.lsmem;
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = P.nb;
+      at[0].val.clusterDim.y = 1;
+      at[0].val.clusterDim.z = 1;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      if (L.lsmem > LC_SMEM || cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+          cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, LC_SMEM) != cudaSuccess ||
+          cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) != cudaSuccess || clusters < 1) {
+        cudaGetLastError();
+        clusters = 0;
+        break;
+      }
+    }
+    if (clusters > 0) break;
+    if (P.nb == 8) return fail(CFDG_ERR_UNSUPPORTED, "block-smoothed multigrid needs a thread-block cluster");
+  }
+  std::vector<unsigned char> recs((size_t)P.count * P.rec, 0);
+  const unsigned zero = (unsigned)(P.x_at + 8 * ((P.count + P.nb - 1) / P.nb * len));
+  for (int q = 0; q < P.count; ++q) {
+    const int g = where[q];
+    unsigned char* r = &recs[(size_t)g * P.rec];
+    std::memcpy(r + 16, &B.factor[(size_t)q * len * W], (size_t)len * W * 8);
+    int t = 0, behind = 0;
+    for (int pass = 0; pass < 2; ++pass) {  // entries with blocks behind and free places, then the others
+      for (int e = 0; e < most[q]; ++e)
+        for (int i = 0; i < len; ++i) {
+          const int at = q * len + i, b = B.outside.off[at], n = B.outside.off[at + 1] - b, place_e = e * len + i;
+          double v = 0.0;
+          unsigned c = L.lshx ? (unsigned)(g % P.nb) << 24 | zero : (unsigned)M.n;
+          int h = P.count;
+          if (e < n) {
+            const int j = B.outside.col[b + e];
+            h = where[block[j]];
+            c = L.lshx ? (unsigned)(h % P.nb) << 24 | (unsigned)(P.x_at + 8 * (h / P.nb * len + place[j])) : (unsigned)j;
+            v = B.outside.val[b + e];
+          }
+          if ((h < g) != (pass == 1)) continue;
+          std::memcpy(r + P.val_at + 8 * (size_t)t, &v, 8);
+          std::memcpy(r + P.col_at + 4 * (size_t)t, &c, 4);
+          std::memcpy(r + P.place_at + 4 * (size_t)t, &place_e, 4);
+          ++t;
+        }
+      if (pass == 0) behind = t;
+    }
+    const int head[3] = {behind, t, most[q]};
+    std::memcpy(r, head, 12);
+    std::memcpy(r + P.row_at, &B.nodes[q * len], (size_t)len * 4);
+  }
+  unsigned char* dr;
+  int* ds;
+  if (int e = D.arena.upload(&dr, recs, s)) return e;
+  if (int e = D.arena.upload(&ds, B.fwd.start, s)) return e;
+  P.recs = dr, P.start = ds;
+  L.lbytes = recs.size() + 4 * B.fwd.start.size();
+  if (!P.staged) {
+    const size_t words = (size_t)P.nb * LCW * P.scr_len;
+    if (int e = D.arena.alloc(&P.scr, words)) return e;
+    L.lbytes += 8 * words;
+  }
+  P.rhs = L.rhs, P.x = L.x;
+  CU(cudaMemsetAsync(L.x + M.n, 0, 8, s));
+  CU(cudaStreamSynchronize(s));  // the records' host copy goes out of scope
+  return 0;
 }
 
 // The cluster plan of levels 1.. (plain_cluster.cuh), where no level has closed groups or
@@ -1494,16 +1544,7 @@ int plan_plain_cluster(DevHierarchy& D, const Hierarchy& H, cudaStream_t s) {
     if (L.terminal) {
       L.nblocks = V.nblocks;
       L.ioff = V.d_ioff, L.idx = V.d_idx, L.foff = V.d_foff, L.fac = V.d_fac;
-      std::vector<double> rd(M.direct_idx.col.size());
-      for (int b = 0; b < L.nblocks; ++b) {
-        const int n = M.direct_idx.off[b + 1] - M.direct_idx.off[b];
-        for (int i = 0; i < n; ++i)
-          rd[M.direct_idx.off[b] + i] = host_recip(M.direct_factor[M.direct_off[b] + (size_t)i * n + i]);
-      }
-      double* d;
-      if (int e = D.arena.upload(&d, rd, s)) return e;
-      L.frd = d;
-      CU(cudaStreamSynchronize(s));
+      L.frd = V.d_frd;
       continue;
     }
     L.roff = V.restrict_.off, L.rcol = V.restrict_.col, L.rval = V.restrict_.val;
@@ -1614,7 +1655,7 @@ int build_mg_dev(cfdg_grid* G, const Poller& poll) {
   D->levels.resize(H.levels.size());
   const bool lines = !H.levels.empty() && !H.levels[0].lines.empty();
   D->full0 = G->structured && H.levels.size() > 1 && !lines;
-  D->coop0 = lines && H.levels.size() > 1;
+  D->lines = lines && H.levels.size() > 1;
   if (D->full0) reindex_level0(G, H);
   for (size_t l = 0; l < H.levels.size(); ++l) {
     MgLevel& M = H.levels[l];
@@ -1648,40 +1689,26 @@ int build_mg_dev(cfdg_grid* G, const Poller& poll) {
       std::vector<long long> foff(M.direct_off.begin(), M.direct_off.end());
       if (int e = D->arena.upload(&L.d_foff, foff, s)) return e;
       if (int e = D->arena.upload(&L.d_fac, M.direct_factor, s)) return e;
+      std::vector<double> rd = direct_recip(M);
+      if (int e = D->arena.upload(&L.d_frd, rd, s)) return e;
     } else {
       if (int e = upload_csr(D->arena, M.prolong, L.prolong, s)) return e;
       if (int e = upload_csr(D->arena, M.restrict, L.restrict_, s)) return e;
     }
     if (int e = D->arena.alloc(&L.rhs, L.n)) return e;
-    if (int e = D->arena.alloc(&L.x, L.n)) return e;
+    if (int e = D->arena.alloc(&L.x, L.n + 1)) return e;  // + a zero behind a block-smoothed level's
     if (int e = D->arena.alloc(&L.res, L.n)) return e;
     if (!M.lines.empty()) {
-      const LineBlocks& B = M.lines[0];  // the reference builds one block group per level
-      L.lines = true;
-      L.llen = B.length;
-      L.lbw = B.bandwidth;
-      L.lcount = B.count();
-      if (int e = D->arena.upload(&L.lnodes, B.nodes, s)) return e;
-      if (int e = D->arena.upload(&L.looff, B.outside.off, s)) return e;
-      if (int e = D->arena.upload(&L.locol, B.outside.col, s)) return e;
-      if (int e = D->arena.upload(&L.loval, B.outside.val, s)) return e;
-      if (int e = D->arena.upload(&L.lfac, B.factor, s)) return e;
-      if (int e = D->arena.alloc(&L.lscr, B.nodes.size())) return e;
-      if (int e = D->arena.upload(&L.lfwd.order, B.fwd.order, s)) return e;
-      if (int e = D->arena.upload(&L.lbwd.order, B.bwd.order, s)) return e;
-      L.lfwd.start = B.fwd.start;
-      L.lbwd.start = B.bwd.start;
-      if (int e = D->arena.upload(&L.lfwd.d_start, B.fwd.start, s)) return e;
-      if (int e = D->arena.upload(&L.lbwd.d_start, B.bwd.start, s)) return e;
+      // The reference builds one block group per level.
+      if (int e = plan_lines(*D, L, M, M.lines[0], s)) return e;
     }
   }
   D->level_cells = H.level_cells;
   D->level_nonzeros = H.level_nonzeros;
-  // Levels 1 .. L-1 (0 .. L-1 for block-smoothed hierarchies) for the cooperative kernel,
-  // when its grid can be co-resident.
-  if (D->levels.size() > 1) {
+  // Levels 1 .. L-1 for the cooperative kernel, when its grid can be co-resident.
+  if (D->levels.size() > 1 && !D->lines) {
     std::vector<PLev> pl;
-    for (size_t l = D->coop0 ? 0 : 1; l < D->levels.size(); ++l) {
+    for (size_t l = 1; l < D->levels.size(); ++l) {
       const DevLevel& L = D->levels[l];
       PLev P{};
       P.n = L.n;
@@ -1701,20 +1728,6 @@ int build_mg_dev(cfdg_grid* G, const Poller& poll) {
       P.poff = L.prolong.off, P.pcol = L.prolong.col, P.pval = L.prolong.val;
       P.rhs = L.rhs, P.x = L.x, P.res = L.res;
       P.ioff = L.d_ioff, P.idx = L.d_idx, P.foff = L.d_foff, P.fac = L.d_fac;
-      P.nsweep = L.lines ? 1 : 2;  // multigrid.rs:676
-      P.lines = L.lines ? 1 : 0;
-      if (L.lines) {
-        P.llen = L.llen, P.lbw = L.lbw;
-        P.lnfwd = (int)L.lfwd.start.size() - 1;
-        P.lnbwd = (int)L.lbwd.start.size() - 1;
-        int lmax = 0;
-        for (int q = 0; q < P.lnfwd; ++q) lmax = std::max(lmax, L.lfwd.start[q + 1] - L.lfwd.start[q]);
-        for (int q = 0; q < P.lnbwd; ++q) lmax = std::max(lmax, L.lbwd.start[q + 1] - L.lbwd.start[q]);
-        P.lblocal = lmax <= BLOCK / 32 ? 1 : 0;  // one warp per block solve
-        P.lnodes = L.lnodes, P.looff = L.looff, P.locol = L.locol, P.loval = L.loval, P.lfac = L.lfac;
-        P.lscr = L.lscr;
-        P.lfo = L.lfwd.order, P.lfs = L.lfwd.d_start, P.lbo = L.lbwd.order, P.lbs = L.lbwd.d_start;
-      }
       pl.push_back(P);
     }
     PLev* dp = nullptr;
@@ -1750,8 +1763,6 @@ int build_mg_dev(cfdg_grid* G, const Poller& poll) {
       D->cluster = clusters > 0;
     }
     if (int e = plan_plain_cluster(*D, H, s)) return e;
-    if (D->coop0 && D->coop_blocks == 0 && !D->cluster)
-      return fail(CFDG_ERR_UNSUPPORTED, "block-smoothed multigrid needs a co-resident cooperative launch");
   }
   CU(cudaStreamSynchronize(s));
   G->host_mg = std::make_shared<Hierarchy>(std::move(H));
@@ -1936,7 +1947,7 @@ int solve_device(cfdg_grid* G, bool use_terms, double tol, uint64_t max_iter, co
       if (L.lines) {
         // multigrid.rs:677-718: one block sweep each way, every block solved.
         bvisits += n;
-        bsolves += 2 * (uint64_t)L.lcount;
+        bsolves += 2 * (uint64_t)L.ll.count;
       }
     }
     inf->smoothing_cell_updates = smooth * cyc;

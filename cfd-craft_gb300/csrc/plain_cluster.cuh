@@ -240,10 +240,9 @@ __device__ void pc_sweep_level(const PcLev& L, int rank, int* ls, unsigned char*
 // lane keeps its row and takes the solved ones off in ascending order; backward, the lanes
 // form a row's products and every lane runs the row's subtractions in ascending order. Blocks
 // of more than 32 rows by one thread.
-__device__ __noinline__ void pc_direct(const PcLev& L, int bk, const double* rhs, double* x) {
-  const int* ix = L.idx + L.ioff[bk];
-  const int n = L.ioff[bk + 1] - L.ioff[bk], ln = threadIdx.x & 31;
-  const double* f = L.fac + L.foff[bk];
+__device__ __noinline__ void pc_direct(const int* ix, int n, const double* f, const double* frd, const double* rhs,
+                                       double* x) {
+  const int ln = threadIdx.x & 31;
   if (n > 32) {
     if (ln == 0) {
       for (int i = 0; i < n; ++i) {
@@ -260,7 +259,7 @@ __device__ __noinline__ void pc_direct(const PcLev& L, int bk, const double* rhs
     return;
   }
   const bool on = ln < n;
-  const double d = on ? __ldg(&f[ln * n + ln]) : 1.0, rd = on ? __ldg(&L.frd[L.ioff[bk] + ln]) : 0.0;
+  const double d = on ? __ldg(&f[ln * n + ln]) : 1.0, rd = on ? __ldg(&frd[ln]) : 0.0;
   double v = on ? rhs[ix[ln]] : 0.0, s = 0.0;
   double fj = on && ln > 0 ? __ldg(&f[ln * n]) : 0.0;
   for (int j = 0; j < n; ++j) {
@@ -318,7 +317,8 @@ __global__ void __launch_bounds__(PCT, 1) k_plain_cluster(const PcPlan* plan, in
       else cg::this_cluster().sync();
       if (L.terminal) {
         if (rank == 0) {
-          for (int bk = threadIdx.x >> 5; bk < L.nblocks; bk += PCT / 32) pc_direct(L, bk, rhs, x);
+          for (int bk = threadIdx.x >> 5; bk < L.nblocks; bk += PCT / 32)
+            pc_direct(L.idx + L.ioff[bk], L.ioff[bk + 1] - L.ioff[bk], L.fac + L.foff[bk], L.frd + L.ioff[bk], rhs, x);
           __syncthreads();
           for (int i = threadIdx.x; i < L.n; i += PCT) L.gx[i] = x[i];
         }

@@ -89,10 +89,11 @@ struct DevCsr {
   int* off = nullptr;
   int* col = nullptr;
   double* val = nullptr;
-  int rows = 0;
+  int rows = 0, most = 0;  // most: entries of the longest row
 };
 inline int upload_csr(Arena& A, const Csr& c, DevCsr& d, cudaStream_t s) {
   d.rows = c.rows();
+  for (int i = 0; i < d.rows; ++i) d.most = std::max(d.most, c.off[i + 1] - c.off[i]);
   if (int e = A.upload(&d.off, c.off, s)) return e;
   if (int e = A.upload(&d.col, c.col, s)) return e;
   if (!c.val.empty() || c.col.empty())
@@ -117,6 +118,28 @@ struct DevIc0 {
   DevSchedule fwd, bwd;
 };
 
+// An anisotropic level's block smoother as its sweeps read it (line_cluster.cuh).
+//
+// The record of a block of `len` rows: three ints (the entries with blocks behind it in the
+// sweep order, all its outside entries, the most of one of its rows) in 16 bytes; the factor,
+// (bw + 1) values per row as LineBlocks::factor, then bw rows of zeros; the values of the
+// outside entries, those with blocks behind first; their columns; the places of their products,
+// [entry of the row][row]; the rows' numbers. Places that a row does not use have an entry of
+// +0.0 with a column that holds +0.0: the difference of that product leaves every number's bits
+// alone. Columns, with the iterate in shared memory: owner << 24 | byte offset there; else the
+// row (n: the zero behind the iterate).
+struct LineLev {
+  int n, len, bw, count, ndep, nb;  // rows, rows per block, half-bandwidth, blocks, dependency levels, cluster size
+  int wide;                         // outside entries per row at most
+  int rec, val_at, col_at, place_at, row_at;  // bytes of a record, offsets of its parts
+  int staged, x_at, buf_at, scr_at;  // records copied ahead; offsets in the dynamic shared memory
+  int scr_len;                      // doubles of a warp's scratch (at scr_at, or scr where not staged)
+  const unsigned char* recs;        // [block in sweep order]
+  const int* start;                 // [ndep + 1]
+  const double* rhs;
+  double *x, *scr;
+};
+
 struct DevLevel {
   int n = 0;
   DevCsr a;
@@ -135,12 +158,13 @@ struct DevLevel {
   long long* d_foff = nullptr;
   double* d_fac = nullptr;
   double *rhs = nullptr, *x = nullptr, *res = nullptr;
-  // Anisotropic levels: the block smoother (setup.hpp LineBlocks) and its scratch.
-  bool lines = false;
-  int llen = 0, lbw = 0, lcount = 0;
-  int *lnodes = nullptr, *looff = nullptr, *locol = nullptr;
-  double *loval = nullptr, *lfac = nullptr, *lscr = nullptr;
-  DevSchedule lfwd, lbwd;
+  double* d_frd = nullptr;  // reciprocals of the terminal factors' diagonals, by solved row
+  // Anisotropic levels: the block smoother, whether its iterate lives in the cluster's shared
+  // memory, the dynamic shared memory of a sweep and the device bytes held.
+  bool lines = false, lshx = false;
+  int lsmem = 0;
+  uint64_t lbytes = 0;
+  LineLev ll{};
 };
 
 struct DevHierarchy {
@@ -162,9 +186,7 @@ struct DevHierarchy {
   // sweep there) and the dynamic shared memory of a launch.
   void* d_pc = nullptr;
   int pc_rest = 0, pc_smem = 0;
-  // Block-smoothed (anisotropic) hierarchies: d_plev starts at level 0 and the whole cycle
-  // is the cooperative launch.
-  bool coop0 = false;
+  bool lines = false;  // block-smoothed (anisotropic): level by level, sweeps on a cluster
 };
 
 }  // namespace cfdg

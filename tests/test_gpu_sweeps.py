@@ -56,3 +56,55 @@ def test_coarse_cluster_cycle_bitwise(pkg, O, cells, boxes):
         oz, _ = og.mg_apply(r)
         assert np.array_equal(bits(dg.precondition(r)), bits(oz))
     dg.close()
+
+
+@pytest.mark.parametrize("cells, size", [
+    ((9, 7, 100), (9.0, 7.0, 2.0)),      # more rows per line than two per lane
+    ((70, 72, 5), (70.0, 72.0, 0.5)),    # more lines per dependency level than warps
+    ((5, 5, 400), (5.0, 5.0, 8.0)),      # records too long to copy ahead
+    ((24, 4, 4), (240.0, 4.0, 4.0)),     # blocks of a whole plane
+    ((470, 460, 2), (470.0, 460.0, 0.2)),  # iterate beyond the cluster's shared memory
+])
+@pytest.mark.parametrize("boundaries", [("open", "wall", "wall"), ("open", "periodic", "wall")])
+def test_line_sweeps_bitwise(pkg, O, cells, size, boundaries):
+    """Block Gauss-Seidel sweeps of anisotropic grids on a cluster, each cycle the oracle's bits."""
+    if boundaries[1] == "periodic" and cells[0] > 100:
+        pytest.skip("the large grid once")
+    case = pkg.synth.case(cells, 1.0, boundaries=boundaries, inflow=1.0, preconditioner="multigrid")
+    case["domain"]["size_m"] = list(size)
+    g = pkg.grid.Grid.build(case)
+    og = O.Grid(case)
+    dg = pkg.pressure.DeviceGrid(g, preconditioner="multigrid")
+    for seed in range(2):
+        r = np.random.default_rng(seed).uniform(-1.0, 1.0, g.count)
+        oz, _ = og.mg_apply(r)
+        assert np.array_equal(bits(dg.precondition(r)), bits(oz))
+    assert dg.multigrid_stats()["block_smoothers"]
+    dg.close()
+
+
+def center_of(x):
+    """x less its mean in the engine's order: 256 strided sums, trees over 32 lanes and 8 warps."""
+    acc = np.zeros(256)
+    for k in range(0, x.size, 256):
+        acc[:x[k:k + 256].size] += x[k:k + 256]
+    w = acc.reshape(8, 32)
+    while w.shape[1] > 1:
+        w = w[:, :w.shape[1] // 2] + w[:, w.shape[1] // 2:]
+    w = w[:, 0]
+    while w.size > 1:
+        w = w[:w.size // 2] + w[w.size // 2:]
+    return x - w[0] / x.size
+
+
+@pytest.mark.parametrize("cells", [(89, 23, 1), (32, 8, 8), (683, 3, 1), (64, 64, 2), (67, 43, 29)])
+def test_center_bitwise(pkg, cells):
+    """The gauge of a closed grid in one launch and in two (2,048 members and more), with
+    members that fill the last stretch of loads and that do not."""
+    g = pkg.grid.Grid.build(pkg.synth.case(cells, 1.0, boundaries=("wall", "wall", "wall"), inflow=0.0))
+    dg = pkg.pressure.DeviceGrid(g, preconditioner="ic0")
+    x = np.random.default_rng(cells[0]).uniform(-1.0, 1.0, g.count) + 0.5
+    want = center_of(x)
+    dg.center_nullspaces(x)
+    assert np.array_equal(bits(x), bits(want))
+    dg.close()
