@@ -1025,7 +1025,7 @@ void launch_vcycle(cfdg_grid* G, const double* r, double* z, const Scalars* S) {
   if (H.masked && !H.full0) {
     k_gather<<<grid_blocks(H.nfluid), BLOCK, 0, s>>>(H.nfluid, H.fluid_idx, r, L0.rhs, S);
     tick(G);
-  } else {
+  } else if (L0.rhs != r) {
     k_copy<<<grid_blocks(N), BLOCK, 0, s>>>(L0.rhs, r, N, S);
     tick(G);
   }
@@ -1063,6 +1063,8 @@ void launch_vcycle(cfdg_grid* G, const double* r, double* z, const Scalars* S) {
       if (G->uniform) k_residual_struct<true><<<grid_blocks(L.n), BLOCK, 0, s>>>(G->g, L.diag, L.rhs, L.x, L.res, L.n, S);
       else k_residual_struct<false><<<grid_blocks(L.n), BLOCK, 0, s>>>(G->g, L.diag, L.rhs, L.x, L.res, L.n, S);
       tick(G);
+    } else if (planned) {
+      k_plan_residual<<<grid_blocks((long long)PCS * H.pc_chunk[l - 1]), BLOCK, 0, s>>>((const PcPlan*)H.d_pc, l - 1, S); tick(G);
     } else {
       k_residual<<<grid_blocks(L.n), BLOCK, 0, s>>>(L.n, L.a.off, L.a.col, L.a.val, L.diag, L.rhs, L.x, L.res, S); tick(G);
     }
@@ -1118,7 +1120,7 @@ void launch_vcycle(cfdg_grid* G, const double* r, double* z, const Scalars* S) {
   if (H.masked && !H.full0) {
     k_fill<<<grid_blocks(N), BLOCK, 0, s>>>(z, 0.0, N, S); tick(G);
     k_scatter<<<grid_blocks(H.nfluid), BLOCK, 0, s>>>(H.nfluid, H.fluid_idx, L0.x, z, S); tick(G);
-  } else {
+  } else if (L0.x != z) {
     k_copy<<<grid_blocks(N), BLOCK, 0, s>>>(z, L0.x, N, S); tick(G);
   }
 }
@@ -1550,7 +1552,8 @@ int plan_plain_cluster(DevHierarchy& D, const Hierarchy& H, cudaStream_t s) {
     L.roff = V.restrict_.off, L.rcol = V.restrict_.col, L.rval = V.restrict_.val;
     L.poff = V.prolong.off, L.pcol = V.prolong.col, L.pval = V.prolong.val;
     const int owners = L.solo ? 1 : PCS;
-    const size_t slots = (size_t)PCS * L.chunk;
+    const size_t slots = (size_t)owners * L.chunk;
+    L.slots = (int)slots;
     std::vector<int> ls((size_t)PCS * (L.ndep + 1), 0), gid(slots, 0), pos(M.n), fill(PCS, 0);
     // Positions: per owner (a contiguous range of rows) by dependency level, rows ascending.
     for (int dep = 0; dep < L.ndep; ++dep) {
@@ -1629,9 +1632,24 @@ int plan_plain_cluster(DevHierarchy& D, const Hierarchy& H, cudaStream_t s) {
   if (int e = D.arena.upload(&dp, one, s)) return e;
   CU(cudaStreamSynchronize(s));
   D.d_pc = dp;
+  D.pc_chunk.clear();
+  for (int l = 1; l <= rest; ++l) D.pc_chunk.push_back(P.lv[l - 1].chunk);
   D.pc_rest = rest + 1;
   D.pc_smem = std::max(at, most);
   return 0;
+}
+
+// A level's matrix and, where its point sweeps read them, their orders.
+int upload_rows(DevHierarchy& D, DevLevel& L, const MgLevel& M, bool orders, cudaStream_t s) {
+  if (int e = upload_csr(D.arena, M.a, L.a, s)) return e;
+  if (int e = D.arena.upload(&L.diag, M.diag, s)) return e;
+  if (!orders) return 0;
+  if (int e = D.arena.upload(&L.fwd.order, M.fwd.order, s)) return e;
+  if (int e = D.arena.upload(&L.bwd.order, M.bwd.order, s)) return e;
+  L.fwd.start = M.fwd.start;
+  L.bwd.start = M.bwd.start;
+  if (int e = D.arena.upload(&L.fwd.d_start, M.fwd.start, s)) return e;
+  return D.arena.upload(&L.bwd.d_start, M.bwd.start, s);
 }
 
 int build_mg_dev(cfdg_grid* G, const Poller& poll) {
@@ -1661,8 +1679,8 @@ int build_mg_dev(cfdg_grid* G, const Poller& poll) {
     MgLevel& M = H.levels[l];
     DevLevel& L = D->levels[l];
     L.n = M.n;
-    if (int e = upload_csr(D->arena, M.a, L.a, s)) return e;
-    if (int e = D->arena.upload(&L.diag, M.diag, s)) return e;
+    if (l == 0 || D->lines)
+      if (int e = upload_rows(*D, L, M, !D->lines, s)) return e;
     if (l == 0 && D->full0) {
       if (int e = D->arena.alloc(&L.rdiag, L.n)) return e;
       CU(cudaMemsetAsync(G->wave_err + 1, 0, sizeof(int), s));
@@ -1672,12 +1690,6 @@ int build_mg_dev(cfdg_grid* G, const Poller& poll) {
       CU(cudaStreamSynchronize(s));
       L.rd_extra = extra != 0;
     }
-    if (int e = D->arena.upload(&L.fwd.order, M.fwd.order, s)) return e;
-    if (int e = D->arena.upload(&L.bwd.order, M.bwd.order, s)) return e;
-    L.fwd.start = M.fwd.start;
-    L.bwd.start = M.bwd.start;
-    if (int e = D->arena.upload(&L.fwd.d_start, M.fwd.start, s)) return e;
-    if (int e = D->arena.upload(&L.bwd.d_start, M.bwd.start, s)) return e;
     L.ngroups = M.groups.rows();
     if (L.ngroups)
       if (int e = upload_csr(D->arena, M.groups, L.groups, s)) return e;
@@ -1695,8 +1707,16 @@ int build_mg_dev(cfdg_grid* G, const Poller& poll) {
       if (int e = upload_csr(D->arena, M.prolong, L.prolong, s)) return e;
       if (int e = upload_csr(D->arena, M.restrict, L.restrict_, s)) return e;
     }
-    if (int e = D->arena.alloc(&L.rhs, L.n)) return e;
-    if (int e = D->arena.alloc(&L.x, L.n + 1)) return e;  // + a zero behind a block-smoothed level's
+    // Level 0 in full-grid layout works on the solver's own vectors (a closed group's gauge
+    // changes the right-hand side, which is the residual that the solver keeps).
+    if (l == 0 && D->full0) {
+      L.x = G->z;
+      if (L.ngroups == 0) L.rhs = G->r;
+    }
+    if (!L.rhs)
+      if (int e = D->arena.alloc(&L.rhs, L.n)) return e;
+    if (!L.x)
+      if (int e = D->arena.alloc(&L.x, L.n + 1)) return e;  // + a zero behind a block-smoothed level's
     if (int e = D->arena.alloc(&L.res, L.n)) return e;
     if (!M.lines.empty()) {
       // The reference builds one block group per level.
@@ -1705,8 +1725,21 @@ int build_mg_dev(cfdg_grid* G, const Poller& poll) {
   }
   D->level_cells = H.level_cells;
   D->level_nonzeros = H.level_nonzeros;
-  // Levels 1 .. L-1 for the cooperative kernel, when its grid can be co-resident.
+  // Levels 1 .. L-1: the cluster plan, whose records stand for the levels' rows, else the rows and sweep orders. A plan that the context's budget has no room for is left out.
   if (D->levels.size() > 1 && !D->lines) {
+    const size_t held = D->arena.ptrs.size();
+    const uint64_t held_bytes = D->arena.bytes;
+    if (int e = plan_plain_cluster(*D, H, s)) {
+      if (e != CFDG_ERR_ADMISSION) return e;
+      CU(cudaStreamSynchronize(s));
+      D->arena.rollback(held, held_bytes);
+      D->pc_rest = 0;
+    }
+    for (size_t l = 1; D->pc_rest == 0 && l < D->levels.size(); ++l)
+      if (int e = upload_rows(*D, D->levels[l], H.levels[l], true, s)) return e;
+  }
+  // Without it, the levels for the cooperative kernel, when its grid can be co-resident.
+  if (D->levels.size() > 1 && !D->lines && D->pc_rest == 0) {
     std::vector<PLev> pl;
     for (size_t l = 1; l < D->levels.size(); ++l) {
       const DevLevel& L = D->levels[l];
@@ -1762,7 +1795,6 @@ int build_mg_dev(cfdg_grid* G, const Poller& poll) {
       }
       D->cluster = clusters > 0;
     }
-    if (int e = plan_plain_cluster(*D, H, s)) return e;
   }
   CU(cudaStreamSynchronize(s));
   G->host_mg = std::make_shared<Hierarchy>(std::move(H));

@@ -48,16 +48,17 @@ static_assert(sizeof(PcRec) == 96, "six 16-byte loads");
 
 struct PcLev {
   int n, chunk, ndep, solo;  // rows, rows per block, dependency levels, all rows in the first block
+  int slots;                 // positions of all owners
   int w;                     // entries per row at most
   int x, rhs;                // offsets in the dynamic shared memory (bytes), the same in every block; x[chunk] is +0.0
   int terminal, nblocks;
   const int* ls;             // [block][ndep + 1]: positions where the dependency levels start
-  const int* gid;            // [block][chunk]: the row at a position
-  const struct PcRec* rec;   // [block][chunk], where w <= PCW; else:
-  const unsigned* col;       // [w][block][chunk]: as PcRec::col
-  const double* val;         // [w][block][chunk]
-  const double *diag, *rd;   // [block][chunk]: diagonal and its reciprocal (recip_of)
-  const unsigned short* cnt;  // [block][chunk]: entries
+  const int* gid;            // [owner][chunk]: the row at a position
+  const struct PcRec* rec;   // [owner][chunk], where w <= PCW; else:
+  const unsigned* col;       // [w][owner][chunk]: as PcRec::col
+  const double* val;         // [w][owner][chunk]
+  const double *diag, *rd;   // [owner][chunk]: diagonal and its reciprocal (recip_of)
+  const unsigned short* cnt;  // [owner][chunk]: entries
   // Transfers and vectors in row numbering (DevLevel).
   const int *roff, *rcol, *poff, *pcol;
   const double *rval, *pval;
@@ -186,7 +187,7 @@ __device__ __noinline__ void pc_sweep_wide(const PcLev& L, int rank, const int* 
   double* x = reinterpret_cast<double*>(smem + L.x);
   const double* rhs = reinterpret_cast<const double*>(smem + L.rhs);
   const unsigned base = pc_addr(smem);
-  const int stride = PCS * L.chunk;
+  const int stride = L.slots;
   for (int q = 0; q < L.ndep; ++q) {
     const int dep = BWD ? L.ndep - 1 - q : q;
     for (int p0 = ls[dep]; p0 < ls[dep + 1]; p0 += PCT) {
@@ -284,6 +285,38 @@ __device__ __noinline__ void pc_direct(const int* ix, int n, const double* f, co
 
 // WHAT 0: two forward sweeps of level `from` from zero, its iterate to global memory. 1: two
 // backward sweeps of its iterate in global memory. 2: the whole cycle from level `from` on.
+// res = rhs - A x of a level whose transfers are grid-wide, from the plan's rows: the vectors in
+// row numbering, the neighbours through their owners' positions.
+__global__ void k_plan_residual(const PcPlan* plan, int l, const Scalars* S) {
+  if (S && S->done) return;
+  const PcLev& L = plan->lv[l];
+  const int slots = L.slots;
+  const auto at = [&](unsigned c) {  // the value that a place's column names
+    const int pos = ((int)(c & 0xffffffu) - L.x) >> 3;
+    return pos < L.chunk ? L.gx[__ldg(&L.gid[(int)(c >> 24) * L.chunk + pos])] : 0.0;
+  };
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < slots; q += gridDim.x * blockDim.x) {
+    if (q % L.chunk >= L.n - q / L.chunk * L.chunk) continue;  // behind the last block's rows
+    const int i = __ldg(&L.gid[q]);
+    double v;
+    if (L.rec) {
+      PcRow R;
+      pc_fetch(L.rec, q, slots, R);
+      v = R.r.d * L.gx[i];
+#pragma unroll
+      for (int a = 0; a < PCW; ++a) {
+        const double t = R.r.val[a] * at(R.r.col[a]);
+        v = v + (R.r.val[a] == 0.0 ? -0.0 : t);  // a free place adds -0.0, as below
+      }
+    } else {
+      v = __ldg(&L.diag[q]) * L.gx[i];
+      const int cnt = __ldg(&L.cnt[q]);
+      for (int a = 0; a < cnt; ++a) v = v + __ldg(&L.val[(size_t)a * slots + q]) * at(__ldg(&L.col[(size_t)a * slots + q]));
+    }
+    L.gres[i] = L.grhs[i] - v;
+  }
+}
+
 __global__ void __launch_bounds__(PCT, 1) k_plain_cluster(const PcPlan* plan, int from, int what, const Scalars* S) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ PcLev sL, sN;
@@ -332,7 +365,7 @@ __global__ void __launch_bounds__(PCT, 1) k_plain_cluster(const PcPlan* plan, in
       }
       // res = rhs - A x (the row's entries in order), then the restriction.
       const unsigned base = pc_addr(smem);
-      const int stride = PCS * L.chunk;
+      const int stride = L.slots;
       for (int p = threadIdx.x; p < m; p += PCT) {
         const int i = rank * L.chunk + p;
         double v;

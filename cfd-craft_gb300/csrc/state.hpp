@@ -77,6 +77,13 @@ struct Arena {
     if (!v.empty()) CU(cudaMemcpyAsync(*p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, s));
     return 0;
   }
+  // Gives back what was allocated after `held` pointers of `held_bytes` bytes.
+  void rollback(size_t held, uint64_t held_bytes) {
+    for (size_t i = held; i < ptrs.size(); ++i) cudaFree(ptrs[i]);
+    ptrs.resize(held);
+    ctx->used -= bytes - held_bytes;
+    bytes = held_bytes;
+  }
   void release() {
     for (void* p : ptrs) cudaFree(p);
     if (ctx) ctx->used -= bytes;
@@ -186,6 +193,7 @@ struct DevHierarchy {
   // sweep there) and the dynamic shared memory of a launch.
   void* d_pc = nullptr;
   int pc_rest = 0, pc_smem = 0;
+  std::vector<int> pc_chunk;  // rows per block of levels 1 .. pc_rest - 1
   bool lines = false;  // block-smoothed (anisotropic): level by level, sweeps on a cluster
 };
 

@@ -58,6 +58,33 @@ def test_coarse_cluster_cycle_bitwise(pkg, O, cells, boxes):
     dg.close()
 
 
+def test_cycle_within_small_budgets(pkg, O):
+    """A context too small for the coarse levels' plan as well still takes the grid, with the
+    same bits: budgets from ample down to the smallest that admits it."""
+    case = pkg.synth.case((60, 44, 24), 2.0, inflow=5.0, preconditioner="multigrid",
+                          boxes=[((20.0, 20.0, 0.0), (42.0, 44.0, 18.0)), ((70.0, 50.0, 0.0), (84.0, 70.0, 30.0))])
+    g = pkg.grid.Grid.build(case)
+    r = np.where(g.fluid == 1, np.random.default_rng(3).uniform(-1.0, 1.0, g.count), 0.0)
+    oz, _ = O.Grid(case).mg_apply(r)
+    lo, hi, held = 0, 1 << 28, set()
+    while hi - lo > 1 << 10:
+        mid = (lo + hi) // 2
+        ctx = pkg.pressure.Context(0, hbm_budget_bytes=mid)
+        try:
+            dg = pkg.pressure.DeviceGrid(g, ctx=ctx, preconditioner="multigrid")
+            try:
+                assert np.array_equal(bits(dg.precondition(r)), bits(oz))
+                held.add(dg.multigrid_stats()["allocated_bytes"])
+                hi = mid
+            finally:
+                dg.close()
+        except pkg.pressure.PressureError as e:
+            assert "budget" in str(e)
+            lo = mid
+        ctx.close()
+    assert len(held) == 2, held  # with the plan and without
+
+
 @pytest.mark.parametrize("cells, size", [
     ((9, 7, 100), (9.0, 7.0, 2.0)),      # more rows per line than two per lane
     ((70, 72, 5), (70.0, 72.0, 0.5)),    # more lines per dependency level than warps
