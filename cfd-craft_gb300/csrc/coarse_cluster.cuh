@@ -448,6 +448,7 @@ __device__ void cl_first_block(const ClCase& C, const CCase& D, int nu, unsigned
 }
 
 __global__ void __launch_bounds__(CLT, 1) k_coarse_cluster(const ClCase* cases, const CCase* cc, const MState* ST, int nu) {
+  pdl_enter();
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ ClCase C;
   const int ci = blockIdx.x / CLS;
@@ -629,6 +630,7 @@ __global__ void __launch_bounds__(CLT, 1) k_coarse_cluster(const ClCase* cases, 
       cl.sync();
     }
   }
+  pdl_leave();
   // The first level's iterate for the level above (the last cluster barrier also keeps every
   // block's shared memory alive until the stores into it have arrived).
   if (nd > 0) {

@@ -631,6 +631,7 @@ __device__ __forceinline__ void b_op(const FineCase* FC, MState* ST, const int2 
   tile_partial2(hi, lo, F, lt, seg_n);
 }
 __global__ void __launch_bounds__(TILE, 5) k_op(const FineCase* FC, MState* ST, const int2* tiles, const int* count) {
+  pdl_enter();
   __shared__ double sh[32];
   TILE_RANGE
   int cached_ = -1;  // case whose descriptor is in shared memory
@@ -644,6 +645,7 @@ __global__ void __launch_bounds__(TILE, 5) k_op(const FineCase* FC, MState* ST, 
     }
     b_op(FC, ST, t, cached_, sh, g.n);
   }
+  pdl_leave();
   close_seg(FC, ST, g, sh, FinOp());
 }
 
@@ -728,6 +730,7 @@ __device__ __forceinline__ void b_update(const FineCase* FC, MState* ST, const i
   }
 }
 __global__ void __launch_bounds__(TILE) k_update(const FineCase* FC, MState* ST, const int2* tiles, const int* count) {
+  pdl_enter();
   __shared__ double sh[32];
   TILE_RANGE
   int cached_ = -1;  // case whose descriptor is in shared memory
@@ -746,6 +749,7 @@ __global__ void __launch_bounds__(TILE) k_update(const FineCase* FC, MState* ST,
     b_update(FC, ST, t, n, cached_, g.n);
     ti += n;
   }
+  pdl_leave();
   close_seg(FC, ST, g, sh, FinUpdate());
 }
 
@@ -761,6 +765,7 @@ __device__ __forceinline__ void b_outer(const FineCase* FC, MState* ST, const in
     F.x64[rb + i] = F.x64[rb + i] + scale * (double)F.e[lay(r, (i + rp) & 1, nxh_, i >> 1)];
 }
 __global__ void __launch_bounds__(TILE) k_outer(const FineCase* FC, MState* ST, const int2* tiles, const int* count) {
+  pdl_enter();
   TILE_RANGE
   int cached_ = -1;  // case whose descriptor is in shared memory
   for (int ti = t0_; ti < t1_; ++ti) {
@@ -845,6 +850,7 @@ __device__ __forceinline__ void b_outer_resid(const FineCase* FC, MState* ST, co
   tile_partial(acc, F, lt, sh, seg_n);
 }
 __global__ void __launch_bounds__(TILE) k_outer_resid(const FineCase* FC, MState* ST, const int2* tiles, const int* count) {
+  pdl_enter();
   __shared__ double sh[32];
   TILE_RANGE
   int cached_ = -1;  // case whose descriptor is in shared memory
@@ -858,6 +864,7 @@ __global__ void __launch_bounds__(TILE) k_outer_resid(const FineCase* FC, MState
     }
     b_outer_resid(FC, ST, t, cached_, sh, g.n);
   }
+  pdl_leave();
   close_seg(FC, ST, g, sh, FinOuterResid());
 }
 
@@ -879,6 +886,7 @@ __device__ __forceinline__ void b_scale(const FineCase* FC, MState* ST, const in
         fp32 ? __double2float_rn(F.r64[rb + i]) * inv32 : (float)(F.r64[rb + i] * inv);
 }
 __global__ void __launch_bounds__(TILE) k_scale(const FineCase* FC, MState* ST, const int2* tiles, const int* count) {
+  pdl_enter();
   TILE_RANGE
   int cached_ = -1;  // case whose descriptor is in shared memory
   for (int ti = t0_; ti < t1_; ++ti) {
@@ -889,6 +897,7 @@ __global__ void __launch_bounds__(TILE) k_scale(const FineCase* FC, MState* ST, 
 }
 
 __global__ void k_start_state(MState* ST, int n) {
+  pdl_enter();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n && ST[i].state == SCALE) {
     ST[i].state = START;
@@ -945,6 +954,7 @@ __device__ __forceinline__ void b_rz(const FineCase* FC, MState* ST, const int2 
   }
 }
 __global__ void __launch_bounds__(TILE) k_rz(const FineCase* FC, MState* ST, const int2* tiles, const int* count) {
+  pdl_enter();
   __shared__ double sh[32];
   TILE_RANGE
   int cached_ = -1;  // case whose descriptor is in shared memory
@@ -963,6 +973,7 @@ __global__ void __launch_bounds__(TILE) k_rz(const FineCase* FC, MState* ST, con
     b_rz(FC, ST, t, n, cached_, g.n);
     ti += n;
   }
+  pdl_leave();
   close_seg(FC, ST, g, sh, FinRz());
 }
 
@@ -1015,6 +1026,7 @@ __device__ __forceinline__ void b_p(const FineCase* FC, MState* ST, const int2 t
   }
 }
 __global__ void __launch_bounds__(TILE) k_p(const FineCase* FC, MState* ST, const int2* tiles, const int* count) {
+  pdl_enter();
   TILE_RANGE
   int cached_ = -1;  // case whose descriptor is in shared memory
   for (int ti = t0_; ti < t1_;) {
@@ -1037,6 +1049,7 @@ __device__ __forceinline__ void b_v_rhs(const FineCase* FC, MState* ST, const in
   for (int c = sb + threadIdx.x; c < se; c += TILE) F.rhs0[c] = F.r32[c];
 }
 __global__ void __launch_bounds__(TILE) k_v_rhs(const FineCase* FC, MState* ST, const int2* tiles, const int* count) {
+  pdl_enter();
   TILE_RANGE
   int cached_ = -1;  // case whose descriptor is in shared memory
   for (int ti = t0_; ti < t1_; ++ti) {
@@ -1100,6 +1113,7 @@ __device__ __forceinline__ void b_rb(const FineCase* FC, MState* ST, const int2 
 }
 __global__ void __launch_bounds__(TILE, 5)
     k_rb(const FineCase* FC, MState* ST, const int2* tiles, const int* count, int color, int first) {
+  pdl_enter();
   TILE_RANGE
   int cached_ = -1;  // case whose descriptor is in shared memory
   for (int ti = t0_; ti < t1_; ++ti) {
@@ -1189,6 +1203,7 @@ constexpr int RB_THREADS = TILE + 32;  // RT consumer warps and one producer war
 __global__ void __launch_bounds__(RB_THREADS, 3) k_rb_tma(const FineCase* FC, MState* ST, const int2* tiles,
                                                           const int* count, int color, int first, int hmax, int sr,
                                                           int ns) {
+  pdl_enter();
   extern __shared__ __align__(128) unsigned char rb_dyn[];
   // Stage base on a 128-byte boundary (the launch adds 128 bytes of slack).
   unsigned char* const rb_smem =
@@ -1436,6 +1451,7 @@ __device__ __forceinline__ void b_v_resid(const FineCase* FC, MState* ST, const 
   }
 }
 __global__ void __launch_bounds__(TILE) k_v_resid(const FineCase* FC, MState* ST, const int2* tiles, const int* count) {
+  pdl_enter();
   TILE_RANGE
   int cached_ = -1;  // case whose descriptor is in shared memory
   for (int ti = t0_; ti < t1_; ++ti) {
@@ -1473,6 +1489,7 @@ __device__ __forceinline__ void bin_restrict(const FineCase& F, int q) {
 // rhs1 = R res0: level-1 rows gather their level-0 children. Tiles index level-1 rows.
 __global__ void __launch_bounds__(TILE) k_v_restrict(const FineCase* FC, MState* ST, const int2* tiles1,
                                                      const int* count) {
+  pdl_enter();
   const int n = *count;
   for (int ti = blockIdx.x; ti < n; ti += gridDim.x) {
     const int2 t = tiles1[ti];
@@ -1566,6 +1583,7 @@ __device__ __forceinline__ void b_v_prolong(const FineCase* FC, MState* ST, cons
   }
 }
 __global__ void __launch_bounds__(TILE) k_v_prolong(const FineCase* FC, MState* ST, const int2* tiles, const int* count) {
+  pdl_enter();
   TILE_RANGE
   int cached_ = -1;  // case whose descriptor is in shared memory
   for (int ti = t0_; ti < t1_;) {
@@ -1583,6 +1601,7 @@ __global__ void __launch_bounds__(TILE) k_v_prolong(const FineCase* FC, MState* 
 // Gauge of level-0 closed groups: one block per (case, group); members strided.
 // which: 0 rhs0, 1 x0, 2 res0.
 __global__ void k_center0(const FineCase* FC, MState* ST, const int2* gtab, const int* count, int which) {
+  pdl_enter();
   __shared__ double sh[32];
   __shared__ float mean;
   const int n = *count;
@@ -1845,6 +1864,7 @@ __device__ void c_sweep(const CLev& L, bool backward, int pass, bool gs_on) {
 // nu: Gauss-Seidel sweeps before and after the coarse correction (l1-Jacobi levels run
 // the next even count, so their iterate ends in x).
 __global__ void __launch_bounds__(CT) k_coarse(const CCase* cases, const MState* ST, int nu) {
+  pdl_enter();
   __shared__ double sh[32];
   const int csz = (int)cg::this_cluster().num_blocks();
   const int ci = blockIdx.x / csz;
@@ -2356,6 +2376,7 @@ __device__ __forceinline__ void b_rhs(const FineCase* FC, MState* ST, const int2
   }
 }
 __global__ void __launch_bounds__(TILE) k_rhs(const FineCase* FC, MState* ST, const int2* tiles, const int* count) {
+  pdl_enter();
   TILE_RANGE
   int cached_ = -1;  // case whose descriptor is in shared memory
   for (int ti = t0_; ti < t1_; ++ti) {
@@ -2388,6 +2409,7 @@ __device__ __forceinline__ void b_norm(const FineCase* FC, MState* ST, const int
   tile_partial(acc, F, lt, sh, seg_n);
 }
 __global__ void __launch_bounds__(TILE) k_norm(const FineCase* FC, MState* ST, const int2* tiles, const int* count) {
+  pdl_enter();
   __shared__ double sh[32];
   TILE_RANGE
   int cached_ = -1;  // case whose descriptor is in shared memory
@@ -2401,6 +2423,7 @@ __global__ void __launch_bounds__(TILE) k_norm(const FineCase* FC, MState* ST, c
     }
     b_norm(FC, ST, t, cached_, sh, g.n);
   }
+  pdl_leave();
   close_seg(FC, ST, g, sh, FinNorm());
 }
 
@@ -2430,6 +2453,7 @@ __device__ __forceinline__ void b_addp(const FineCase* FC, MState* ST, const int
   for (int c = cb + threadIdx.x; c < ce; c += TILE) F.pfield[c] = __dadd_rn(F.pfield[c], F.x64[c]);
 }
 __global__ void __launch_bounds__(TILE) k_addp(const FineCase* FC, MState* ST, const int2* tiles, const int* count) {
+  pdl_enter();
   TILE_RANGE
   int cached_ = -1;  // case whose descriptor is in shared memory
   for (int ti = t0_; ti < t1_; ++ti) {
@@ -3608,8 +3632,10 @@ void cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, unsigned c
   at[0].val.clusterDim.x = size;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
 }
 
 // The coarse levels of every case: one cluster per case where its levels allow it
@@ -3617,7 +3643,7 @@ void cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, unsigned c
 void launch_coarse(cfdg_batch* B, cudaStream_t s) {
   const unsigned nc = (unsigned)B->cases.size();
   cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   if (B->any_tab[1]) launch_phases<1>(B, 1, s);
   if (B->any_cl) {
     cluster_config(cfg, at, nc, CLS, CLT, B->cl_smem, s);
@@ -3635,14 +3661,14 @@ void launch_coarse(cfdg_batch* B, cudaStream_t s) {
 }
 
 #define FINE(K, W, ...) \
-  K<<<grid_of(K, TILE, B->g_fine), TILE, 0, s>>>(B->d_fc, B->d_st, (W).tiles, (W).counts, ##__VA_ARGS__)
+  launch_pdl(K, grid_of(K, TILE, B->g_fine), TILE, 0, s, B->d_fc, B->d_st, (W).tiles, (W).counts, ##__VA_ARGS__)
 
 // One red-black half sweep of level 0 over the work-list: the staged kernel when every case
 // has its tensor maps, else the register kernel (the same bits either way).
 void launch_rb(cfdg_batch* B, const WorkLists& W, int color, int first, cudaStream_t s) {
   if (B->rb_tma)
-    k_rb_tma<<<B->rb_grid, RB_THREADS, B->rb_smem, s>>>(B->d_fc, B->d_st, W.tiles, W.counts, color, first,
-                                                        B->rb_hmax, B->rb_sr, B->rb_ns);
+    launch_pdl(k_rb_tma, B->rb_grid, RB_THREADS, B->rb_smem, s, B->d_fc, B->d_st, W.tiles, W.counts, color, first,
+               B->rb_hmax, B->rb_sr, B->rb_ns);
   else
     FINE(k_rb, W, color, first);
 }
@@ -3651,17 +3677,17 @@ void enqueue_vcycle(cfdg_batch* B, cudaStream_t s) {
   const WorkLists& W = B->run;
   if (B->any_groups) {
     FINE(k_v_rhs, W);
-    k_center0<<<grid_of(k_center0, 256, B->g_g), 256, 0, s>>>(B->d_fc, B->d_st, W.gtab, W.counts + 3, 0);
+    launch_pdl(k_center0, grid_of(k_center0, 256, B->g_g), 256, 0, s, B->d_fc, B->d_st, W.gtab, W.counts + 3, 0);
   }
   // nu0 forward sweeps: red, black, red, black, ... (the first red starts from x = 0).
   for (int sw = 0; sw < B->nu0; ++sw) {
     launch_rb(B, W, 0, sw == 0 ? 1 : 0, s);
     launch_rb(B, W, 1, 0, s);
   }
-  if (B->any_groups) k_center0<<<grid_of(k_center0, 256, B->g_g), 256, 0, s>>>(B->d_fc, B->d_st, W.gtab, W.counts + 3, 1);
+  if (B->any_groups) launch_pdl(k_center0, grid_of(k_center0, 256, B->g_g), 256, 0, s, B->d_fc, B->d_st, W.gtab, W.counts + 3, 1);
   FINE(k_v_resid, W);
-  if (B->any_groups) k_center0<<<grid_of(k_center0, 256, B->g_g), 256, 0, s>>>(B->d_fc, B->d_st, W.gtab, W.counts + 3, 2);
-  k_v_restrict<<<grid_of(k_v_restrict, TILE, B->g_1), TILE, 0, s>>>(B->d_fc, B->d_st, W.tiles1, W.counts + 1);
+  if (B->any_groups) launch_pdl(k_center0, grid_of(k_center0, 256, B->g_g), 256, 0, s, B->d_fc, B->d_st, W.gtab, W.counts + 3, 2);
+  launch_pdl(k_v_restrict, grid_of(k_v_restrict, TILE, B->g_1), TILE, 0, s, B->d_fc, B->d_st, W.tiles1, W.counts + 1);
   launch_coarse(B, s);
   FINE(k_v_prolong, W);
   // nu0 backward sweeps: black, red, ...
@@ -3669,7 +3695,7 @@ void enqueue_vcycle(cfdg_batch* B, cudaStream_t s) {
     launch_rb(B, W, 1, 0, s);
     launch_rb(B, W, 0, 0, s);
   }
-  if (B->any_groups) k_center0<<<grid_of(k_center0, 256, B->g_g), 256, 0, s>>>(B->d_fc, B->d_st, W.gtab, W.counts + 3, 1);
+  if (B->any_groups) launch_pdl(k_center0, grid_of(k_center0, 256, B->g_g), 256, 0, s, B->d_fc, B->d_st, W.gtab, W.counts + 3, 1);
 }
 
 // One iteration of the per-case state machine.
@@ -3681,7 +3707,7 @@ void enqueue_iteration(cfdg_batch* B, cudaStream_t s) {
   FINE(k_outer, W);
   FINE(k_outer_resid, W);
   FINE(k_scale, W);
-  k_start_state<<<(nc + 127) / 128, 128, 0, s>>>(B->d_st, nc);
+  launch_pdl(k_start_state, (nc + 127) / 128, 128, 0, s, B->d_st, nc);
   enqueue_vcycle(B, s);
   FINE(k_rz, W);
   FINE(k_p, W);
@@ -3926,8 +3952,9 @@ int cfdg_mixed_pack(cfdg_batch* B) {
     }
     int clusters = 0;
     cudaLaunchConfig_t cfg;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     cluster_config(cfg, at, 1, CLS, CLT, B->cl_smem, s);
+    cfg.numAttrs = 1;
     if (cudaFuncSetAttribute(k_coarse_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
         cudaFuncSetAttribute(k_coarse_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, CL_SMEM) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&clusters, k_coarse_cluster, &cfg) != cudaSuccess || clusters < 1) {
@@ -4415,7 +4442,7 @@ int cfdg_batch_time_kernel(cfdg_batch* B, int32_t which, int32_t reps, double* m
         break;
       case 7:  // level-0 residual and its restriction to level 1
         FINE(k_v_resid, B->run);
-        k_v_restrict<<<grid_of(k_v_restrict, TILE, B->g_1), TILE, 0, s>>>(B->d_fc, B->d_st, B->run.tiles1,
+        launch_pdl(k_v_restrict, grid_of(k_v_restrict, TILE, B->g_1), TILE, 0, s, B->d_fc, B->d_st, B->run.tiles1,
                                                                           B->run.counts + 1);
         break;
       case 9:  // e += alpha p, r -= alpha q with |r|^2

@@ -38,4 +38,12 @@ struct Scalars {
   unsigned counter;
 };
 
+#ifdef __CUDACC__
+// First statement of every kernel launched by launch_pdl, in every thread: waits until the
+// kernels before it have finished and their writes are visible.
+__device__ __forceinline__ void pdl_enter() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The next launch may schedule its blocks once every block is past this point (or has exited).
+__device__ __forceinline__ void pdl_leave() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+#endif
+
 }  // namespace cfdg

@@ -197,6 +197,23 @@ struct DevHierarchy {
   bool lines = false;  // block-smoothed (anisotropic): level by level, sweeps on a cluster
 };
 
+// A launch whose blocks may be scheduled while the kernel before it is still running: every
+// kernel launched this way begins with pdl_enter.
+template <class... Params, class... Args>
+void launch_pdl(void (*kernel)(Params...), int grid, int threads, size_t smem, cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid, 1, 1);
+  cfg.blockDim = dim3((unsigned)threads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+}
+
 }  // namespace cfdg
 
 using namespace cfdg;
