@@ -6,7 +6,7 @@
 // CLS blocks per case the barrier is the cluster's (0.3 us) and the iterates stay in the
 // blocks' shared memory. Measured per cycle: 128x128x64 (131,072 rows on the first coarse
 // level) 256 -> 55 us, 100x84x50 235 -> 45 us, sixteen cases of 128x128x64 368 -> 158 us
-// (seven clusters fit the device at once), 8.4 M cells (first level grid-wide) 331 -> 215 us.
+// (seven clusters fit the device at once), 8.4 M cells (first level grid-wide) 331 -> 136 us.
 // What bounds it now is the chain of barriers and shared-memory round trips.
 //
 // Levels laid out as the grid of 2x2x2 bins (build_case) are split into slabs of bin layers
@@ -24,8 +24,10 @@
 // and the iterate in global memory (one L2 round trip a phase). Small bin levels and the
 // levels below (any aggregation level of at most two colours without closed groups, the
 // terminal blocks) run in the cluster's first block with block barriers. Levels too large for
-// this stay with the grid-wide phases (k_coarse_all), which hand over at the first cluster
-// level.
+// this run grid-wide: bin levels over their row types (k_up_*), others in the phases of
+// k_coarse_all, which hand over at the first cluster level. (Handing over one level later than
+// the shared memory asks for was slower: 100x84x50 43 -> 55 us, eight uneven cases 6.73 -> 7.24
+// ms a projection.)
 //
 // Every row sees the operations of the grid-wide phases in the same order (its entries and
 // children in the order of the hierarchy), so the results are the same bits (tested against
@@ -61,6 +63,15 @@ struct ClCase {
   float alpha;       // scale of the coarse corrections
   int smem;          // bytes
   ClBin b[CLB];
+};
+// The bin levels above the cluster's first one (lv[n], whose right-hand side they give and whose
+// iterate they take): grid-wide kernels over the same row types (k_up_*).
+constexpr int CLUP = 4;
+struct ClUp {
+  int n;
+  float alpha;
+  float* rhs[CLUP + 1];
+  ClBin lv[CLUP + 1];
 };
 static_assert(sizeof(ClCase) % 8 == 0, "ClCase is copied to shared memory in 8-byte words");
 
@@ -640,4 +651,83 @@ __global__ void __launch_bounds__(CLT, 1) k_coarse_cluster(const ClCase* cases, 
       V0.B->gx[c * V0.B->h + at + q] = V0.x[c * V0.ldx + V0.B->plane + q];
     }
   }
+}
+
+// ------------------------------------------------------------ levels above the clusters
+// One launch a phase over every case (blockIdx.y), UPR rows a thread. The row types make a row
+// 14 bytes of traffic (right-hand side, type, own and other colour) where its index list has
+// about 70, and a launch that follows the one before closely costs less than the grid barrier
+// and work search of the cooperative phases: the coarse levels of 8.4 M cells (1,048,576 rows on
+// the first) 206 -> 136 us, of 160x160x80 cells 166 -> 99 us, the projections 11.97 -> 10.81 ms
+// and, of eight uneven cases, 7.53 -> 6.73 ms.
+constexpr int UPT = 256, UPR = 2;
+
+template <int C, bool FIRST>
+__global__ void __launch_bounds__(UPT) k_up_sweep(const ClUp* ups, const MState* ST, int l) {
+  pdl_enter();
+  const ClUp& U = ups[blockIdx.y];
+  if (l >= U.n || !active(ST, blockIdx.y)) return;
+  const ClBin& B = U.lv[l];
+  const int h = B.h;
+  const float* __restrict__ xo = B.gx + (1 - C) * h;
+  unsigned type[UPR];
+  float v[UPR];
+#pragma unroll
+  for (int m = 0; m < UPR; ++m) {
+    const int q = (blockIdx.x * UPR + m) * UPT + threadIdx.x;
+    type[m] = q < h ? __ldg(&B.gtype[C * h + q]) : 0;
+    v[m] = q < h ? B.grhs[C * h + q] : 0.0f;
+  }
+#pragma unroll
+  for (int m = 0; m < UPR; ++m) {
+    const int q = (blockIdx.x * UPR + m) * UPT + threadIdx.x;
+    if (q >= h) break;
+    const float4 *t = B.gtab + 3 * type[m], b = __ldg(t + 1);
+    if (!FIRST) {
+      ClRow r;
+      r.a = __ldg(t);
+      r.b = b;
+      r.o = __ldg(reinterpret_cast<const int4*>(t + 2));
+      v[m] = cl_sum<true>(v[m], xo + q, r);
+    }
+    B.gx[C * h + q] = v[m] * b.w;
+  }
+}
+
+// The next level's right-hand side from the colour-0 residuals of its children.
+__global__ void __launch_bounds__(UPT) k_up_restrict(const ClUp* ups, const MState* ST, int l) {
+  pdl_enter();
+  const ClUp& U = ups[blockIdx.y];
+  if (l >= U.n || !active(ST, blockIdx.y)) return;
+  const ClBin &B = U.lv[l], &N = U.lv[l + 1];
+  const int e = blockIdx.x * UPT + threadIdx.x;
+  if (e >= 2 * N.h) return;
+  const int c = e >= N.h ? 1 : 0, q = e - c * N.h;
+  ClView W;
+  W.B = &N;
+  W.k0 = 0;
+  const int order = __float_as_int(__ldg(&N.gtab[3 * __ldg(&N.gtype[e]) + 2].w));
+  U.rhs[l + 1][e] = cl_restrict(W, c, q, order, B.nby, B.nbz, B.nbh, [&](int k, int j, int s) {
+    const int f = (k * B.nby + j) * B.nbh + s;
+    const float4* t = B.gtab + 3 * __ldg(&B.gtype[f]);
+    ClRow r;
+    r.a = __ldg(t);
+    r.b = __ldg(t + 1);
+    r.o = __ldg(reinterpret_cast<const int4*>(t + 2));
+    return B.grhs[f] - cl_sum<false>(__fmul_rn(r.b.z, B.gx[f]), B.gx + B.h + f, r);
+  });
+}
+
+// Colour 0 takes its correction (colour 1 is swept next without being read).
+__global__ void __launch_bounds__(UPT) k_up_prolong(const ClUp* ups, const MState* ST, int l) {
+  pdl_enter();
+  const ClUp& U = ups[blockIdx.y];
+  if (l >= U.n || !active(ST, blockIdx.y)) return;
+  const ClBin &B = U.lv[l], &N = U.lv[l + 1];
+  const int q = blockIdx.x * UPT + threadIdx.x;
+  if (q >= B.h) return;
+  ClView V;
+  V.B = &B;
+  V.k0 = 0;
+  B.gx[q] = __fadd_rn(B.gx[q], __fmul_rn(U.alpha, cl_parent_global(V, N, q)));
 }

@@ -2517,7 +2517,10 @@ struct CaseState {
   Arena arena;
   FineCase F{};
   CCase C{};
-  ClCase cl{};  // on: the coarse levels from cl.lc run on a cluster of their own
+  // on: the coarse levels from cl.lc run on a cluster of their own, those above grid-wide (over
+  // their row types, where all are bin levels: up).
+  ClCase cl{};
+  ClUp up{};
   std::vector<std::vector<int32_t>> colors;  // per coarse level: colour offsets (host copy)
   struct LevelStats {
     long long rows, nnz, ell, groups, blocks;
@@ -2608,6 +2611,25 @@ struct BinMatrix {
 };
 constexpr int CL_TYPES = 2048;  // more types than this: the level is not planned as a bin level
 
+ClBin bin_shape(const BinMatrix& M, const CLev& L) {
+  ClBin B{};
+  B.nby = M.nb[1], B.nbz = M.nb[2], B.nbh = M.nbh, B.h = M.h, B.plane = M.nb[1] * M.nbh;
+  auto magic = [](int d) { return (unsigned)((((uint64_t)1 << 32) + d - 1) / d); };
+  B.mh = magic(B.nbh), B.my = magic(B.nby);
+  B.ntypes = (int)M.tab.size();
+  B.grhs = L.rhs, B.gx = L.x, B.gres = L.res;
+  return B;
+}
+int upload_types(Arena& A, cudaStream_t s, const BinMatrix& M, ClBin& B) {
+  unsigned short* dt;
+  std::array<uint32_t, 12>* dr;
+  if (int e = A.upload(&dt, M.type, s)) return e;
+  if (int e = A.upload(&dr, M.tab, s)) return e;
+  B.gtype = dt;
+  B.gtab = reinterpret_cast<const float4*>(dr);
+  return 0;
+}
+
 // Plans k_coarse_cluster for a case whose coarse levels allow it (aggregation levels of at
 // most two colours without closed groups) and uploads what it needs; bins[l] holds the bin
 // levels among levels 1.. (h == 0: not a bin level). Levels are split over the cluster's
@@ -2616,9 +2638,11 @@ constexpr int CL_TYPES = 2048;  // more types than this: the level is not planne
 // without a bin layout are split above 1,500 rows. The cluster starts at the first level
 // whose slabs fit the blocks' registers and shared memory; a level split by rows is taken up
 // to 32,768 of them (four a thread).
+// Where the levels above are bin levels, too, U describes them.
 int plan_cluster(Arena& A, cudaStream_t s, const CCase& C, const std::vector<int>& jacobi, const std::vector<BinMatrix>& bins,
-                 float alpha, ClCase& K) {
+                 float alpha, ClCase& K, ClUp& U) {
   K = ClCase{};
+  U = ClUp{};
   for (int l = 1; l <= C.nl; ++l)
     if (C.lv[l - 1].ngroups || jacobi[l] || C.lv[l - 1].ncolors > 2) return 0;
   for (int lc = 1; lc <= C.nl; ++lc) {
@@ -2643,9 +2667,7 @@ int plan_cluster(Arena& A, cudaStream_t s, const CCase& C, const std::vector<int
     for (int t = 0; t < T.nb && ok; ++t) {
       const BinMatrix& M = bins[lc + t];
       ClBin& B = T.b[t];
-      B.nby = M.nb[1], B.nbz = M.nb[2], B.nbh = M.nbh, B.h = M.h, B.plane = M.nb[1] * M.nbh;
-      auto magic = [](int d) { return (unsigned)((((uint64_t)1 << 32) + d - 1) / d); };
-      B.mh = magic(B.nbh), B.my = magic(B.nby);
+      B = bin_shape(M, C.lv[lc + t - 1]);
       B.layers = B.nbz;
       if (t < T.nd) {
         B.layers = 0;
@@ -2657,12 +2679,9 @@ int plan_cluster(Arena& A, cudaStream_t s, const CCase& C, const std::vector<int
       const size_t rows = (size_t)B.layers * B.plane;
       ok = (uint64_t)rows * B.nbh < ((uint64_t)1 << 32);  // cl_div
       B.x = take(2 * (rows + 2 * B.plane) * 4);
-      B.ntypes = (int)M.tab.size();
       B.tab = take(48 * M.tab.size());
       B.rhs = B.type = -1;
       if (t > 0 || T.nd == 0 || rows > (size_t)CLR * CLT) B.rhs = take(2 * rows * 4), B.type = take(2 * rows * 2);
-      const CLev& L = C.lv[lc + t - 1];
-      B.grhs = L.rhs, B.gx = L.x, B.gres = L.res;
     }
     for (int t = T.nb; t < T.nb + T.ng && ok; ++t) {
       const CLev& L = C.lv[lc + t - 1];
@@ -2677,14 +2696,20 @@ int plan_cluster(Arena& A, cudaStream_t s, const CCase& C, const std::vector<int
     if (!ok || at > (size_t)CL_SMEM) continue;
     T.smem = (int)at;
     T.on = 1;
-    for (int t = 0; t < T.nb; ++t) {
-      ClBin& B = T.b[t];
-      unsigned short* dt;
-      std::array<uint32_t, 12>* dr;
-      if (int e = A.upload(&dt, bins[lc + t].type, s)) return e;
-      if (int e = A.upload(&dr, bins[lc + t].tab, s)) return e;
-      B.gtype = dt;
-      B.gtab = reinterpret_cast<const float4*>(dr);
+    for (int t = 0; t < T.nb; ++t)
+      if (int e = upload_types(A, s, bins[lc + t], T.b[t])) return e;
+    bool up = T.lc > 0 && T.lc <= CLUP && T.nb > 0;
+    for (int l = 1; l < lc; ++l)
+      up = up && bins[l].h > 0 && (uint64_t)bins[l].h * bins[l].nbh < ((uint64_t)1 << 32);  // cl_div
+    if (up) {
+      U.n = T.lc;
+      U.alpha = alpha;
+      for (int l = 1; l < lc; ++l) {
+        U.lv[l - 1] = bin_shape(bins[l], C.lv[l - 1]);
+        if (int e = upload_types(A, s, bins[l], U.lv[l - 1])) return e;
+      }
+      U.lv[T.lc] = T.b[0];
+      for (int l = 0; l <= T.lc; ++l) U.rhs[l] = C.lv[l].rhs;
     }
     K = T;
     return 0;
@@ -3299,7 +3324,7 @@ int build_case(cfdg_grid* G, CaseState& cs) {
       for (int a = 0; a < 3; ++a) M.nb[a] = B.nb[a];
       M.nbh = B.nbh, M.h = B.h;
     }
-    if (int e = plan_cluster(A, s, C, ljacobi, bins, alpha, cs.cl)) return e;
+    if (int e = plan_cluster(A, s, C, ljacobi, bins, alpha, cs.cl, cs.up)) return e;
   }
   F.n1 = C.lv[0].n;
   F.rhs1 = C.lv[0].rhs;
@@ -3372,7 +3397,11 @@ struct cfdg_batch {
   bool any_tab[2] = {false, false};
   // The cluster kernel's cases, and the shared memory the largest of them asks for.
   ClCase* d_cl = nullptr;
-  std::vector<char> clustered;
+  ClUp* d_up = nullptr;
+  std::vector<ClCase> plan;
+  std::vector<ClUp> ups;
+  int up_levels = 0;             // most grid-wide bin levels of a case
+  int up_h[CLUP] = {0, 0, 0, 0}, up_next[CLUP] = {0, 0, 0, 0};  // most rows per colour there and on the level after
   bool any_cl = false;
   int cl_smem = 0;
   int nlev_all = 0;
@@ -3512,7 +3541,7 @@ int fill_lists(cfdg_batch* B, WorkLists& W, const std::vector<char>& on, cudaStr
 int fill_tab(cfdg_batch* B, int which, const std::vector<char>& on, cudaStream_t s) {
   const int nc = (int)B->cases.size(), nlev = B->nlev_all, w = nc + 1;
   CoarseTab& T = B->h_tab[which];
-  auto depth = [&](int i) { return which ? B->cases[i]->cl.lc : B->cases[i]->C.nl; };
+  auto depth = [&](int i) { return which ? B->plan[i].lc : B->cases[i]->C.nl; };
   static thread_local std::vector<int32_t> buf;
   const size_t words = (size_t)nlev * w * (6 + 2 * MAXC);
   buf.assign(words, 0);
@@ -3597,7 +3626,7 @@ int set_active(cfdg_batch* B, cudaStream_t s) {
     if (!B->any_tab[which]) continue;
     std::vector<char> on(B->active);
     for (size_t i = 0; i < on.size(); ++i)
-      on[i] = on[i] && (which ? B->clustered[i] && B->cases[i]->cl.lc > 0 : !B->clustered[i]);
+      on[i] = on[i] && (which ? B->plan[i].on && B->plan[i].lc > 0 && B->ups[i].n == 0 : !B->plan[i].on);
     if (int e = fill_tab(B, which, on, s)) return e;
   }
   return 0;
@@ -3644,11 +3673,31 @@ void launch_coarse(cfdg_batch* B, cudaStream_t s) {
   const unsigned nc = (unsigned)B->cases.size();
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute at[2];
+  const auto up = [&](void (*k)(const ClUp*, const MState*, int), int l, int rows) {
+    launch_pdl(k, dim3((unsigned)((rows + UPT - 1) / UPT), nc), UPT, 0, s, B->d_up, B->d_st, l);
+  };
+  const auto sweep = [&](int l, int c, bool first) {
+    up(c ? k_up_sweep<1, false> : first ? k_up_sweep<0, true> : k_up_sweep<0, false>, l, (B->up_h[l] + UPR - 1) / UPR);
+  };
   if (B->any_tab[1]) launch_phases<1>(B, 1, s);
+  for (int l = 0; l < B->up_levels; ++l) {
+    for (int sw = 0; sw < B->nuc; ++sw) {
+      sweep(l, 0, sw == 0);
+      sweep(l, 1, false);
+    }
+    up(k_up_restrict, l, 2 * B->up_next[l]);
+  }
   if (B->any_cl) {
     cluster_config(cfg, at, nc, CLS, CLT, B->cl_smem, s);
     cudaLaunchKernelEx(&cfg, k_coarse_cluster, (const ClCase*)B->d_cl, (const CCase*)B->d_cc, (const MState*)B->d_st,
                        B->nuc);
+  }
+  for (int l = B->up_levels - 1; l >= 0; --l) {
+    up(k_up_prolong, l, B->up_h[l]);
+    for (int sw = 0; sw < B->nuc; ++sw) {
+      sweep(l, 1, false);
+      sweep(l, 0, false);
+    }
   }
   if (B->any_tab[1]) launch_phases<2>(B, 1, s);
   if (!B->any_tab[0]) return;
@@ -3943,11 +3992,14 @@ int cfdg_mixed_pack(cfdg_batch* B) {
   // Which cases run their coarse levels on clusters: all that have a plan, when such a cluster
   // fits the device (and, for those with levels above it, the cooperative launch).
   {
-    std::vector<ClCase> cl(nc);
+    std::vector<ClCase>& cl = B->plan;
+    std::vector<ClUp>& up = B->ups;
     B->cl_smem = 0;
+    cl.assign(nc, ClCase{});
+    up.assign(nc, ClUp{});
     for (int i = 0; i < nc; ++i) {
-      const ClCase& K = B->cases[i]->cl;
-      if (K.on && (K.lc == 0 || B->coop)) cl[i] = K;
+      const CaseState& K = *B->cases[i];
+      if (K.cl.on && (K.cl.lc == 0 || K.up.n > 0 || B->coop)) cl[i] = K.cl, up[i] = K.up;
       B->cl_smem = std::max(B->cl_smem, cl[i].smem);
     }
     int clusters = 0;
@@ -3959,16 +4011,24 @@ int cfdg_mixed_pack(cfdg_batch* B) {
         cudaFuncSetAttribute(k_coarse_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, CL_SMEM) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&clusters, k_coarse_cluster, &cfg) != cudaSuccess || clusters < 1) {
       cudaGetLastError();
-      for (ClCase& K : cl) K = ClCase{};
+      cl.assign(nc, ClCase{});
+      up.assign(nc, ClUp{});
     }
-    B->clustered.assign(nc, 0);
     B->any_cl = B->any_tab[0] = B->any_tab[1] = false;
+    B->up_levels = 0;
+    std::fill(B->up_h, B->up_h + CLUP, 0);
+    std::fill(B->up_next, B->up_next + CLUP, 0);
     for (int i = 0; i < nc; ++i) {
-      B->clustered[i] = cl[i].on != 0;
       B->any_cl |= cl[i].on != 0;
       B->any_tab[0] |= !cl[i].on;
-      B->any_tab[1] |= cl[i].on && cl[i].lc > 0;
+      B->any_tab[1] |= cl[i].on && cl[i].lc > 0 && up[i].n == 0;
+      B->up_levels = std::max(B->up_levels, up[i].n);
+      for (int l = 0; l < up[i].n; ++l) {
+        B->up_h[l] = std::max(B->up_h[l], up[i].lv[l].h);
+        B->up_next[l] = std::max(B->up_next[l], up[i].lv[l + 1].h);
+      }
     }
+    if (int e = A.upload(&B->d_up, up, s)) return e;
     if (int e = A.upload(&B->d_cl, cl, s)) return e;
     CU(cudaStreamSynchronize(s));
   }

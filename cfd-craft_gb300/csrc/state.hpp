@@ -200,9 +200,9 @@ struct DevHierarchy {
 // A launch whose blocks may be scheduled while the kernel before it is still running: every
 // kernel launched this way begins with pdl_enter.
 template <class... Params, class... Args>
-void launch_pdl(void (*kernel)(Params...), int grid, int threads, size_t smem, cudaStream_t s, Args... args) {
+void launch_pdl(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t s, Args... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid, 1, 1);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3((unsigned)threads, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;

@@ -43,6 +43,7 @@ SHAPES = {
     "one block": [((24, 20, 16), 2.0, 1), ((12, 10, 8), 2.0, 0)],
     "thin": [((96, 80, 10), 2.0, 4), ((30, 8, 60), 2.0, 0)],
     "three levels split": [((128, 96, 64), 2.0, 12)],
+    "two grid-wide levels": [((500, 500, 8), 2.0, 4), ((40, 36, 27), 2.0, 2)],
     "grid-wide first level": [((176, 160, 80), 2.0, 10), ((48, 48, 48), 2.0, 3)],
 }
 
