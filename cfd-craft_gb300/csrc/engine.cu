@@ -2226,6 +2226,7 @@ __global__ void k_ssprk_combine(FlowDev D, double* __restrict__ u, const double*
 // so the same bits; zeros, subnormals, infinities and NaNs take the FP64 instruction),
 // and `x + 0.0` only turns -0.0 into +0.0.
 // A factor 2^e (value v) when `ok`; otherwise the factor is not a power of two.
+enum ScalarDiv { DIVIDE = 0, POW2 = 1, RECIP = 2, RECIP2 = 3 };
 struct Pow2 {
   double v;
   int e;
@@ -2246,7 +2247,21 @@ struct ScalarDev {
   // (interior, inlet, outlet), equal bit for bit on every such face.
   double area_k[3][3], dist_k[3][3];
   Pow2 area_p[3][3], inv_dist_p[3][3];
+  double rdist[3][3], rvolume;  // reciprocals as div_pre takes them
 };
+
+// v / d by a known positive divisor, as div_pre (three operations of 31 ns, five with EXTRA,
+// against 272 ns). A zero (a field is zero wherever nothing has arrived) is its own quotient.
+template <bool EXTRA>
+__device__ __forceinline__ double div_known(double v, double d, double rd) {
+  const double r = EXTRA ? fabs(rd) : rd;
+  double q = __dmul_rn(v, r);
+  q = __fma_rn(__fma_rn(-q, d, v), r, q);
+  if (EXTRA) q = __fma_rn(__fma_rn(-q, d, v), r, q);
+  const int hi = __double2hiint(v) & 0x7fffffff;
+  if (((unsigned)hi >> 20) - 123u > 1800u) q = (hi | __double2loint(v)) == 0 ? v : div_rare(v, d);
+  return q;
+}
 
 constexpr int STX = 32, STY = 8;  // cells of one transport tile in x and y (its z extent is chosen per grid)
 
@@ -2330,19 +2345,33 @@ __device__ __forceinline__ double mc_slope(double lo, double xc, double hi) {
 // The flux / volume of face f on axis a between cells lo_cell and hi_cell (its structural
 // neighbours, -1 outside the domain), evaluated on the field x; false if the face does not
 // transport. UNI: the layout's lo/hi (interior iff both are fluid) and per-axis constants.
-// P2 (with UNI): the volume and every transporting face's area and distance are powers of
-// two, so the products and quotients by them go through the exponent field.
+// DIV, other than DIVIDE with UNI only: POW2 where the volume and every transporting face's
+// area and distance are powers of two, so the products and quotients by them go through the
+// exponent field; RECIP, RECIP2 quotients through the constants' reciprocals (RECIP2 where one
+// of those needs the extra correction).
 // MUSCL (transport.rs:670-694): the donor is the upwind cell's value plus (flow towards hi)
 // or minus half its slope along a, whose neighbours are the cells across the upwind cell's
 // two faces on a (faces f -+ one face stride; the grid is not periodic, so both exist).
-template <bool UNI, bool P2, bool MUSCL = false>
+struct FaceIn {  // a face's kind and velocity, the values and diffusivities of its cells
+  uint8_t k;
+  double u, xl, xr, dl, dr;
+};
+// The loads of a face, none behind a branch (a cell outside the domain is replaced by the
+// other one: its value is not used).
+__device__ __forceinline__ FaceIn face_load(const ScalarDev& D, long long f, long long lo_cell, long long hi_cell,
+                                            const double* __restrict__ x, const double* __restrict__ u,
+                                            const double* __restrict__ d) {
+  const long long l = lo_cell >= 0 ? lo_cell : hi_cell, h = hi_cell >= 0 ? hi_cell : lo_cell;
+  return FaceIn{D.kind[f], u[f], x[l], x[h], d[l], d[h]};
+}
+template <bool UNI, int DIV, bool MUSCL = false>
 __device__ __forceinline__ bool face_eval(const ScalarDev& D, int a, long long f, long long lo_cell,
-                                          long long hi_cell, const double* __restrict__ x,
-                                          const double* __restrict__ u, const double* __restrict__ d, double& pv) {
-  const uint8_t k = D.kind[f];
+                                          long long hi_cell, const double* __restrict__ x, const FaceIn& in,
+                                          double& pv) {
+  const uint8_t k = in.k;
   if (k != INTERIOR && k != INLET && k != OUTLET) return false;
   bool hl, hh;
-  double area = 0.0, dist = 0.0;
+  double area = 0.0, dist = 0.0, rdist = 0.0;
   Pow2 area_p{0.0, 0, 0}, inv_dist_p{0.0, 0, 0};
   if (UNI) {
     if (k == INTERIOR) {
@@ -2352,12 +2381,13 @@ __device__ __forceinline__ bool face_eval(const ScalarDev& D, int a, long long f
       hh = hi_cell >= 0 && D.fluid[hi_cell];
     }
     const int t = transport_slot(k);
-    if (P2) {
+    if (DIV == POW2) {
       area_p = D.area_p[a][t];
       inv_dist_p = D.inv_dist_p[a][t];
     } else {
       area = D.area_k[a][t];
       dist = D.dist_k[a][t];
+      rdist = D.rdist[a][t];
     }
   } else {
     hl = D.lo[f] >= 0;
@@ -2365,8 +2395,8 @@ __device__ __forceinline__ bool face_eval(const ScalarDev& D, int a, long long f
     area = D.area[f];
     dist = D.dist[f];
   }
-  const double cl = hl ? x[lo_cell] : 0.0, cr = hh ? x[hi_cell] : 0.0;
-  const double uf = u[f];
+  const double cl = hl ? in.xl : 0.0, cr = hh ? in.xr : 0.0;
+  const double uf = in.u;
   double donor;
   if (MUSCL) {
     const long long cs = a == 0 ? 1 : (a == 1 ? (long long)D.n[0] : (long long)D.n[0] * D.n[1]);
@@ -2392,16 +2422,18 @@ __device__ __forceinline__ bool face_eval(const ScalarDev& D, int a, long long f
     donor = nonneg(uf) ? plus_zero(cl) : cr;
   }
   double diffusivity;
-  if (hl && hh) diffusivity = half(d[lo_cell] + d[hi_cell]);
-  else if (hl) diffusivity = d[lo_cell];
-  else if (hh) diffusivity = d[hi_cell];
+  if (hl && hh) diffusivity = half(in.dl + in.dr);
+  else if (hl) diffusivity = in.dl;
+  else if (hh) diffusivity = in.dr;
   else diffusivity = 0.0;
-  if (P2) {
+  if (DIV == POW2) {
     const double diff = k == OUTLET ? 0.0 : mul_pow2(diffusivity * (cl - cr), inv_dist_p);
     pv = mul_pow2(mul_pow2(uf * donor + diff, area_p), D.inv_volume);
   } else {
-    const double diff = k == OUTLET ? 0.0 : diffusivity * (cl - cr) / dist;
-    pv = (uf * donor + diff) * area / D.volume;
+    const double grad = diffusivity * (cl - cr);
+    const double diff = k == OUTLET ? 0.0 : DIV == DIVIDE ? grad / dist : div_known<DIV == RECIP2>(grad, dist, rdist);
+    const double flux = (uf * donor + diff) * area;
+    pv = DIV == DIVIDE ? flux / D.volume : div_known<DIV == RECIP2>(flux, D.volume, D.rvolume);
   }
   return true;
 }
@@ -2453,14 +2485,20 @@ __device__ __forceinline__ bool sc_flux(const ScalarDev& D, int a, long long f, 
 // emitted = Σ source × volume, and over the faces on the domain boundary (lo or hi absent)
 // the outward flux's positive part (outflow) and negative part (inflow), in kg/s, with the
 // face flux (u donor + diffusion) area of the same transport faces. Per block, in part[3b ..
-// 3b+2]; k_scalar_budget sums the blocks in order. The sums differ from the reference's
+// 3b+2]; k_scalar_budget sums the blocks. The sums differ from the reference's
 // sequential ones by rounding only (the budgets serve mass accounting, not bits).
 constexpr int SR_BLOCKS = 128, SR_THREADS = 256;
 __global__ void __launch_bounds__(SR_THREADS) k_scalar_rates(ScalarDev D, const double* __restrict__ x,
                                                             const double* __restrict__ u,
                                                             const double* __restrict__ d,
                                                             const double* __restrict__ source, long long N,
-                                                            double* __restrict__ part, int muscl) {
+                                                            double* __restrict__ part, int muscl,
+                                                            const double* __restrict__ x2) {
+  if (blockIdx.y) {  // the second stage's field (its emission is the first's)
+    x = x2;
+    part += 3 * SR_BLOCKS;
+    N = 0;
+  }
   double em = 0.0, inflow = 0.0, outflow = 0.0;
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x, nth = (long long)gridDim.x * blockDim.x;
   for (long long i = tid; i < N; i += nth) em += source[i];
@@ -2498,86 +2536,142 @@ __global__ void __launch_bounds__(SR_THREADS) k_scalar_rates(ScalarDev D, const 
   }
 }
 
-// The block sums of the two stages' rates in block order; the emission is the source sum
-// times the volume. budget += dt (a + b) / 2 per quantity (solver.rs:851-853) when budget is
-// set; rates (when set) receive the first stage's rates.
-__global__ void k_scalar_budget(const double* __restrict__ pa, const double* __restrict__ pb, double volume, double dt,
-                                double* __restrict__ budget, double* __restrict__ rates) {
-  if (threadIdx.x >= 3) return;
-  const int k = threadIdx.x;
+// The sums of the blocks' rates of the two stages, a warp per quantity (in block order by one
+// thread: 10 us); the emission, the same in both, is the source sum times the volume. budget +=
+// dt (a + b) / 2 per quantity (solver.rs:851-853) when budget is set; rates (when set) receive
+// the first stage's rates.
+__global__ void __launch_bounds__(96) k_scalar_budget(const double* __restrict__ pa, const double* __restrict__ pb,
+                                                      double volume, double dt, double* __restrict__ budget,
+                                                      double* __restrict__ rates) {
+  const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double a = 0.0, b = 0.0;
-  for (int blk = 0; blk < SR_BLOCKS; ++blk) {
-    a += pa[3 * blk + k];
-    if (pb) b += pb[3 * blk + k];
+#pragma unroll
+  for (int m = 0; m < SR_BLOCKS / 32; ++m) {
+    a += pa[3 * (lane + 32 * m) + k];
+    if (pb && k) b += pb[3 * (lane + 32 * m) + k];
   }
+  for (int o = 16; o > 0; o >>= 1) {
+    a += __shfl_down_sync(0xffffffffu, a, o);
+    b += __shfl_down_sync(0xffffffffu, b, o);
+  }
+  if (lane) return;
   if (k == 0) {
     a *= volume;
-    b *= volume;
+    b = a;
   }
   if (rates) rates[k] = a;
   if (budget) budget[k] += 0.5 * dt * (a + b);
 }
 
-// One pass of the SSPRK2 step over a tile of (32, 8, zs) cells. MODE 0 (solver.rs:845-847):
-// stage = c + dt rhs(c). MODE 1 (solver.rs:848-850): c = (c + stage + dt rhs(stage)) / 2, in
-// place (a thread reads c only at its own cell). Blocks are (32, 8); every thread reaches
-// every barrier and shuffle.
-template <bool UNI, bool P2, bool MUSCL, int MODE>
-__global__ void __launch_bounds__(STX * STY) k_scalar_pass(ScalarDev D, double* __restrict__ c,
-                                                          double* __restrict__ stage, const double* __restrict__ u,
-                                                          const double* __restrict__ d,
-                                                          const double* __restrict__ source, double dt, int zs) {
-  __shared__ double s_pv[STY][STX];
-  __shared__ uint8_t s_on[STY][STX];
+// One pass of the SSPRK2 step. MODE 0 (solver.rs:845-847): stage = c + dt rhs(c). MODE 1
+// (solver.rs:848-850): c = (c + stage + dt rhs(stage)) / 2, in place (a thread reads c only at
+// its own cell).
+//
+// The FP64 pipe bounds it (64 cycles a warp's operation, however many lanes are active), so no
+// operation is spent on a few lanes: the face at the end of a tile's rows is evaluated for its
+// eight rows and four slices at once by one warp (in turn), not by one lane of every warp. The
+// slices of all (32, 8) columns form one sequence of `units`, of which every block takes an
+// equal share (nz per column; a share that begins in a column evaluates that z face itself).
+// The row of tiles that also evaluates the tile's last y faces moves over the SM's sub-cores
+// from block to block (`sms` blocks apart on one SM). Every thread reaches every barrier and
+// shuffle; the exchanged faces are double-buffered, with one barrier a slice, and a slice's loads
+// go out before its arithmetic. A step of 128x128x64 (upwind, powers of two) 181 -> 136 us, 76 %
+// of the pipe's cycles while the blocks run; 90x70x45 (MUSCL, spacing 1.5, with the budget) 240 ->
+// 146 us, of which the divisions by constants through their reciprocals are the most. Four blocks
+// per SM (three for MUSCL), which spilled registers, took 143 and 156 us.
+template <bool UNI, int DIV, bool MUSCL, int MODE>
+__global__ void __launch_bounds__(STX * STY, MUSCL ? 2 : 3)
+    k_scalar_pass(ScalarDev D, double* __restrict__ c, double* __restrict__ stage, const double* __restrict__ u,
+                  const double* __restrict__ d, const double* __restrict__ source, double dt, int columns, int sms) {
+  __shared__ double s_y[2][STY][STX], s_x[2][4][STY];
+  __shared__ uint8_t s_yon[2][STY][STX], s_xon[2][4][STY];
   const double* __restrict__ x = MODE == 0 ? c : stage;  // the field the right-hand side reads
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const int nx = D.n[0], ny = D.n[1], nz = D.n[2];
-  const int i = blockIdx.x * STX + tx, j = blockIdx.y * STY + ty;
-  const int z0 = blockIdx.z * zs, z1 = min(z0 + zs, nz);
-  const bool valid = i < nx && j < ny;
+  const int tx = threadIdx.x, warp = threadIdx.y, ty = (warp + blockIdx.x / sms) & (STY - 1);
+  const int nx = D.n[0], ny = D.n[1], nz = D.n[2], tiles_x = (nx + STX - 1) / STX;
   const long long sx = nx, sxy = (long long)nx * ny;
+  const long long units = (long long)columns * nz;
+  const long long u0 = units * blockIdx.x / gridDim.x, u1 = units * (blockIdx.x + 1) / gridDim.x;
+  int col = (int)(u0 / nz), z = (int)(u0 - (long long)col * nz);
+  bool fresh = true;  // a column begins (or the share does): its z face is not at hand
+  int yb = 0, xb = 0, bs = 0;
   double zlo = 0.0;
   bool zlo_on = false;
-  if (valid) {  // the z-lo face of the first slice
-    const long long cell = z0 * sxy + j * sx + i;
-    const long long f = D.face_off[2] + ((long long)z0 * D.fdim[2][1] + j) * D.fdim[2][0] + i;
-    zlo_on = face_eval<UNI, P2, MUSCL>(D, 2, f, z0 > 0 ? cell - sxy : -1, cell, x, u, d, zlo);
-  }
-  for (int z = z0; z < z1; ++z) {
-    const long long cell = z * sxy + j * sx + i;
-    double xlo = 0.0, xhi = 0.0, ylo = 0.0, yhi = 0.0, zhi = 0.0;
-    bool xlo_on = false, xhi_on = false, ylo_on = false, yhi_on = false, zhi_on = false;
-    if (valid) {
-      const long long fx = D.face_off[0] + ((long long)z * D.fdim[0][1] + j) * D.fdim[0][0] + i;
-      xlo_on = face_eval<UNI, P2, MUSCL>(D, 0, fx, i > 0 ? cell - 1 : -1, cell, x, u, d, xlo);
-      const long long fy = D.face_off[1] + ((long long)z * D.fdim[1][1] + j) * D.fdim[1][0] + i;
-      ylo_on = face_eval<UNI, P2, MUSCL>(D, 1, fy, j > 0 ? cell - sx : -1, cell, x, u, d, ylo);
-      const long long fz = D.face_off[2] + ((long long)(z + 1) * D.fdim[2][1] + j) * D.fdim[2][0] + i;
-      zhi_on = face_eval<UNI, P2, MUSCL>(D, 2, fz, cell, z + 1 < nz ? cell + sxy : -1, x, u, d, zhi);
+  for (long long unit = u0; unit < u1; ++unit, ++z) {
+    if (z == nz) {
+      z = 0;
+      ++col;
+      fresh = true;
     }
-    // x-hi: the next lane's x-lo, or computed here at the tile's or the domain's edge.
-    const double nxt = __shfl_down_sync(0xffffffffu, xlo, 1);
-    const int nxt_on = __shfl_down_sync(0xffffffffu, (int)xlo_on, 1);
-    s_pv[ty][tx] = ylo;
-    s_on[ty][tx] = ylo_on;
+    const int i0 = col % tiles_x * STX, j0 = col / tiles_x * STY;
+    const int i = i0 + tx, j = j0 + ty;
+    const bool valid = i < nx && j < ny;
+    const long long cell = z * sxy + j * sx + i;
+    if (fresh) {
+      fresh = false;
+      bs = 0;
+      zlo_on = false;
+      if (valid) {
+        const long long f = D.face_off[2] + ((long long)z * D.fdim[2][1] + j) * D.fdim[2][0] + i;
+        const long long below = z > 0 ? cell - sxy : -1;
+        zlo_on = face_eval<UNI, DIV, MUSCL>(D, 2, f, below, cell, x, face_load(D, f, below, cell, x, u, d), zlo);
+      }
+    }
+    if (bs == 0) {  // the end faces of this slice and the next three
+      xb ^= 1;
+      if (warp == (yb >> 2 & (STY - 1))) {
+        const int r = tx & (STY - 1), m = tx / STY, ie = min(i0 + STX, nx), zz = z + m, jj = j0 + r;
+        double v = 0.0;
+        bool on = false;
+        if (jj < ny && zz < nz && unit + m < u1) {
+          const long long end = zz * sxy + jj * sx + ie;  // the cell behind the face
+          const long long f = D.face_off[0] + ((long long)zz * D.fdim[0][1] + jj) * D.fdim[0][0] + ie;
+          const long long behind = ie < nx ? end : -1;
+          on = face_eval<UNI, DIV, MUSCL>(D, 0, f, end - 1, behind, x, face_load(D, f, end - 1, behind, x, u, d), v);
+        }
+        s_x[xb][m][r] = v;
+        s_xon[xb][m][r] = on;
+      }
+    }
+    double xlo = 0.0, ylo = 0.0, zhi = 0.0, acc = 0.0, c0 = 0.0, c1 = 0.0;
+    uint8_t fluid = 0;
+    bool xlo_on = false, ylo_on = false, zhi_on = false;
+    if (valid) {
+      // All loads of the slice before its arithmetic.
+      const long long fx = D.face_off[0] + ((long long)z * D.fdim[0][1] + j) * D.fdim[0][0] + i;
+      const long long fy = D.face_off[1] + ((long long)z * D.fdim[1][1] + j) * D.fdim[1][0] + i;
+      const long long fz = D.face_off[2] + ((long long)(z + 1) * D.fdim[2][1] + j) * D.fdim[2][0] + i;
+      const long long cx = i > 0 ? cell - 1 : -1, cy = j > 0 ? cell - sx : -1, cz = z + 1 < nz ? cell + sxy : -1;
+      const FaceIn ax = face_load(D, fx, cx, cell, x, u, d), ay = face_load(D, fy, cy, cell, x, u, d),
+                   az = face_load(D, fz, cell, cz, x, u, d);
+      acc = source[cell];
+      fluid = D.fluid[cell];
+      c0 = c[cell];
+      if (MODE == 1) c1 = stage[cell];
+      xlo_on = face_eval<UNI, DIV, MUSCL>(D, 0, fx, cx, cell, x, ax, xlo);
+      ylo_on = face_eval<UNI, DIV, MUSCL>(D, 1, fy, cy, cell, x, ay, ylo);
+      zhi_on = face_eval<UNI, DIV, MUSCL>(D, 2, fz, cell, cz, x, az, zhi);
+    }
+    double xhi = __shfl_down_sync(0xffffffffu, xlo, 1);
+    bool xhi_on = __shfl_down_sync(0xffffffffu, (int)xlo_on, 1) != 0;
+    s_y[yb & 1][ty][tx] = ylo;
+    s_yon[yb & 1][ty][tx] = ylo_on;
     __syncthreads();
     if (valid) {
       if (tx == STX - 1 || i == nx - 1) {
-        const long long fx = D.face_off[0] + ((long long)z * D.fdim[0][1] + j) * D.fdim[0][0] + i + 1;
-        xhi_on = face_eval<UNI, P2, MUSCL>(D, 0, fx, cell, i + 1 < nx ? cell + 1 : -1, x, u, d, xhi);
-      } else {
-        xhi = nxt;
-        xhi_on = nxt_on != 0;
+        xhi = s_x[xb][bs][ty];
+        xhi_on = s_xon[xb][bs][ty] != 0;
       }
+      double yhi = 0.0;
+      bool yhi_on;
       if (ty == STY - 1 || j == ny - 1) {
         const long long fy = D.face_off[1] + ((long long)z * D.fdim[1][1] + j + 1) * D.fdim[1][0] + i;
-        yhi_on = face_eval<UNI, P2, MUSCL>(D, 1, fy, cell, j + 1 < ny ? cell + sx : -1, x, u, d, yhi);
+        const long long beyond = j + 1 < ny ? cell + sx : -1;
+        yhi_on = face_eval<UNI, DIV, MUSCL>(D, 1, fy, cell, beyond, x, face_load(D, fy, cell, beyond, x, u, d), yhi);
       } else {
-        yhi = s_pv[ty + 1][tx];
-        yhi_on = s_on[ty + 1][tx] != 0;
+        yhi = s_y[yb & 1][ty + 1][tx];
+        yhi_on = s_yon[yb & 1][ty + 1][tx] != 0;
       }
-      double acc = source[cell];
-      if (D.fluid[cell]) {  // a solid cell is on no face: its rate is its source
+      if (fluid) {  // a solid cell is on no face: its rate is its source
         if (xlo_on) acc = acc + xlo;
         if (xhi_on) acc = acc - xhi;
         if (ylo_on) acc = acc + ylo;
@@ -2585,37 +2679,14 @@ __global__ void __launch_bounds__(STX * STY) k_scalar_pass(ScalarDev D, double* 
         if (zlo_on) acc = acc + zlo;
         if (zhi_on) acc = acc - zhi;
       }
-      if (MODE == 0) stage[cell] = c[cell] + dt * acc;
-      else c[cell] = half(c[cell] + stage[cell] + dt * acc);
+      if (MODE == 0) stage[cell] = c0 + dt * acc;
+      else c[cell] = half(c0 + c1 + dt * acc);
     }
     zlo = zhi;
     zlo_on = zhi_on;
-    __syncthreads();  // s_pv is rewritten by the next slice
+    bs = (bs + 1) & 3;
+    yb += 1;
   }
-}
-
-// Slices per block of the scalar passes: the z extent split so that the blocks' slices
-// spread evenly over the SMs (the passes are FP64-pipe bound, so an SM's time follows the
-// slices it is given: about ceil(blocks / SMs) zs), counting the z face each block
-// evaluates once more than its slices need (a third of a slice's faces), among the splits
-// that give every SM its four resident blocks (the smallest split where none does).
-int scalar_zsplit(const int32_t n[3], int device) {
-  int sms = 0;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  sms = std::max(sms, 1);
-  const long long cols = (long long)((n[0] + STX - 1) / STX) * ((n[1] + STY - 1) / STY);
-  int best = 2;
-  double best_cost = 1e300;
-  for (int zs = 2; zs <= 16; ++zs) {
-    const long long blocks = cols * ((n[2] + zs - 1) / zs);
-    if (zs > 2 && blocks < 4LL * sms) continue;
-    const double cost = (double)((blocks + sms - 1) / sms) * std::min(zs, n[2]) * (1.0 + 1.0 / (3.0 * zs));
-    if (cost < best_cost - 1e-9) {
-      best_cost = cost;
-      best = zs;
-    }
-  }
-  return best;
 }
 
 FlowDev flow_dev(cfdg_grid* G) {
@@ -3021,6 +3092,7 @@ static int scalar_impl(cfdg_grid* G, const double* d_u, double* d_c, const doubl
   }
   D.volume = G->h.volume;
   D.inv_volume = pow2_of(G->h.volume, true);
+  D.rvolume = host_recip(G->h.volume);
   D.kind = G->d_kind;
   D.fluid = G->d_fluid;
   D.lo = G->d_lo;
@@ -3033,6 +3105,7 @@ static int scalar_impl(cfdg_grid* G, const double* d_u, double* d_c, const doubl
       D.dist_k[a][t] = G->sc_dist[a][t];
       D.area_p[a][t] = pow2_of(G->sc_area[a][t], false);
       D.inv_dist_p[a][t] = pow2_of(G->sc_dist[a][t], true);
+      D.rdist[a][t] = host_recip(G->sc_dist[a][t]);
     }
   double* stage = G->st_sc;
   cudaStream_t s = G->stream;
@@ -3040,47 +3113,56 @@ static int scalar_impl(cfdg_grid* G, const double* d_u, double* d_c, const doubl
     if (int e = G->arena.alloc(&G->sc_part, (size_t)2 * 3 * SR_BLOCKS + 3)) return e;
   }
   if (mode == 2) {
-    k_scalar_rates<<<SR_BLOCKS, SR_THREADS, 0, s>>>(D, d_c, d_u, d_diff, d_source, N, G->sc_part, G->sc_muscl);
+    k_scalar_rates<<<SR_BLOCKS, SR_THREADS, 0, s>>>(D, d_c, d_u, d_diff, d_source, N, G->sc_part, G->sc_muscl,
+                                                    nullptr);
     double* dr = G->sc_part + 6 * SR_BLOCKS;
-    k_scalar_budget<<<1, 32, 0, s>>>(G->sc_part, nullptr, D.volume, 0.0, nullptr, dr);
+    k_scalar_budget<<<1, 96, 0, s>>>(G->sc_part, nullptr, D.volume, 0.0, nullptr, dr);
     count(2);
     CU(cudaMemcpyAsync(rates, dr, 3 * sizeof(double), cudaMemcpyDeviceToHost, s));
     CU(cudaStreamSynchronize(s));
     return 0;
   }
-  const int zs = scalar_zsplit(G->h.n, G->ctx->device);
-  const dim3 blk(STX, STY), grd((G->h.n[0] + STX - 1) / STX, (G->h.n[1] + STY - 1) / STY, (G->h.n[2] + zs - 1) / zs);
+  int sms = 0;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, G->ctx->device);
+  sms = std::max(sms, 1);
+  const int columns = ((G->h.n[0] + STX - 1) / STX) * ((G->h.n[1] + STY - 1) / STY);
+  const dim3 blk(STX, STY);
   // The budget's rates: of c before the second pass overwrites it, and of the stage.
   auto rates_of_stages = [&]() {
     if (mode != 1) return;
-    k_scalar_rates<<<SR_BLOCKS, SR_THREADS, 0, s>>>(D, d_c, d_u, d_diff, d_source, N, G->sc_part, G->sc_muscl);
-    k_scalar_rates<<<SR_BLOCKS, SR_THREADS, 0, s>>>(D, stage, d_u, d_diff, d_source, N, G->sc_part + 3 * SR_BLOCKS,
-                                                    G->sc_muscl);
-    count(2);
+    k_scalar_rates<<<dim3(SR_BLOCKS, 2), SR_THREADS, 0, s>>>(D, d_c, d_u, d_diff, d_source, N, G->sc_part, G->sc_muscl,
+                                                             stage);
+    count();
   };
-  bool p2 = G->sc_uniform && D.inv_volume.ok;
+  // How the passes divide (face_eval DIV).
+  bool p2 = G->sc_uniform && D.inv_volume.ok, known = G->sc_uniform && D.rvolume != 0.0, again = D.rvolume < 0.0;
   for (int a = 0; a < 3; ++a)
     for (int t = 0; t < 3; ++t)
-      if (G->sc_used[a][t]) p2 = p2 && D.area_p[a][t].ok && D.inv_dist_p[a][t].ok;
-  auto passes = [&](auto uni, auto p2c, auto muscl) {
-    constexpr bool U = decltype(uni)::value, P = decltype(p2c)::value, M = decltype(muscl)::value;
-    k_scalar_pass<U, P, M, 0><<<grd, blk, 0, s>>>(D, d_c, stage, d_u, d_diff, d_source, dt, zs); tick(G);
+      if (G->sc_used[a][t]) {
+        p2 = p2 && D.area_p[a][t].ok && D.inv_dist_p[a][t].ok;
+        known = known && D.rdist[a][t] != 0.0;
+        again = again || D.rdist[a][t] < 0.0;
+      }
+  auto passes = [&](auto uni, auto div, auto muscl) {
+    constexpr bool U = decltype(uni)::value, M = decltype(muscl)::value;
+    constexpr int V = decltype(div)::value;
+    // As many blocks as fit the device at once, or one per slice of a column.
+    const int grd = (int)std::min<long long>((long long)columns * G->h.n[2], (M ? 2LL : 3LL) * sms);
+    k_scalar_pass<U, V, M, 0><<<grd, blk, 0, s>>>(D, d_c, stage, d_u, d_diff, d_source, dt, columns, sms); tick(G);
     rates_of_stages();
-    k_scalar_pass<U, P, M, 1><<<grd, blk, 0, s>>>(D, d_c, stage, d_u, d_diff, d_source, dt, zs); tick(G);
+    k_scalar_pass<U, V, M, 1><<<grd, blk, 0, s>>>(D, d_c, stage, d_u, d_diff, d_source, dt, columns, sms); tick(G);
   };
-  using T = std::true_type;
-  using F = std::false_type;
-  if (G->sc_muscl) {
-    if (p2) passes(T{}, T{}, T{});
-    else if (G->sc_uniform) passes(T{}, F{}, T{});
-    else passes(F{}, F{}, T{});
-  } else {
-    if (p2) passes(T{}, T{}, F{});
-    else if (G->sc_uniform) passes(T{}, F{}, F{});
-    else passes(F{}, F{}, F{});
-  }
+  auto with = [&](auto muscl) {
+    if (p2) passes(std::true_type{}, std::integral_constant<int, POW2>{}, muscl);
+    else if (known && !again) passes(std::true_type{}, std::integral_constant<int, RECIP>{}, muscl);
+    else if (known) passes(std::true_type{}, std::integral_constant<int, RECIP2>{}, muscl);
+    else if (G->sc_uniform) passes(std::true_type{}, std::integral_constant<int, DIVIDE>{}, muscl);
+    else passes(std::false_type{}, std::integral_constant<int, DIVIDE>{}, muscl);
+  };
+  if (G->sc_muscl) with(std::true_type{});
+  else with(std::false_type{});
   if (mode == 1) {
-    k_scalar_budget<<<1, 32, 0, s>>>(G->sc_part, G->sc_part + 3 * SR_BLOCKS, D.volume, dt, d_budget, nullptr);
+    k_scalar_budget<<<1, 96, 0, s>>>(G->sc_part, G->sc_part + 3 * SR_BLOCKS, D.volume, dt, d_budget, nullptr);
     count();
   }
   CU(cudaGetLastError());

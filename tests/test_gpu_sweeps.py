@@ -135,3 +135,34 @@ def test_center_bitwise(pkg, cells):
     dg.center_nullspaces(x)
     assert np.array_equal(bits(x), bits(want))
     dg.close()
+
+
+@pytest.mark.parametrize("muscl", [False, True])
+@pytest.mark.parametrize("cells, dx", [((31, 8, 5), 2.0), ((33, 9, 4), 1.5), ((64, 7, 3), 1.9), ((95, 17, 2), 2.3),
+                                       ((2, 40, 37), 0.3), ((160, 130, 23), 1.3)])
+def test_scalar_pass_bitwise_at_tile_edges(pkg, O, cells, dx, muscl):
+    """The scalar passes at the edges of their 32 x 8 tiles, shares of a column's slices and
+    end faces of less than four slices, with spacings whose quotients go through the exponent
+    field, a reciprocal and a reciprocal with the extra correction: the oracle's bits."""
+    torch = pytest.importorskip("torch")
+    case = pkg.synth.case(cells, dx, inflow=2.0, preconditioner="multigrid",
+                          boxes=[] if min(cells) < 5 else [((4 * dx, 2 * dx, 0.0), (9 * dx, 5 * dx, 3 * dx))])
+    g = pkg.grid.Grid.build(case)
+    og = O.Grid(case)
+    rng = np.random.default_rng(sum(cells))
+    open_ = np.isin(g.face_kind, (pkg.grid.INTERIOR, pkg.grid.INLET, pkg.grid.OUTLET))
+    u = np.where(open_, rng.uniform(-2.0, 2.0, g.n_faces), 0.0)
+    fluid = g.fluid.astype(bool)
+    c = np.where(fluid & (rng.uniform(size=g.count) < 0.7), rng.uniform(0.0, 1e-3, g.count), 0.0)
+    d = np.where(fluid, rng.uniform(0.01, 0.5, g.count), 0.0)
+    source = np.where(rng.uniform(size=g.count) < 0.01, 1e-3, 0.0)
+    dg = pkg.pressure.DeviceGrid(g, preconditioner="multigrid")
+    dg.set_advection("muscl" if muscl else "linear_upwind")
+    d_u, d_c, d_d, d_s = (torch.from_numpy(v.copy()).cuda() for v in (u, c, d, source))
+    ref = c
+    for _ in range(2):
+        ref = og.scalar_step(ref, u, d, source, 0.01, muscl=muscl)
+        dg.scalar_step_device(d_u.data_ptr(), d_c.data_ptr(), d_d.data_ptr(), d_s.data_ptr(), 0.01)
+        torch.cuda.synchronize()
+        assert np.array_equal(bits(d_c.cpu().numpy()), bits(ref))
+    dg.close()
