@@ -169,6 +169,7 @@ __global__ void k_apply(GridDev g, const double* __restrict__ x, double* __restr
 template <bool UNIFORM>
 __global__ void k_pcg_op(GridDev g, const double* __restrict__ p, double* __restrict__ ap, int N, double* partials,
                          Scalars* S) {
+  pdl_enter();
   __shared__ double sh[32];
   if (S->done) return;
   if (S->it >= S->max_it) {
@@ -184,6 +185,7 @@ __global__ void k_pcg_op(GridDev g, const double* __restrict__ p, double* __rest
     ap[c] = v;
     acc += p[c] * v;
   }
+  pdl_leave();
   double bs = block_sum(acc, sh);
   if (arrive(bs, partials, &S->counter)) {
     double denom = gather_partials(partials, sh, &S->counter);
@@ -201,6 +203,7 @@ __global__ void k_pcg_op(GridDev g, const double* __restrict__ p, double* __rest
 // x += alpha p, r -= alpha Ap, rel = |r|/|b_c| (pressure.rs:398-403).
 __global__ void k_pcg_xr(double* __restrict__ x, double* __restrict__ r, const double* __restrict__ p,
                          const double* __restrict__ ap, int N, double* partials, Scalars* S) {
+  pdl_enter();
   __shared__ double sh[32];
   if (S->done) return;
   const double alpha = S->alpha;
@@ -211,6 +214,7 @@ __global__ void k_pcg_xr(double* __restrict__ x, double* __restrict__ r, const d
     r[i] = v;
     acc += v * v;
   }
+  pdl_leave();
   double bs = block_sum(acc, sh);
   if (arrive(bs, partials, &S->counter)) {
     double rr = gather_partials(partials, sh, &S->counter);
@@ -225,6 +229,7 @@ __global__ void k_pcg_xr(double* __restrict__ x, double* __restrict__ r, const d
 template <bool UNIFORM>
 __global__ void k_pcg_true(GridDev g, const double* __restrict__ x, const double* __restrict__ bc, int N,
                            double* partials, Scalars* S) {
+  pdl_enter();
   __shared__ double sh[32];
   if (S->done || !S->check) return;
   double acc = 0.0;
@@ -236,6 +241,7 @@ __global__ void k_pcg_true(GridDev g, const double* __restrict__ x, const double
     double d = v - bc[c];
     acc += d * d;
   }
+  pdl_leave();
   double bs = block_sum(acc, sh);
   if (arrive(bs, partials, &S->counter)) {
     double s = gather_partials(partials, sh, &S->counter);
@@ -302,10 +308,12 @@ __global__ void k_residual_norm_noalloc(GridDev g, const double* __restrict__ x,
 // rz' = r.z, beta = rz'/rz, it += 1 (pressure.rs:428-433). init: the first rz.
 __global__ void k_pcg_rz(const double* __restrict__ r, const double* __restrict__ z, int N, double* partials,
                          Scalars* S, int init) {
+  pdl_enter();
   __shared__ double sh[32];
   if (S->done) return;
   double acc = 0.0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) acc += r[i] * z[i];
+  pdl_leave();
   double bs = block_sum(acc, sh);
   if (arrive(bs, partials, &S->counter)) {
     double next = gather_partials(partials, sh, &S->counter);
@@ -322,6 +330,7 @@ __global__ void k_pcg_rz(const double* __restrict__ r, const double* __restrict_
 }
 
 __global__ void k_pcg_p(double* __restrict__ p, const double* __restrict__ z, int N, const Scalars* S) {
+  pdl_enter();
   if (S->done) return;
   const double beta = S->beta;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) p[i] = z[i] + beta * p[i];
@@ -920,7 +929,7 @@ void launch_wave_spread(cfdg_grid* G, const WaveArgs& A) {
   // Just more than the share that per + 1 tiles would have: room for `per`, not for one more.
   const int want = L.smem_sm / (per + 1) - L.reserved - L.fixed + 1024;
   const int dyn = std::max(0, std::min(want, std::min(L.most, L.smem_sm / per - L.reserved - L.fixed)));
-  k_wave<MODE, UNIFORM, EXTRA><<<tiles, WTHREADS, dyn, G->stream>>>(A);
+  launch_pdl(k_wave<MODE, UNIFORM, EXTRA>, tiles, WTHREADS, dyn, G->stream, A);
   tick(G);
 }
 
@@ -1137,12 +1146,12 @@ void launch_iteration_t(cfdg_grid* G) {
   const int N = (int)G->h.cells;
   const int nb = grid_blocks(N);
   cudaStream_t s = G->stream;
-  k_pcg_op<U><<<nb, BLOCK, 0, s>>>(G->g, G->p, G->ap, N, G->partials, G->S); tick(G);
-  k_pcg_xr<<<nb, BLOCK, 0, s>>>(G->x, G->r, G->p, G->ap, N, G->partials, G->S); tick(G);
-  k_pcg_true<U><<<nb, BLOCK, 0, s>>>(G->g, G->x, G->bc, N, G->partials, G->S); tick(G);
+  launch_pdl(k_pcg_op<U>, nb, BLOCK, 0, s, G->g, G->p, G->ap, N, G->partials, G->S); tick(G);
+  launch_pdl(k_pcg_xr, nb, BLOCK, 0, s, G->x, G->r, G->p, G->ap, N, G->partials, G->S); tick(G);
+  launch_pdl(k_pcg_true<U>, nb, BLOCK, 0, s, G->g, G->x, G->bc, N, G->partials, G->S); tick(G);
   launch_precondition(G, G->S);
-  k_pcg_rz<<<nb, BLOCK, 0, s>>>(G->r, G->z, N, G->partials, G->S, 0); tick(G);
-  k_pcg_p<<<nb, BLOCK, 0, s>>>(G->p, G->z, N, G->S); tick(G);
+  launch_pdl(k_pcg_rz, nb, BLOCK, 0, s, G->r, G->z, N, G->partials, G->S, 0); tick(G);
+  launch_pdl(k_pcg_p, nb, BLOCK, 0, s, G->p, G->z, N, G->S); tick(G);
 }
 void launch_iteration(cfdg_grid* G) {
   if (G->uniform) launch_iteration_t<true>(G);

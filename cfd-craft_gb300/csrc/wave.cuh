@@ -159,6 +159,7 @@ __global__ void __launch_bounds__(WTHREADS) k_wave(WaveArgs A) {
   __shared__ volatile int passed;       // steps whose barrier the compute warps have passed
   __shared__ volatile int bail;
   __shared__ unsigned long long ticket;
+  pdl_enter();
   if (A.S && A.S->done) return;
   const int nx = A.n[0], ny = A.n[1], nz = A.n[2];
   if (threadIdx.x == 0) {
