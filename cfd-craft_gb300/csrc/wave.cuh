@@ -107,8 +107,10 @@ __device__ __noinline__ double div_rare(double v, double d) { return __ddiv_rn(v
 // |r d - 1| <= 2^-54: with significands v, d in [1, 2) its error is at most v |r - 1/d|
 // plus half an ulp of q, v |r - 1/d| <= 2^-54 v/d, and v/d < 1 halves the ulp, so both
 // cases stay within one ulp. Otherwise (rd < 0) one more correction first makes it so.
-// Zeros, subnormals, NaN, infinities and v outside [2^-900, 2^900] (where a product or
-// remainder could leave the normal range) take the division. The tests are on the bits: a
+// A zero is its own quotient (solid cells, and cells that nothing has reached yet: with a
+// division for them an IC(0) iteration of 24x20x16 took 157 us instead of 115). Subnormals,
+// NaN, infinities and other v outside [2^-900, 2^900] (where a product or remainder could
+// leave the normal range) take the division. The tests are on the bits: a
 // comparison of doubles would queue for the FP64 pipe. on: whether the result is used;
 // EXTRA: whether some rd is negative (a warp's FP64 operations take 64 cycles each, also
 // where no lane needs them).
@@ -124,7 +126,11 @@ __device__ __forceinline__ double div_pre(double v, double d, double rd, bool on
     q = __fma_rn(rem, r, q);
   }
   const unsigned e = ((unsigned)__double2hiint(v) >> 20) & 0x7ffu;
-  if (on && (e - 123u > 1800u || hi == 0)) q = div_rare(v, d);
+  if (on && (e - 123u > 1800u || hi == 0)) {
+    const unsigned mag = (unsigned)__double2hiint(v) << 1 | (unsigned)__double2loint(v);
+    if (mag == 0 && hi != 0) q = v;
+    else q = div_rare(v, d);
+  }
   return q;
 }
 
