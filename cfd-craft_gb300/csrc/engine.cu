@@ -8,8 +8,10 @@
 //   fw     f64[F]   face weights area/(distance*volume), recomputed when faces change
 //   face_kind u8[F], face_lo/face_hi i32[F], face_dist f64[F]   (velocity correction)
 //   x r z p ap bc b terms  f64[N]   PCG and projection vectors
-//   IC(0): lower CSR (i32 off/col, f64 val), its transpose, diag, level orders
-//   multigrid: per level CSR + diag, level orders, transfer CSRs, vectors
+//   IC(0): lower coefficients per cell, diag and its reciprocals (structured grids); else
+//     lower CSR (i32 off/col, f64 val), its transpose, diag, level orders
+//   multigrid: per level the cluster plan's or the lines' records, or CSR + diag and level
+//     orders; transfer CSRs, vectors
 // The PCG loop runs as CUDA graphs of 8 iterations; every kernel first reads the
 // device Scalars and returns at once when the solve has finished, so the host only
 // synchronises between chunks, where it polls the caller's Control.
@@ -615,7 +617,8 @@ __global__ void k_prolong(int n, const int* __restrict__ off, const int* __restr
 }
 
 // ----------------------------------------------------------------- coarse levels, one launch
-// Levels 1 .. L-1 of the V-cycle in one cooperative kernel: each dependency level of a
+// Levels 1 .. L-1 of the V-cycle in one cooperative kernel, where no cluster plan
+// (plain_cluster.cuh) covers them: each dependency level of a
 // lexicographic sweep, the residual, the restriction, the prolongation and the gauges is
 // a phase separated by a grid barrier (level-by-level launches cost a launch each: about
 // 1,300 per cycle on a 128x128x64 grid). Levels whose dependency levels have at most one
@@ -1039,7 +1042,8 @@ void launch_vcycle(cfdg_grid* G, const double* r, double* z, const Scalars* S) {
     tick(G);
   }
   const int nl = (int)H.levels.size();
-  // Levels 1 .. L-1 in one cooperative launch when available, else level by level.
+  // Levels 1 .. L-1 on the cluster plan, or in one cooperative launch when available, else level
+  // by level.
   const bool coop = !H.lines && (H.coop_blocks > 0 || H.cluster || H.pc_rest > 0) && nl > 1;
   // The first level of the cooperative launch, or of the cluster plan's whole cycle.
   const int first = H.pc_rest > 0 ? H.pc_rest : 1;

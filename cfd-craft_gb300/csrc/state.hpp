@@ -183,7 +183,7 @@ struct DevHierarchy {
   int* fluid_idx = nullptr;
   std::vector<DevLevel> levels;
   std::vector<uint64_t> level_cells, level_nonzeros;
-  // Levels 1 .. L-1 as one cooperative kernel's descriptors (engine.cu PLev), and its grid
+  // Without a cluster plan: levels 1 .. L-1 as one cooperative kernel's descriptors (engine.cu PLev), and its grid
   // (0: not co-resident, the level-by-level launches are used instead).
   void* d_plev = nullptr;
   int coop_blocks = 0;

@@ -304,7 +304,7 @@ int cfdg_batch_project(cfdg_batch *batch, double *const *u, double *const *p, co
                        uint64_t max_iter, cfdg_poll_fn poll, void *poll_ctx, cfdg_info *infos, int32_t *codes);
 /* Times one unit of the batch's work `reps` times with CUDA events on the batch's
  * stream, every case in its inner-iteration state: which = 0 one red-black half sweep
- * over all fine levels, 1 the FP32 operator, 2 all coarse levels (one cooperative launch), 3 one
+ * over all fine levels, 1 the FP32 operator, 2 all coarse levels, 3 one
  * V-cycle, 4 the half sweep of 0 with the unstaged register kernel, 5 the FP64 true
  * residual of every case, 6 the FP64 right-hand side of every case (only after a
  * host-buffer cfdg_batch_project, whose inputs the batch keeps), 7 the level-0 residual
