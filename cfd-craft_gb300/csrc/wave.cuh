@@ -34,17 +34,12 @@
 // sweeps run the same machinery mirrored (i, j, k descending).
 #pragma once
 #include "plain_kernels.cuh"
+#include "wave_place.hpp"
 
 namespace cfdg {
 
-constexpr int WTJ = 8, WTK = 8;       // tile of pencils per CTA
-constexpr int WCT = WTJ * WTK;        // compute threads (two warps)
-constexpr int WTHREADS = WCT + 32;    // and the receiver warp
-constexpr int WRING = 256;            // received values per boundary pencil held in shared memory
+constexpr int WTHREADS = WCT + 32;    // the compute threads and the receiver warp
 constexpr int WPF = 4;                // steps of operands in flight per compute thread
-constexpr int WHALO = WTJ + WTK;      // boundary pencils of a tile that its consumers read
-
-enum WaveMode { IC0_FWD = 0, IC0_BWD = 1, GS_FWD = 2, GS_BWD = 3 };
 
 struct WaveArgs {
   int n[3];
@@ -158,8 +153,7 @@ template <int MODE, bool UNIFORM, bool EXTRA>
 __global__ void __launch_bounds__(WTHREADS) k_wave(WaveArgs A) {
   constexpr bool BWD = (MODE == IC0_BWD || MODE == GS_BWD);
   constexpr bool GS = MODE >= GS_FWD;
-  // The last two steps' values, [step & 1][thread], then the received values, [pencil][WRING].
-  __shared__ double sh[2 * WCT + WHALO * WRING];
+  __shared__ double sh[WSHARED];
   double* const ring = sh + 2 * WCT;
   __shared__ volatile int seen[WHALO];  // values received per boundary pencil
   __shared__ volatile int passed;       // steps whose barrier the compute warps have passed
@@ -233,39 +227,23 @@ __global__ void __launch_bounds__(WTHREADS) k_wave(WaveArgs A) {
     }
     return;
   }
-  const int tj = threadIdx.x % WTJ, tk = threadIdx.x / WTJ;
-  const int j = J * WTJ + tj, k = K * WTK + tk;
-  const bool lane_ok = j < ny && k < nz;
-  const int len = lane_ok ? nx : 0;  // cells of this thread's pencil
-  // Distance of this pencil from the tile's first pencil in sweep order, the way along it and
-  // (structured grids have fewer than 2^31 cells) the offsets of the neighbours.
-  const int dj = BWD ? WTJ - 1 - tj : tj, dk = BWD ? WTK - 1 - tk : tk;
+  // A thread without a pencil goes through the motions on the first one (WavePlace); its values
+  // are not stored, published or read by any other cell.
+  const WavePlace<MODE> P((int)threadIdx.x, J, K, nx, ny, nz);
+  const int tj = P.tj, tk = P.tk;
+  const int len = P.on ? nx : 0;  // cells of this thread's pencil
   constexpr int dir = BWD ? -1 : 1;
   const int nsteps = nx + WTJ + WTK - 2;
-  const bool has_ny = BWD ? j + 1 < ny : j > 0, has_nz = BWD ? k + 1 < nz : k > 0;
-  const bool edge_y = lane_ok && dj == 0 && has_ny, edge_z = lane_ok && dk == 0 && has_nz;
-  // The neighbours along j and k: IC(0) backward reads their rows' coefficients, Gauss-Seidel
-  // the values not updated yet. Where there is none the cell's own entry stands in, unused.
-  const bool has_oy = MODE == IC0_BWD ? has_ny : (BWD ? j > 0 : j + 1 < ny);
-  const bool has_oz = MODE == IC0_BWD ? has_nz : (BWD ? k > 0 : k + 1 < nz);
-  const int oy = has_oy ? (MODE == IC0_BWD ? nx : dir * nx) : 0, oz = has_oz ? (MODE == IC0_BWD ? nx * ny : dir * nx * ny) : 0;
-  // Where a new value along j or k is read: the tile's previous step, or the ring.
-  const int near_y = has_ny && !edge_y ? (int)threadIdx.x - dir : (int)threadIdx.x;
-  const int near_z = has_nz && !edge_z ? (int)threadIdx.x - dir * WTJ : (int)threadIdx.x;
-  const int ring_y = 2 * WCT + tk * WRING, ring_z = 2 * WCT + (WTK + tj) * WRING;
-  const bool pub_y = lane_ok && dj == WTJ - 1 && (BWD ? J > 0 : J + 1 < A.tiles_j) && t != A.hold_tile;
-  const bool pub_z = lane_ok && dk == WTK - 1 && (BWD ? K > 0 : K + 1 < A.tiles_k) && t != A.hold_tile;
+  const bool pub_y = P.on && P.dj == WTJ - 1 && (BWD ? J > 0 : J + 1 < A.tiles_j) && t != A.hold_tile;
+  const bool pub_z = P.on && P.dk == WTK - 1 && (BWD ? K > 0 : K + 1 < A.tiles_k) && t != A.hold_tile;
   ulonglong2* pub = A.halo + (long long)t * nx * WHALO;
-  // A thread without a pencil goes through the motions on the first one; its values are not
-  // stored, published or read by any other cell.
-  const int row = lane_ok ? (k * ny + j) * nx : 0;
   using Cell = WaveCell<MODE, UNIFORM>;
   Cell cell[WPF];
-  int fat = -dj - dk;  // the cell (in sweep order) fetched next
+  int fat = -P.dj - P.dk;  // the cell (in sweep order) fetched next
   // No branch: outside the pencil its end cell is fetched again, unused.
   auto fetch = [&](Cell& C) {
     const int at = min(max(fat, 0), nx - 1);
-    const int c = row + (BWD ? nx - 1 - at : at);
+    const int c = P.cell(at, nx);
     C.fl = A.flags[c];
     C.d = A.diag[c];
     C.rd = A.rdiag[c];
@@ -275,16 +253,16 @@ __global__ void __launch_bounds__(WTHREADS) k_wave(WaveArgs A) {
     } else if (MODE == IC0_BWD) {
       // Rows (k+1), (j+1), (i+1), each with its coefficient towards this cell.
       C.in = A.x[c];
-      C.o[0] = A.lx[at > 0 ? c + 1 : c];
-      C.o[1] = A.ly[c + oy];
-      C.o[2] = A.lz[c + oz];
+      C.o[0] = A.lx[c + P.ox(at, nx)];
+      C.o[1] = A.ly[c + P.oy];
+      C.o[2] = A.lz[c + P.oz];
     } else {
       C.in = A.in[c];
-      C.o[0] = A.x[at + 1 < nx ? c + dir : c];
-      C.o[1] = A.x[c + oy];
-      C.o[2] = A.x[c + oz];
+      C.o[0] = A.x[c + P.ox(at, nx)];
+      C.o[1] = A.x[c + P.oy];
+      C.o[2] = A.x[c + P.oz];
       if (!UNIFORM) {
-        const int q[3] = {BWD ? nx - 1 - at : at, lane_ok ? j : 0, lane_ok ? k : 0};
+        const int q[3] = {BWD ? nx - 1 - at : at, P.on ? P.j : 0, P.on ? P.k : 0};
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
           int f[3] = {q[0], q[1], q[2]};
@@ -315,27 +293,26 @@ __global__ void __launch_bounds__(WTHREADS) k_wave(WaveArgs A) {
     }
   };
   double prev = 0.0;  // this pencil's value at the previous cell in sweep order
-  int have_y = edge_y ? 0 : nx, have_z = edge_z ? 0 : nx;  // received values as last seen
+  int have_y = P.edge_y ? 0 : nx, have_z = P.edge_z ? 0 : nx;  // received values as last seen
 #pragma unroll
   for (int m = 0; m < WPF; ++m) fetch(cell[m]);
   old_terms(cell[0]);
-  int at = -dj - dk, c = row + (BWD ? nx - 1 : 0) + dir * at;
+  int at = -P.dj - P.dk, c = P.row + (BWD ? nx - 1 : 0) + dir * at;
   for (int s0 = 0; s0 < nsteps; s0 += WPF) {  // steps past nsteps - 1 find no cell in range
 #pragma unroll
     for (int m = 0; m < WPF; ++m, ++at, c += dir) {
       Cell& C = cell[m];
       const bool on = (unsigned)at < (unsigned)len;
       while (__any_sync(0xffffffffu, on && (have_y <= at || have_z <= at))) {
-        if (edge_y) have_y = seen[tk];
-        if (edge_z) have_z = seen[WTK + tj];
+        if (P.edge_y) have_y = seen[tk];
+        if (P.edge_z) have_z = seen[WTK + tj];
         if (bail) have_y = have_z = nx;
       }
       asm volatile("bar.sync 1, %0;" ::"n"(WCT) : "memory");  // the step before is in sh
       if (m == 0 && threadIdx.x == 0) passed = s0;
       const int before = ((m + 1) & 1) * WCT;  // WPF is even: step parity is m's
-      const int slot = at & (WRING - 1);
-      const double newy = sh[edge_y ? ring_y + slot : before + near_y];
-      const double newz = sh[edge_z ? ring_z + slot : before + near_z];
+      const double newy = sh[P.new_y(at, before)];
+      const double newz = sh[P.new_z(at, before)];
       double v = C.in;
       if (MODE == IC0_FWD) {
         // Ascending columns: (k-1), (j-1), (i-1).
