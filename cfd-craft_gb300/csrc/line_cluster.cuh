@@ -234,13 +234,11 @@ __global__ void __launch_bounds__(LCT, 1) k_line_sweep(LineLev L, const Scalars*
       ++k;
     }
     if (!SHX) __threadfence();
-    __syncwarp();
     pc_arrive();
     if (!ready && valid(g)) {
       prepare();
       ready = true;
     }
-    __syncwarp();
     pc_wait();
   }
   asm volatile("cp.async.wait_all;" ::: "memory");

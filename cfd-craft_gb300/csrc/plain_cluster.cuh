@@ -87,8 +87,16 @@ __device__ __forceinline__ double pc_ld(unsigned base, unsigned col) {
   }
   return v;
 }
-__device__ __forceinline__ void pc_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void pc_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// The aligned forms ask for the whole warp to be at the instruction together, which nothing else
+// promises behind a predicated store, the branch of div_rare or a loop of a few lanes.
+__device__ __forceinline__ void pc_arrive() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void pc_wait() {
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 
 // v / d through the reciprocal; the extra correction where some lane of the warp needs it.
 __device__ __forceinline__ double pc_div(double v, double d, double rd, bool on) {

@@ -308,7 +308,8 @@ __global__ void __launch_bounds__(WTHREADS) k_wave(WaveArgs A) {
         if (P.edge_z) have_z = seen[WTK + tj];
         if (bail) have_y = have_z = nx;
       }
-      asm volatile("bar.sync 1, %0;" ::"n"(WCT) : "memory");  // the step before is in sh
+      // The step before is in sh. (The vote that ends the loop above has brought the warp together.)
+      asm volatile("bar.sync 1, %0;" ::"n"(WCT) : "memory");
       if (m == 0 && threadIdx.x == 0) passed = s0;
       const int before = ((m + 1) & 1) * WCT;  // WPF is even: step parity is m's
       const double newy = sh[P.new_y(at, before)];
