@@ -664,11 +664,11 @@ namespace {
 // Dense Cholesky solves of the terminal level, one warp per block.
 __global__ void k_direct(int nblocks, const int* __restrict__ ioff, const int* __restrict__ idx,
                          const long long* __restrict__ foff, const double* __restrict__ f,
-                         const double* __restrict__ frd, const double* rhs, double* x, const Scalars* S) {
+                         const double* rhs, double* x, const Scalars* S) {
   if (S && S->done) return;
   const int bk = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (bk >= nblocks) return;
-  pc_direct(idx + ioff[bk], ioff[bk + 1] - ioff[bk], f + foff[bk], frd + ioff[bk], rhs, x);
+  pc_direct(idx + ioff[bk], ioff[bk + 1] - ioff[bk], f + foff[bk], rhs, x);
 }
 
 template <class Bar>
@@ -1057,8 +1057,8 @@ void launch_vcycle(cfdg_grid* G, const double* r, double* z, const Scalars* S) {
     }
     if (L.terminal) {
       if (L.nblocks > 0) {
-        k_direct<<<(L.nblocks + 1) / 2, 64, 0, s>>>(L.nblocks, L.d_ioff, L.d_idx, L.d_foff, L.d_fac, L.d_frd, L.rhs,
-                                                    L.x, S); tick(G);
+        k_direct<<<(L.nblocks + 1) / 2, 64, 0, s>>>(L.nblocks, L.d_ioff, L.d_idx, L.d_foff, L.d_fac, L.rhs, L.x,
+                                                    S); tick(G);
       }
       launch_center(G, L.groups, L.ngroups, L.x, S);
       break;
@@ -1237,6 +1237,30 @@ int refresh_weights(cfdg_grid* G) {
   return 0;
 }
 
+// What the wavefront sweeps of a grid hand over with: tickets and epochs, and the entries between
+// the tiles (no epoch is 0, so zeroed entries are unset). For the first preconditioner that
+// sweeps so.
+int ensure_wave(cfdg_grid* G) {
+  if (G->wave_halo) return 0;
+  const size_t n = (size_t)wave_halo_size(G->h.n[0], G->tiles_j, G->tiles_k);
+  const size_t held = G->arena.ptrs.size();
+  const uint64_t held_bytes = G->arena.bytes;
+  unsigned long long* sync = nullptr;
+  ulonglong2* halo = nullptr;
+  int e = G->arena.alloc(&sync, 3);
+  if (!e) e = G->arena.alloc(&halo, n);
+  if (e) {
+    G->arena.rollback(held, held_bytes);
+    return e;
+  }
+  CU(cudaMemsetAsync(sync, 0, 3 * sizeof(unsigned long long), G->stream));
+  CU(cudaMemsetAsync(halo, 0, std::max<size_t>(n, 1) * sizeof(ulonglong2), G->stream));
+  CU(cudaStreamSynchronize(G->stream));
+  G->wave_sync = sync;
+  G->wave_halo = halo;
+  return 0;
+}
+
 int build_ic0_dev(cfdg_grid* G) {
   Ic0 F;
   build_ic0(G->h, F);
@@ -1266,8 +1290,9 @@ int build_ic0_dev(cfdg_grid* G) {
     if (int e = D->arena.upload(&D->lx, lx, s)) return e;
     if (int e = D->arena.upload(&D->ly, ly, s)) return e;
     if (int e = D->arena.upload(&D->lz, lz, s)) return e;
+    if (int e = ensure_wave(G)) return e;
     if (int e = D->arena.alloc(&D->rdiag, N)) return e;
-    k_recip<<<grid_blocks(N), BLOCK, 0, s>>>(D->diag, D->rdiag, N, G->wave_err + 1); tick(G);
+    k_recip<<<grid_blocks(N), BLOCK, 0, s>>>(D->diag, D->rdiag, N, reinterpret_cast<int*>(G->wave_sync + 2)); tick(G);
     CU(cudaGetLastError());
   }
   CU(cudaStreamSynchronize(s));
@@ -1367,17 +1392,6 @@ double host_recip(double d) {
   if (!(d >= 0x1p-60 && d <= 0x1p60)) return 0.0;
   const double r = 1.0 / d;
   return std::fabs(std::fma(r, d, -1.0)) <= 0x1p-54 ? r : -r;
-}
-
-// Reciprocals of a terminal level's factor diagonals, by solved row.
-std::vector<double> direct_recip(const MgLevel& M) {
-  std::vector<double> rd(M.direct_idx.col.size());
-  for (int b = 0; b < M.direct_idx.rows(); ++b) {
-    const int n = M.direct_idx.off[b + 1] - M.direct_idx.off[b];
-    for (int i = 0; i < n; ++i)
-      rd[M.direct_idx.off[b] + i] = host_recip(M.direct_factor[M.direct_off[b] + (size_t)i * n + i]);
-  }
-  return rd;
 }
 
 // The sweeps of an anisotropic level (line_cluster.cuh): a cluster of 16 blocks (8 where the
@@ -1559,7 +1573,6 @@ int plan_plain_cluster(DevHierarchy& D, const Hierarchy& H, cudaStream_t s) {
     if (L.terminal) {
       L.nblocks = V.nblocks;
       L.ioff = V.d_ioff, L.idx = V.d_idx, L.foff = V.d_foff, L.fac = V.d_fac;
-      L.frd = V.d_frd;
       continue;
     }
     L.roff = V.restrict_.off, L.rcol = V.restrict_.col, L.rval = V.restrict_.val;
@@ -1695,11 +1708,13 @@ int build_mg_dev(cfdg_grid* G, const Poller& poll) {
     if (l == 0 || D->lines)
       if (int e = upload_rows(*D, L, M, !D->lines, s)) return e;
     if (l == 0 && D->full0) {
+      if (int e = ensure_wave(G)) return e;
       if (int e = D->arena.alloc(&L.rdiag, L.n)) return e;
-      CU(cudaMemsetAsync(G->wave_err + 1, 0, sizeof(int), s));
-      k_recip<<<grid_blocks(L.n), BLOCK, 0, s>>>(L.diag, L.rdiag, L.n, G->wave_err + 1); tick(G);
+      int* some = reinterpret_cast<int*>(G->wave_sync + 2);
+      CU(cudaMemsetAsync(some, 0, sizeof(int), s));
+      k_recip<<<grid_blocks(L.n), BLOCK, 0, s>>>(L.diag, L.rdiag, L.n, some); tick(G);
       int extra = 1;
-      CU(cudaMemcpyAsync(&extra, G->wave_err + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
+      CU(cudaMemcpyAsync(&extra, some, sizeof(int), cudaMemcpyDeviceToHost, s));
       CU(cudaStreamSynchronize(s));
       L.rd_extra = extra != 0;
     }
@@ -1714,23 +1729,24 @@ int build_mg_dev(cfdg_grid* G, const Poller& poll) {
       std::vector<long long> foff(M.direct_off.begin(), M.direct_off.end());
       if (int e = D->arena.upload(&L.d_foff, foff, s)) return e;
       if (int e = D->arena.upload(&L.d_fac, M.direct_factor, s)) return e;
-      std::vector<double> rd = direct_recip(M);
-      if (int e = D->arena.upload(&L.d_frd, rd, s)) return e;
     } else {
       if (int e = upload_csr(D->arena, M.prolong, L.prolong, s)) return e;
       if (int e = upload_csr(D->arena, M.restrict, L.restrict_, s)) return e;
     }
     // Level 0 in full-grid layout works on the solver's own vectors (a closed group's gauge
-    // changes the right-hand side, which is the residual that the solver keeps).
+    // changes the right-hand side, which is the residual that the solver keeps; A p is used up
+    // when the preconditioner runs).
     if (l == 0 && D->full0) {
       L.x = G->z;
+      L.res = G->ap;
       if (L.ngroups == 0) L.rhs = G->r;
     }
     if (!L.rhs)
       if (int e = D->arena.alloc(&L.rhs, L.n)) return e;
     if (!L.x)
-      if (int e = D->arena.alloc(&L.x, L.n + 1)) return e;  // + a zero behind a block-smoothed level's
-    if (int e = D->arena.alloc(&L.res, L.n)) return e;
+      if (int e = D->arena.alloc(&L.x, L.n + (M.lines.empty() ? 0 : 1))) return e;  // + a zero behind the rows
+    if (!L.res)
+      if (int e = D->arena.alloc(&L.res, L.n)) return e;
     if (!M.lines.empty()) {
       // The reference builds one block group per level.
       if (int e = plan_lines(*D, L, M, M.lines[0], s)) return e;
@@ -1862,21 +1878,8 @@ int prepare_mg_impl(cfdg_grid* G, const Poller& poll, cfdg_info* info) {
   return 0;
 }
 
-// The hand-off entries of the wavefront sweeps (no epoch is 0, so zeroed entries are unset).
-int ensure_wave(cfdg_grid* G) {
-  if (!G->structured || G->wave_halo) return 0;
-  const size_t n = (size_t)G->tiles_j * G->tiles_k * G->h.n[0] * WHALO;
-  ulonglong2* p = nullptr;
-  if (int e = G->arena.alloc(&p, n)) return e;
-  CU(cudaMemsetAsync(p, 0, n * sizeof(ulonglong2), G->stream));
-  CU(cudaStreamSynchronize(G->stream));
-  G->wave_halo = p;
-  return 0;
-}
-
 // pressure.rs:55-97: the cached factor, or the hierarchy checked against its signature.
 int prepare_preconditioner(cfdg_grid* G, const Poller& poll, cfdg_info* info) {
-  if (int e = ensure_wave(G)) return e;
   if (G->preconditioner == CFDG_PRECOND_MULTIGRID) return prepare_mg_impl(G, poll, info);
   if (!G->ic0) {
     reset_chunk(G);
@@ -2912,7 +2915,7 @@ int cfdg_grid_open(cfdg_context* ctx, const cfdg_grid_desc* d, cfdg_grid** out) 
       (e = A.alloc(&G->d_fw, F)) || (e = A.alloc(&G->x, N)) || (e = A.alloc(&G->r, N)) || (e = A.alloc(&G->z, N)) ||
       (e = A.alloc(&G->p, N)) || (e = A.alloc(&G->ap, N)) || (e = A.alloc(&G->bc, N)) || (e = A.alloc(&G->b, N)) ||
       (e = A.alloc(&G->terms, N)) || (e = A.alloc(&G->u, F)) || (e = A.alloc(&G->pp, N)) ||
-      (e = A.alloc(&G->partials, MAX_BLOCKS)) || (e = A.alloc(&G->S, 1))) {
+      (e = A.alloc(&G->partials, MAX_BLOCKS)) || (e = A.alloc(&G->S, 1)) || (e = A.alloc(&G->wave_err, 1))) {
     A.release();
     return e;
   }
@@ -2931,8 +2934,6 @@ int cfdg_grid_open(cfdg_context* ctx, const cfdg_grid_desc* d, cfdg_grid** out) 
   G->structured = !h.periodic[0] && !h.periodic[1] && !h.periodic[2] && h.n[0] >= 2 && h.n[1] >= 2 && h.n[2] >= 2;
   G->tiles_j = (h.n[1] + WTJ - 1) / WTJ;
   G->tiles_k = (h.n[2] + WTK - 1) / WTK;
-  if ((e = A.alloc(&G->wave_sync, 2)) || (e = A.alloc(&G->wave_err, 2))) return e;
-  CU(cudaMemsetAsync(G->wave_sync, 0, 2 * sizeof(unsigned long long), s));
   CU(cudaMemsetAsync(G->wave_err, 0, sizeof(int), s));
   if ((e = refresh_weights(G.get()))) return e;
   CU(cudaStreamSynchronize(s));

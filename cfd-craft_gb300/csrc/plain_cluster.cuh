@@ -65,7 +65,7 @@ struct PcLev {
   double *grhs, *gx, *gres;
   const int *ioff, *idx;
   const long long* foff;
-  const double *fac, *frd;   // terminal factors and the reciprocals of their diagonals (by solved row)
+  const double* fac;         // terminal factors
 };
 struct PcPlan {
   int nl;
@@ -249,8 +249,7 @@ __device__ void pc_sweep_level(const PcLev& L, int rank, int* ls, unsigned char*
 // lane keeps its row and takes the solved ones off in ascending order; backward, the lanes
 // form a row's products and every lane runs the row's subtractions in ascending order. Blocks
 // of more than 32 rows by one thread.
-__device__ __noinline__ void pc_direct(const int* ix, int n, const double* f, const double* frd, const double* rhs,
-                                       double* x) {
+__device__ __noinline__ void pc_direct(const int* ix, int n, const double* f, const double* rhs, double* x) {
   const int ln = threadIdx.x & 31;
   if (n > 32) {
     if (ln == 0) {
@@ -268,7 +267,7 @@ __device__ __noinline__ void pc_direct(const int* ix, int n, const double* f, co
     return;
   }
   const bool on = ln < n;
-  const double d = on ? __ldg(&f[ln * n + ln]) : 1.0, rd = on ? __ldg(&frd[ln]) : 0.0;
+  const double d = on ? __ldg(&f[ln * n + ln]) : 1.0, rd = recip_of(d);
   double v = on ? rhs[ix[ln]] : 0.0, s = 0.0;
   double fj = on && ln > 0 ? __ldg(&f[ln * n]) : 0.0;
   for (int j = 0; j < n; ++j) {
@@ -359,7 +358,7 @@ __global__ void __launch_bounds__(PCT, 1) k_plain_cluster(const PcPlan* plan, in
       if (L.terminal) {
         if (rank == 0) {
           for (int bk = threadIdx.x >> 5; bk < L.nblocks; bk += PCT / 32)
-            pc_direct(L.idx + L.ioff[bk], L.ioff[bk + 1] - L.ioff[bk], L.fac + L.foff[bk], L.frd + L.ioff[bk], rhs, x);
+            pc_direct(L.idx + L.ioff[bk], L.ioff[bk + 1] - L.ioff[bk], L.fac + L.foff[bk], rhs, x);
           __syncthreads();
           for (int i = threadIdx.x; i < L.n; i += PCT) L.gx[i] = x[i];
         }

@@ -165,7 +165,6 @@ struct DevLevel {
   long long* d_foff = nullptr;
   double* d_fac = nullptr;
   double *rhs = nullptr, *x = nullptr, *res = nullptr;
-  double* d_frd = nullptr;  // reciprocals of the terminal factors' diagonals, by solved row
   // Anisotropic levels: the block smoother, whether its iterate lives in the cluster's shared
   // memory, the dynamic shared memory of a sweep and the device bytes held.
   bool lines = false, lshx = false;
@@ -252,11 +251,12 @@ struct cfdg_grid {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   bool structured = false;  // no periodic axis: pipelined wavefront sweeps on the fine level
   int tiles_j = 0, tiles_k = 0;
-  // Wavefront sweeps (wave.cuh): tickets taken and the last epoch that gave up; the boundary
-  // values handed from tile to tile, allocated by the first plain preconditioner.
+  // Wavefront sweeps (wave.cuh): tickets taken, the last epoch that gave up and the scratch of
+  // k_recip; the boundary values handed from tile to tile. Allocated by the first preconditioner
+  // that sweeps so.
   unsigned long long* wave_sync = nullptr;
   ulonglong2* wave_halo = nullptr;
-  int* wave_err = nullptr;   // [0] set when a wavefront wait gave up, [1] scratch of k_recip
+  int* wave_err = nullptr;   // set when a wavefront wait gave up
   long long wave_spin_limit = WAVE_SPIN_LIMIT;  // cfdg_debug_wave_stall
   int wave_hold_tile = -1;
   std::shared_ptr<cfdg::Hierarchy> host_mg;  // the hierarchy as uploaded (level 0 re-indexed when full0)

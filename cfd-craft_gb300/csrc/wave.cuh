@@ -58,7 +58,7 @@ struct WaveArgs {
   long long face_off[3];
   int fdim[3][3];
   unsigned long long* sync;  // [0] tickets taken so far, [1] epoch of the last launch that gave up
-  ulonglong2* halo;          // [tile][step along x][WHALO]: a boundary value's bits and its epoch
+  ulonglong2* halo;          // boundary values (wave_halo_y, wave_halo_z): their bits and epoch
   int* error;                // persistent: set to 1 when a wait gave up
   const Scalars* S;
   long long spin_limit;  // polls before a wait gives up (WAVE_SPIN_LIMIT)
@@ -186,8 +186,10 @@ __global__ void __launch_bounds__(WTHREADS) k_wave(WaveArgs A) {
     const int p = along_j ? lane : lane - WTK;
     bool open = lane < WHALO && (along_j ? (BWD ? J + 1 < A.tiles_j : J > 0) && K * WTK + p < nz
                                          : (BWD ? K + 1 < A.tiles_k : K > 0) && J * WTJ + p < ny);
-    const int back = along_j ? 1 : A.tiles_j;  // the producer's ticket is t - back
-    const ulonglong2* src = A.halo + (long long)(open ? t - back : t) * nx * WHALO + (open ? lane : 0);
+    const ulonglong2* src = A.halo;
+    if (open)
+      src += p + (along_j ? WavePlace<MODE>::from_y(J, K, nx, A.tiles_j)
+                          : WavePlace<MODE>::from_z(J, K, nx, A.tiles_j, A.tiles_k));
     // The pencil's first cell is used at step `late`: entries below passed - late are free.
     const int late = BWD ? (along_j ? WTK : WTJ) - 1 - p : p;
     int got = 0;
@@ -198,7 +200,7 @@ __global__ void __launch_bounds__(WTHREADS) k_wave(WaveArgs A) {
       if (room) {
         ulonglong2 v[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) v[q] = ld_halo(src + (long long)min(got + q, nx - 1) * WHALO);
+        for (int q = 0; q < 4; ++q) v[q] = ld_halo(src + (long long)min(got + q, nx - 1) * WTK);
 #pragma unroll
         for (int q = 0; q < 4; ++q)
           if (m == q && got + q < nx && v[q].y == epoch) {
@@ -236,7 +238,9 @@ __global__ void __launch_bounds__(WTHREADS) k_wave(WaveArgs A) {
   const int nsteps = nx + WTJ + WTK - 2;
   const bool pub_y = P.on && P.dj == WTJ - 1 && (BWD ? J > 0 : J + 1 < A.tiles_j) && t != A.hold_tile;
   const bool pub_z = P.on && P.dk == WTK - 1 && (BWD ? K > 0 : K + 1 < A.tiles_k) && t != A.hold_tile;
-  ulonglong2* pub = A.halo + (long long)t * nx * WHALO;
+  // Entries (fewer than half the cells) that this pencil's next values go to.
+  int to_y = (pub_y ? (int)P.to_y(J, K, nx, A.tiles_j) : 0) - (P.dj + P.dk) * WTK;
+  int to_z = (pub_z ? (int)P.to_z(J, K, nx, A.tiles_j, A.tiles_k) : 0) - (P.dj + P.dk) * WTJ;
   using Cell = WaveCell<MODE, UNIFORM>;
   Cell cell[WPF];
   int fat = -P.dj - P.dk;  // the cell (in sweep order) fetched next
@@ -300,7 +304,7 @@ __global__ void __launch_bounds__(WTHREADS) k_wave(WaveArgs A) {
   int at = -P.dj - P.dk, c = P.row + (BWD ? nx - 1 : 0) + dir * at;
   for (int s0 = 0; s0 < nsteps; s0 += WPF) {  // steps past nsteps - 1 find no cell in range
 #pragma unroll
-    for (int m = 0; m < WPF; ++m, ++at, c += dir) {
+    for (int m = 0; m < WPF; ++m, ++at, c += dir, to_y += WTK, to_z += WTJ) {
       Cell& C = cell[m];
       const bool on = (unsigned)at < (unsigned)len;
       while (__any_sync(0xffffffffu, on && (have_y <= at || have_z <= at))) {
@@ -346,8 +350,8 @@ __global__ void __launch_bounds__(WTHREADS) k_wave(WaveArgs A) {
       }
       sh[(m & 1) * WCT + threadIdx.x] = v;
       prev = v;
-      st_halo(pub + at * WHALO + tk, v, epoch, on && pub_y);
-      st_halo(pub + at * WHALO + WTK + tj, v, epoch, on && pub_z);
+      st_halo(A.halo + to_y, v, epoch, on && pub_y);
+      st_halo(A.halo + to_z, v, epoch, on && pub_z);
       if (on) A.x[c] = v;
       old_terms(cell[(m + 1) % WPF]);
       fetch(C);
@@ -355,6 +359,7 @@ __global__ void __launch_bounds__(WTHREADS) k_wave(WaveArgs A) {
   }
 }
 
+static_assert(WTJ == WTK, "the receiver's lanes step alike along both boundaries");
 static_assert(WPF % 2 == 0, "the step's buffer is chosen by its place in the unrolled group");
 
 }  // namespace cfdg

@@ -19,6 +19,15 @@ constexpr int WSHARED = 2 * WCT + WHALO * WRING;  // the last two steps' values,
 
 enum WaveMode { IC0_FWD = 0, IC0_BWD = 1, GS_FWD = 2, GS_BWD = 3 };
 
+// Hand-off entries: the boundary pencils between tiles that follow one another along j, [K][J][step
+// along x][k in the tile], then those along k, [K][J][step along x][j in the tile]; J, K the lower
+// tile of the two. A sweep either way uses the same ones.
+CFDG_HD long long wave_halo_y(int J, int K, int nx, int tiles_j) { return ((long long)K * (tiles_j - 1) + J) * nx * WTK; }
+CFDG_HD long long wave_halo_z(int J, int K, int nx, int tiles_j, int tiles_k) {
+  return (long long)tiles_k * (tiles_j - 1) * nx * WTK + ((long long)K * tiles_j + J) * nx * WTJ;
+}
+CFDG_HD long long wave_halo_size(int nx, int tiles_j, int tiles_k) { return wave_halo_z(0, tiles_k - 1, nx, tiles_j, tiles_k); }
+
 template <int MODE>
 struct WavePlace {
   static constexpr bool BWD = MODE == IC0_BWD || MODE == GS_BWD;
@@ -56,6 +65,17 @@ struct WavePlace {
   CFDG_HD int cell(int at, int nx) const { return row + (BWD ? nx - 1 - at : at); }
   static CFDG_HD int ox(int at, int nx) {
     return MODE == IC0_BWD ? (at > 0 ? 1 : 0) : (at + 1 < nx ? dir : 0);
+  }
+  // Where the new values that the tile before this one along j (k) hands over start, this one's
+  // lane first, and where this pencil's go to the tile behind it; the values of a pencil follow
+  // one another WTK (WTJ) entries apart. Only for tiles that have one before, behind.
+  static CFDG_HD long long from_y(int J, int K, int nx, int tiles_j) { return wave_halo_y(BWD ? J : J - 1, K, nx, tiles_j); }
+  static CFDG_HD long long from_z(int J, int K, int nx, int tiles_j, int tiles_k) {
+    return wave_halo_z(J, BWD ? K : K - 1, nx, tiles_j, tiles_k);
+  }
+  CFDG_HD long long to_y(int J, int K, int nx, int tiles_j) const { return wave_halo_y(BWD ? J - 1 : J, K, nx, tiles_j) + tk; }
+  CFDG_HD long long to_z(int J, int K, int nx, int tiles_j, int tiles_k) const {
+    return wave_halo_z(J, BWD ? K - 1 : K, nx, tiles_j, tiles_k) + tj;
   }
   // Places in the shared array of the new values along j and k; `at` is any number.
   CFDG_HD int new_y(int at, int before) const {

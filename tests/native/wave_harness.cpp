@@ -2,10 +2,37 @@
 // (cfd-craft_gb300/csrc/wave_place.hpp, the arithmetic that the kernel runs) over all places of
 // its pencil and counts the reads outside the arrays and the neighbours that are not the cell's.
 #include <cstdint>
+#include <vector>
 
 #include "wave_place.hpp"
 
 using namespace cfdg;
+
+// The hand-off entries: every value goes where the tile behind reads it, none is shared.
+template <int MODE>
+static void halo(int nx, int ny, int nz, int64_t* out) {
+  using P = WavePlace<MODE>;
+  const int tj = (ny + WTJ - 1) / WTJ, tk = (nz + WTK - 1) / WTK, s = P::dir;
+  std::vector<int> used(wave_halo_size(nx, tj, tk), 0);
+  for (int K = 0; K < tk; ++K)
+    for (int J = 0; J < tj; ++J)
+      for (int tid = 0; tid < WCT; ++tid) {
+        const P p(tid, J, K, nx, ny, nz);
+        if (!p.on) continue;
+        for (int way = 0; way < 2; ++way) {
+          const int J2 = way ? J : J + s, K2 = way ? K + s : K, d = way ? p.dk : p.dj;
+          if (d != WTJ - 1 || J2 < 0 || J2 >= tj || K2 < 0 || K2 >= tk) continue;
+          const long long to = way ? p.to_z(J, K, nx, tj, tk) : p.to_y(J, K, nx, tj);
+          const long long from =
+              way ? P::from_z(J2, K2, nx, tj, tk) + p.tj : P::from_y(J2, K2, nx, tj) + p.tk;
+          if (to != from) ++out[2];
+          for (int at = 0; at < nx; ++at) {
+            const long long e = to + (long long)at * WTK;
+            if (e < 0 || e >= (long long)used.size() || used[e]++) ++out[0];
+          }
+        }
+      }
+}
 
 template <int MODE>
 static void scan(int nx, int ny, int nz, int64_t* out) {
@@ -52,12 +79,12 @@ static void scan(int nx, int ny, int nz, int64_t* out) {
       }
 }
 
-// out: reads outside the arrays, reads outside the shared array or its parts, wrong neighbours,
+// out: reads (and hand-off entries) outside the arrays, reads outside the shared array or its parts, wrong neighbours,
 // cells visited by their own threads (with the clamped steps).
 extern "C" void wave_scan(int mode, int nx, int ny, int nz, int64_t* out) {
   for (int a = 0; a < 4; ++a) out[a] = 0;
-  if (mode == IC0_FWD) scan<IC0_FWD>(nx, ny, nz, out);
-  if (mode == IC0_BWD) scan<IC0_BWD>(nx, ny, nz, out);
-  if (mode == GS_FWD) scan<GS_FWD>(nx, ny, nz, out);
-  if (mode == GS_BWD) scan<GS_BWD>(nx, ny, nz, out);
+  if (mode == IC0_FWD) scan<IC0_FWD>(nx, ny, nz, out), halo<IC0_FWD>(nx, ny, nz, out);
+  if (mode == IC0_BWD) scan<IC0_BWD>(nx, ny, nz, out), halo<IC0_BWD>(nx, ny, nz, out);
+  if (mode == GS_FWD) scan<GS_FWD>(nx, ny, nz, out), halo<GS_FWD>(nx, ny, nz, out);
+  if (mode == GS_BWD) scan<GS_BWD>(nx, ny, nz, out), halo<GS_BWD>(nx, ny, nz, out);
 }
