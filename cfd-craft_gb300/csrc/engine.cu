@@ -1010,21 +1010,26 @@ void launch_plain_cluster(cfdg_grid* G, const DevHierarchy& H, int from, int wha
   tick(G);
 }
 
-// A block Gauss-Seidel sweep of an anisotropic level (line_cluster.cuh).
-void launch_lines(cfdg_grid* G, const DevLevel& L, bool backward, const Scalars* S) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(L.ll.nb, 1, 1);
+void line_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, int blocks, int smem, cudaStream_t s) {
+  cfg.gridDim = dim3(blocks, 1, 1);
   cfg.blockDim = dim3(LCT, 1, 1);
-  cfg.dynamicSmemBytes = (size_t)L.lsmem;
-  cfg.stream = G->stream;
-  cudaLaunchAttribute at[1];
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.stream = s;
   at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = L.ll.nb;
+  at[0].val.clusterDim.x = blocks;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, line_kernel(backward, L.lshx), L.ll, S);
+}
+
+// A block Gauss-Seidel sweep of an anisotropic level (line_cluster.cuh).
+void launch_lines(cfdg_grid* G, const DevLevel& L, bool backward, const Scalars* S) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  line_config(cfg, at, L.lean ? L.le.nb : L.ll.nb, L.lsmem, G->stream);
+  if (L.lean) cudaLaunchKernelEx(&cfg, backward ? k_line_sweep_lean<true> : k_line_sweep_lean<false>, L.le, S);
+  else cudaLaunchKernelEx(&cfg, line_kernel(backward, L.lshx), L.ll, S);
   tick(G);
 }
 
@@ -1396,12 +1401,15 @@ double host_recip(double d) {
 
 // The sweeps of an anisotropic level (line_cluster.cuh): a cluster of 16 blocks (8 where the
 // device does not schedule the non-portable size), the iterate in its shared memory and the
-// records copied ahead where both fit, else only the copies, else neither.
+// records copied ahead where both fit, else only the copies, else neither. NO_PLAN where the level
+// is beyond what the records describe (lean_lines takes it).
+constexpr int NO_PLAN = 1;
 int plan_lines(DevHierarchy& D, DevLevel& L, const MgLevel& M, const LineBlocks& B, cudaStream_t s) {
   L.lines = true;
   LineLev& P = L.ll;
   P.n = M.n, P.len = B.length, P.bw = B.bandwidth, P.count = B.count(), P.ndep = B.fwd.levels();
   const int len = P.len, W = P.bw + 1;
+  if (4LL * (P.ndep + 1) + 16 > LC_SMEM) return NO_PLAN;  // the dependency levels' starts are kept there
   std::vector<int> most(P.count, 0), where(P.count), block(M.n), place(M.n);
   int wide = 0;
   for (int q = 0; q < P.count; ++q) {
@@ -1412,6 +1420,7 @@ int plan_lines(DevHierarchy& D, DevLevel& L, const MgLevel& M, const LineBlocks&
     }
     wide = std::max(wide, most[q]);
   }
+  if (((long long)len + P.bw) * W * 8 + 20LL * wide * len > (1LL << 30)) return NO_PLAN;  // offsets in a record are ints
   P.wide = wide;
   P.val_at = 16 + (len + P.bw) * W * 8;
   P.col_at = P.val_at + wide * len * 8;
@@ -1433,17 +1442,9 @@ int plan_lines(DevHierarchy& D, DevLevel& L, const MgLevel& M, const LineBlocks&
     for (int way = 0; way < 2; ++way) {
       const auto k = line_kernel(way == 1, L.lshx);
       cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(P.nb, 1, 1);
-      cfg.blockDim = dim3(LCT, 1, 1);
-      cfg.dynamicSmemBytes = (size_t)L.lsmem;
       cudaLaunchAttribute at[1];
-      at[0].id = cudaLaunchAttributeClusterDimension;
-      at[0].val.clusterDim.x = P.nb;
-      at[0].val.clusterDim.y = 1;
-      at[0].val.clusterDim.z = 1;
-      cfg.attrs = at;
-      cfg.numAttrs = 1;
-      if (L.lsmem > LC_SMEM || cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+      line_config(cfg, at, P.nb, L.lsmem, s);
+      if (cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
           cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, LC_SMEM) != cudaSuccess ||
           cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) != cudaSuccess || clusters < 1) {
         cudaGetLastError();
@@ -1500,6 +1501,51 @@ int plan_lines(DevHierarchy& D, DevLevel& L, const MgLevel& M, const LineBlocks&
   P.rhs = L.rhs, P.x = L.x;
   CU(cudaMemsetAsync(L.x + M.n, 0, 8, s));
   CU(cudaStreamSynchronize(s));  // the records' host copy goes out of scope
+  return 0;
+}
+
+// The sweeps of an anisotropic level without records (line_cluster.cuh k_line_sweep_lean): the
+// bytes are the block smoother's own.
+int lean_lines(DevHierarchy& D, DevLevel& L, const MgLevel& M, const LineBlocks& B, cudaStream_t s) {
+  L.lines = L.lean = true;
+  L.lshx = false;
+  LineLean& P = L.le;
+  P.len = B.length, P.bw = B.bandwidth, P.ndep = B.fwd.levels();
+  L.ll.count = B.count();
+  const size_t scr = 8 * (size_t)LCW * P.len;
+  L.lsmem = scr <= (size_t)LC_SMEM ? (int)scr : 0;
+  for (P.nb = 16;; P.nb = 8) {
+    int clusters = 0;
+    for (const auto k : {k_line_sweep_lean<false>, k_line_sweep_lean<true>}) {
+      cudaLaunchConfig_t cfg = {};
+      cudaLaunchAttribute at[1];
+      line_config(cfg, at, P.nb, L.lsmem, s);
+      if (cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+          cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, LC_SMEM) != cudaSuccess ||
+          cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) != cudaSuccess || clusters < 1) {
+        cudaGetLastError();
+        clusters = 0;
+        break;
+      }
+    }
+    if (clusters > 0) break;
+    if (P.nb == 8) return fail(CFDG_ERR_UNSUPPORTED, "block-smoothed multigrid needs a thread-block cluster");
+  }
+  const uint64_t before = D.arena.bytes;
+  int *nodes, *off, *col, *order, *start;
+  double *val, *fac;
+  if (int e = D.arena.upload(&nodes, B.nodes, s)) return e;
+  if (int e = D.arena.upload(&off, B.outside.off, s)) return e;
+  if (int e = D.arena.upload(&col, B.outside.col, s)) return e;
+  if (int e = D.arena.upload(&val, B.outside.val, s)) return e;
+  if (int e = D.arena.upload(&fac, B.factor, s)) return e;
+  if (int e = D.arena.upload(&order, B.fwd.order, s)) return e;
+  if (int e = D.arena.upload(&start, B.fwd.start, s)) return e;
+  P.nodes = nodes, P.off = off, P.col = col, P.val = val, P.fac = fac, P.order = order, P.start = start;
+  if (L.lsmem == 0)
+    if (int e = D.arena.alloc(&P.scr, (size_t)M.n)) return e;
+  P.rhs = L.rhs, P.x = L.x;
+  L.lbytes = D.arena.bytes - before;
   return 0;
 }
 
@@ -1678,6 +1724,104 @@ int upload_rows(DevHierarchy& D, DevLevel& L, const MgLevel& M, bool orders, cud
   return D.arena.upload(&L.bwd.d_start, M.bwd.start, s);
 }
 
+// Levels 1 .. L-1 by their rows and orders, for the cooperative kernel when its grid can be
+// co-resident.
+int row_levels(DevHierarchy& D, const Hierarchy& H, cudaStream_t s) {
+  for (size_t l = 1; l < D.levels.size(); ++l)
+    if (int e = upload_rows(D, D.levels[l], H.levels[l], true, s)) return e;
+  std::vector<PLev> pl;
+  for (size_t l = 1; l < D.levels.size(); ++l) {
+    const DevLevel& L = D.levels[l];
+    PLev P{};
+    P.n = L.n;
+    P.terminal = L.terminal ? 1 : 0;
+    P.ngroups = L.ngroups;
+    P.nblocks = L.nblocks;
+    P.nfwd = (int)L.fwd.start.size() - 1;
+    P.nbwd = (int)L.bwd.start.size() - 1;
+    int dl_max = 0;
+    for (int q = 0; q < P.nfwd; ++q) dl_max = std::max(dl_max, L.fwd.start[q + 1] - L.fwd.start[q]);
+    for (int q = 0; q < P.nbwd; ++q) dl_max = std::max(dl_max, L.bwd.start[q + 1] - L.bwd.start[q]);
+    P.blocal = dl_max <= BLOCK ? 1 : 0;
+    P.off = L.a.off, P.col = L.a.col, P.val = L.a.val, P.diag = L.diag;
+    P.fo = L.fwd.order, P.fs = L.fwd.d_start, P.bo = L.bwd.order, P.bs = L.bwd.d_start;
+    P.goff = L.groups.off, P.gmem = L.groups.col;
+    P.roff = L.restrict_.off, P.rcol = L.restrict_.col, P.rval = L.restrict_.val;
+    P.poff = L.prolong.off, P.pcol = L.prolong.col, P.pval = L.prolong.val;
+    P.rhs = L.rhs, P.x = L.x, P.res = L.res;
+    P.ioff = L.d_ioff, P.idx = L.d_idx, P.foff = L.d_foff, P.fac = L.d_fac;
+    pl.push_back(P);
+  }
+  PLev* dp = nullptr;
+  if (int e = D.arena.upload(&dp, pl, s)) return e;
+  D.d_plev = dp;
+  // One block per SM: a dependency level fits in one pass and whole-level phases
+  // (residual, transfers) have a few rows per thread.
+  int dev = 0, sms = 0, per = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_plain_coarse, BLOCK, 0) != cudaSuccess || per < 1) {
+    cudaGetLastError();
+    per = 0;
+  }
+  D.coop_blocks = per > 0 ? sms : 0;
+  // A cluster of PC_CLUSTER blocks, when one fits an SM group.
+  {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(PC_CLUSTER, 1, 1);
+    cfg.blockDim = dim3(BLOCK, 1, 1);
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = PC_CLUSTER;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, k_plain_coarse_cluster, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      clusters = 0;
+    }
+    D.cluster = clusters > 0;
+  }
+  CU(cudaStreamSynchronize(s));  // the descriptors' host copy goes out of scope
+  return 0;
+}
+
+// What the sweeps of the levels read beside what every form of them needs (whose end in the arena
+// D.base_ptrs marks): block smoothers' records, the cluster plan of levels 1 .. L-1, whose records
+// stand for the levels' rows, or the rows.
+int plan_levels(DevHierarchy& D, const Hierarchy& H, cudaStream_t s) {
+  for (size_t l = 0; l < D.levels.size(); ++l) {
+    const MgLevel& M = H.levels[l];
+    if (M.lines.empty()) continue;
+    int e = plan_lines(D, D.levels[l], M, M.lines[0], s);  // the reference builds one block group per level
+    if (e == NO_PLAN) e = lean_lines(D, D.levels[l], M, M.lines[0], s);
+    if (e) return e;
+  }
+  if (D.levels.size() < 2 || D.lines) return 0;
+  if (int e = plan_plain_cluster(D, H, s)) return e;
+  if (D.pc_rest > 0) return 0;
+  CU(cudaStreamSynchronize(s));
+  D.arena.rollback(D.base_ptrs, D.base_bytes);  // a plan given up on the way
+  return row_levels(D, H, s);
+}
+
+// The same within the fewest bytes, in place of what plan_levels has allocated.
+int lean_levels(DevHierarchy& D, const Hierarchy& H, cudaStream_t s) {
+  CU(cudaStreamSynchronize(s));
+  D.arena.rollback(D.base_ptrs, D.base_bytes);
+  D.lean = true;
+  D.d_pc = nullptr;
+  D.pc_rest = D.pc_smem = 0;
+  D.pc_chunk.clear();
+  for (size_t l = 0; l < D.levels.size(); ++l)
+    if (!H.levels[l].lines.empty())
+      if (int e = lean_lines(D, D.levels[l], H.levels[l], H.levels[l].lines[0], s)) return e;
+  if (D.levels.size() < 2 || D.lines) return 0;
+  return row_levels(D, H, s);
+}
+
 int build_mg_dev(cfdg_grid* G, const Poller& poll) {
   Hierarchy H;
   if (int e = build_hierarchy(G->h, poll, H)) {
@@ -1747,84 +1891,14 @@ int build_mg_dev(cfdg_grid* G, const Poller& poll) {
       if (int e = D->arena.alloc(&L.x, L.n + (M.lines.empty() ? 0 : 1))) return e;  // + a zero behind the rows
     if (!L.res)
       if (int e = D->arena.alloc(&L.res, L.n)) return e;
-    if (!M.lines.empty()) {
-      // The reference builds one block group per level.
-      if (int e = plan_lines(*D, L, M, M.lines[0], s)) return e;
-    }
   }
   D->level_cells = H.level_cells;
   D->level_nonzeros = H.level_nonzeros;
-  // Levels 1 .. L-1: the cluster plan, whose records stand for the levels' rows, else the rows and sweep orders. A plan that the context's budget has no room for is left out.
-  if (D->levels.size() > 1 && !D->lines) {
-    const size_t held = D->arena.ptrs.size();
-    const uint64_t held_bytes = D->arena.bytes;
-    if (int e = plan_plain_cluster(*D, H, s)) {
-      if (e != CFDG_ERR_ADMISSION) return e;
-      CU(cudaStreamSynchronize(s));
-      D->arena.rollback(held, held_bytes);
-      D->pc_rest = 0;
-    }
-    for (size_t l = 1; D->pc_rest == 0 && l < D->levels.size(); ++l)
-      if (int e = upload_rows(*D, D->levels[l], H.levels[l], true, s)) return e;
-  }
-  // Without it, the levels for the cooperative kernel, when its grid can be co-resident.
-  if (D->levels.size() > 1 && !D->lines && D->pc_rest == 0) {
-    std::vector<PLev> pl;
-    for (size_t l = 1; l < D->levels.size(); ++l) {
-      const DevLevel& L = D->levels[l];
-      PLev P{};
-      P.n = L.n;
-      P.terminal = L.terminal ? 1 : 0;
-      P.ngroups = L.ngroups;
-      P.nblocks = L.nblocks;
-      P.nfwd = (int)L.fwd.start.size() - 1;
-      P.nbwd = (int)L.bwd.start.size() - 1;
-      int dl_max = 0;
-      for (int q = 0; q < P.nfwd; ++q) dl_max = std::max(dl_max, L.fwd.start[q + 1] - L.fwd.start[q]);
-      for (int q = 0; q < P.nbwd; ++q) dl_max = std::max(dl_max, L.bwd.start[q + 1] - L.bwd.start[q]);
-      P.blocal = dl_max <= BLOCK ? 1 : 0;
-      P.off = L.a.off, P.col = L.a.col, P.val = L.a.val, P.diag = L.diag;
-      P.fo = L.fwd.order, P.fs = L.fwd.d_start, P.bo = L.bwd.order, P.bs = L.bwd.d_start;
-      P.goff = L.groups.off, P.gmem = L.groups.col;
-      P.roff = L.restrict_.off, P.rcol = L.restrict_.col, P.rval = L.restrict_.val;
-      P.poff = L.prolong.off, P.pcol = L.prolong.col, P.pval = L.prolong.val;
-      P.rhs = L.rhs, P.x = L.x, P.res = L.res;
-      P.ioff = L.d_ioff, P.idx = L.d_idx, P.foff = L.d_foff, P.fac = L.d_fac;
-      pl.push_back(P);
-    }
-    PLev* dp = nullptr;
-    if (int e = D->arena.upload(&dp, pl, s)) return e;
-    D->d_plev = dp;
-    // One block per SM: a dependency level fits in one pass and whole-level phases
-    // (residual, transfers) have a few rows per thread.
-    int dev = 0, sms = 0, per = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_plain_coarse, BLOCK, 0) != cudaSuccess || per < 1) {
-      cudaGetLastError();
-      per = 0;
-    }
-    D->coop_blocks = per > 0 ? sms : 0;
-    // A cluster of PC_CLUSTER blocks, when one fits an SM group.
-    {
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(PC_CLUSTER, 1, 1);
-      cfg.blockDim = dim3(BLOCK, 1, 1);
-      cudaLaunchAttribute at[1];
-      at[0].id = cudaLaunchAttributeClusterDimension;
-      at[0].val.clusterDim.x = PC_CLUSTER;
-      at[0].val.clusterDim.y = 1;
-      at[0].val.clusterDim.z = 1;
-      cfg.attrs = at;
-      cfg.numAttrs = 1;
-      int clusters = 0;
-      if (cudaOccupancyMaxActiveClusters(&clusters, k_plain_coarse_cluster, &cfg) != cudaSuccess) {
-        cudaGetLastError();
-        clusters = 0;
-      }
-      D->cluster = clusters > 0;
-    }
-  }
+  D->base_ptrs = D->arena.ptrs.size();
+  D->base_bytes = D->arena.bytes;
+  int e = plan_levels(*D, H, s);
+  if (e == CFDG_ERR_ADMISSION) e = lean_levels(*D, H, s);
+  if (e) return e;
   CU(cudaStreamSynchronize(s));
   G->host_mg = std::make_shared<Hierarchy>(std::move(H));
   {

@@ -34,10 +34,16 @@ constexpr int LC_SMEM = 208 * 1024;  // dynamic shared memory a sweep may ask fo
 
 // The banded forward and backward substitutions of one block (multigrid/line.rs:172-185)
 // for a half-bandwidth BW: the last BW results stay in registers and the next row's values are
-// loaded ahead of the chain. Rows before the first and after the last give products of zeros.
-template <int BW>
-__device__ __forceinline__ void line_subst(double* s, const double* f, int len) {
+// loaded ahead of the chain. Rows before the first and after the last give products of zeros; PAD:
+// the factor has BW rows of zeros behind the last one, else they are left out of the loads.
+template <int BW, bool PAD>
+__device__ __forceinline__ void line_subst(double* s, const double* fac, int len) {
   constexpr int W = BW + 1;
+  struct {
+    const double* p;
+    int end;
+    __device__ __forceinline__ double operator[](int k) const { return PAD || k < end ? p[k] : 0.0; }
+  } const f{fac, len * W};
   double w[BW], c[W], n[W];  // w[d]: the result d + 1 rows back (forward) or ahead (backward)
 #pragma unroll
   for (int d = 0; d < BW; ++d) w[d] = 0.0;
@@ -100,12 +106,13 @@ __device__ __noinline__ void line_subst_any(double* s, const double* f, int len,
     s[i] = v * f[i * W];
   }
 }
+template <bool PAD>
 __device__ __forceinline__ void line_solve(double* s, const double* f, int len, int bw) {
   switch (bw) {
-    case 1: line_subst<1>(s, f, len); break;
-    case 2: line_subst<2>(s, f, len); break;
-    case 3: line_subst<3>(s, f, len); break;
-    case 4: line_subst<4>(s, f, len); break;
+    case 1: line_subst<1, PAD>(s, f, len); break;
+    case 2: line_subst<2, PAD>(s, f, len); break;
+    case 3: line_subst<3, PAD>(s, f, len); break;
+    case 4: line_subst<4, PAD>(s, f, len); break;
     default: line_subst_any(s, f, len, bw); break;
   }
 }
@@ -224,7 +231,7 @@ __global__ void __launch_bounds__(LCT, 1) k_line_sweep(LineLev L, const Scalars*
         if (ib < len) s[ib] = vb;
       }
       __syncwarp();
-      if (lane == 0) line_solve(s, reinterpret_cast<const double*>(rec + 16), len, L.bw);
+      if (lane == 0) line_solve<true>(s, reinterpret_cast<const double*>(rec + 16), len, L.bw);
       __syncwarp();
       if (!SHX) {
         for (int i = lane; i < len; i += 32) L.x[rows[i]] = s[i];
@@ -247,6 +254,41 @@ __global__ void __launch_bounds__(LCT, 1) k_line_sweep(LineLev L, const Scalars*
       const int* rows = rows_of(rank + q * L.nb);
       for (int i = lane; i < len; i += 32) L.x[rows[i]] = xs[q * len + i];
     }
+}
+
+// One sweep without records, for grids that their context has room for only so, and for levels
+// beyond what a record describes: the block smoother's arrays as the host holds them, the iterate
+// in global memory, a block's rows summed by the lanes one entry after the other. In the same order,
+// so the same bits. The cycle of 48^3 cells, thickness 0.1: 9.3 ms in 112.0 MB with records, 13.7 ms
+// in 101.5 MB without; 470 x 460 x 2 and other blocks of a row or two about half as fast.
+template <bool BWD>
+__global__ void __launch_bounds__(LCT, 1) k_line_sweep_lean(LineLean L, const Scalars* S) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  if (S && S->done) return;  // the whole cluster
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, len = L.len;
+  const int first = (int)cg::this_cluster().block_rank() + L.nb * warp;
+  for (int d = 0; d < L.ndep; ++d) {
+    const int q = BWD ? L.ndep - 1 - d : d, hi = __ldg(&L.start[q + 1]);
+    for (int t = __ldg(&L.start[q]) + first; t < hi; t += L.nb * LCW) {
+      const long long at = (long long)__ldg(&L.order[t]) * len;
+      double* s = L.scr ? L.scr + at : reinterpret_cast<double*>(smem) + (size_t)warp * len;
+      for (int i = lane; i < len; i += 32) {
+        double v = __ldcg(&L.rhs[__ldg(&L.nodes[at + i])]);
+        const int end = __ldg(&L.off[at + i + 1]);
+#pragma unroll 4
+        for (int e = __ldg(&L.off[at + i]); e < end; ++e) v = v - __ldg(&L.val[e]) * __ldcg(&L.x[__ldg(&L.col[e])]);
+        s[i] = v;
+      }
+      __syncwarp();
+      if (lane == 0) line_solve<false>(s, L.fac + at * (L.bw + 1), len, L.bw);
+      __syncwarp();
+      for (int i = lane; i < len; i += 32) L.x[__ldg(&L.nodes[at + i])] = s[i];
+      __syncwarp();  // the row is reused by the warp's next block
+    }
+    __threadfence();
+    pc_arrive();
+    pc_wait();
+  }
 }
 
 using LineKernel = void (*)(LineLev, const Scalars*);

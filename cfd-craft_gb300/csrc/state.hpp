@@ -147,6 +147,16 @@ struct LineLev {
   double *x, *scr;
 };
 
+// The same block smoother in the fewest bytes (k_line_sweep_lean): the host's arrays as they are.
+struct LineLean {
+  int len, bw, ndep, nb;              // rows per block, half-bandwidth, dependency levels, cluster size
+  const int *nodes, *off, *col;       // a block's rows, their outside entries
+  const double *val, *fac;            // the entries' values, the factor
+  const int *order, *start;           // blocks by dependency level, [ndep + 1]
+  const double* rhs;
+  double *x, *scr;                    // scr: [rows] by block, where a block's rows don't fit the shared memory
+};
+
 struct DevLevel {
   int n = 0;
   DevCsr a;
@@ -165,12 +175,14 @@ struct DevLevel {
   long long* d_foff = nullptr;
   double* d_fac = nullptr;
   double *rhs = nullptr, *x = nullptr, *res = nullptr;
-  // Anisotropic levels: the block smoother, whether its iterate lives in the cluster's shared
-  // memory, the dynamic shared memory of a sweep and the device bytes held.
-  bool lines = false, lshx = false;
+  // Anisotropic levels: the block smoother (lean: le instead of ll's records), whether its iterate
+  // lives in the cluster's shared memory, the dynamic shared memory of a sweep and the device bytes
+  // held.
+  bool lines = false, lean = false, lshx = false;
   int lsmem = 0;
   uint64_t lbytes = 0;
   LineLev ll{};
+  LineLean le{};
 };
 
 struct DevHierarchy {
@@ -194,6 +206,11 @@ struct DevHierarchy {
   int pc_rest = 0, pc_smem = 0;
   std::vector<int> pc_chunk;  // rows per block of levels 1 .. pc_rest - 1
   bool lines = false;  // block-smoothed (anisotropic): level by level, sweeps on a cluster
+  // Where the arena ends without the plan, the records or the rows of the sweeps; lean: these were
+  // built for the fewest bytes.
+  size_t base_ptrs = 0;
+  uint64_t base_bytes = 0;
+  bool lean = false;
 };
 
 // A launch whose blocks may be scheduled while the kernel before it is still running: every

@@ -46,3 +46,45 @@ def test_plain_form_within_the_bytes(pkg, name):
         dg.close()
         ctx.close()
     assert np.array_equal(bits(out[0]), bits(out[1]))
+
+
+THIN = {  # cells, size, boundaries, bytes
+    "lines": ((48, 48, 48), (1.0, 1.0, 0.1), ("open", "wall", "wall"), 105091160),
+    "folded lines, closed": ((48, 48, 48), (1.0, 1.0, 0.1), ("wall", "periodic", "wall"), 106928508),
+    "long lines": ((9, 7, 100), (9.0, 7.0, 2.0), ("open", "wall", "wall"), 5974167),
+    "many lines": ((70, 72, 5), (70.0, 72.0, 0.5), ("open", "wall", "wall"), 24348898),
+    "records not copied ahead": ((5, 5, 400), (5.0, 5.0, 8.0), ("open", "wall", "wall"), 9323877),
+    "planes": ((24, 4, 4), (240.0, 4.0, 4.0), ("open", "wall", "wall"), 259812),
+    "single rows": ((40, 30, 1), (40.0, 30.0, 0.05), ("open", "wall", "wall"), 850766),
+    "lines beyond the shared memory": ((3, 3, 7000), (3.0, 3.0, 35.0), ("open", "wall", "wall"), 55920741),
+}
+
+
+@pytest.mark.parametrize("name", list(THIN))
+def test_anisotropic_grids_within_the_bytes(pkg, name):
+    cells, size, boundaries, held = THIN[name]
+    case = pkg.synth.case(cells, 1.0, boundaries=boundaries, inflow=1.0 if boundaries[0] == "open" else 0.0,
+                          preconditioner="multigrid")
+    case["domain"]["size_m"] = list(size)
+    g = pkg.grid.Grid.build(case)
+    r = np.random.default_rng(3).uniform(-1.0, 1.0, g.count)
+    out = []
+    for budget in (1 << 36, held):
+        ctx = pkg.pressure.Context(0, hbm_budget_bytes=budget)
+        dg = pkg.pressure.DeviceGrid(g, ctx=ctx, preconditioner="multigrid")
+        out.append([dg.precondition(r) for _ in range(2)])
+        dg.close()
+        ctx.close()
+    assert np.array_equal(bits(out[0]), bits(out[1]))
+
+
+def test_more_dependency_levels_than_shared_memory_holds(pkg, O):
+    """A duct of 60,000 cells: more dependency levels of its lines than a record sweep keeps starts of."""
+    case = pkg.synth.case((60000, 2, 2), 1.0, boundaries=("open", "wall", "wall"), inflow=1.0, preconditioner="multigrid")
+    case["domain"]["size_m"] = [60000.0, 2.0, 0.2]
+    g = pkg.grid.Grid.build(case)
+    r = np.random.default_rng(3).uniform(-1.0, 1.0, g.count)
+    oz, _ = O.Grid(case).mg_apply(r)
+    dg = pkg.pressure.DeviceGrid(g, preconditioner="multigrid")
+    assert np.array_equal(bits(dg.precondition(r)), bits(oz))
+    dg.close()
