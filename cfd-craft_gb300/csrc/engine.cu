@@ -1811,7 +1811,6 @@ int plan_levels(DevHierarchy& D, const Hierarchy& H, cudaStream_t s) {
 int lean_levels(DevHierarchy& D, const Hierarchy& H, cudaStream_t s) {
   CU(cudaStreamSynchronize(s));
   D.arena.rollback(D.base_ptrs, D.base_bytes);
-  D.lean = true;
   D.d_pc = nullptr;
   D.pc_rest = D.pc_smem = 0;
   D.pc_chunk.clear();
@@ -1896,9 +1895,6 @@ int build_mg_dev(cfdg_grid* G, const Poller& poll) {
   D->level_nonzeros = H.level_nonzeros;
   D->base_ptrs = D->arena.ptrs.size();
   D->base_bytes = D->arena.bytes;
-  int e = plan_levels(*D, H, s);
-  if (e == CFDG_ERR_ADMISSION) e = lean_levels(*D, H, s);
-  if (e) return e;
   CU(cudaStreamSynchronize(s));
   G->host_mg = std::make_shared<Hierarchy>(std::move(H));
   {
@@ -1952,9 +1948,37 @@ int prepare_mg_impl(cfdg_grid* G, const Poller& poll, cfdg_info* info) {
   return 0;
 }
 
+// What only the sweeps of the plain form's cycle read, on its first use: mixed solves, which take
+// nothing but level 0's diagonal from this hierarchy, find its bytes free for their own levels.
+int ensure_sweeps(cfdg_grid* G, cfdg_info* info) {
+  DevHierarchy& D = *G->mg;
+  if (!D.ready) {
+    const auto t0 = std::chrono::steady_clock::now();
+    cudaStream_t s = G->stream;
+    for (DevLevel& L : D.levels) L.lean = false;
+    int e = plan_levels(D, *G->host_mg, s);
+    if (e == CFDG_ERR_ADMISSION) e = lean_levels(D, *G->host_mg, s);
+    const cudaError_t c = cudaStreamSynchronize(s);
+    if (!e && c != cudaSuccess) e = fail(CFDG_ERR_CUDA, cudaGetErrorString(c));
+    if (e) {
+      D.arena.rollback(D.base_ptrs, D.base_bytes);
+      return e;
+    }
+    D.ready = true;
+    std::lock_guard<std::mutex> lk(G->stats_mu);
+    G->stats_json = stats_json_of(D, *G->host_mg);
+    if (info) info->multigrid_setup_seconds += seconds_since(t0);
+  }
+  if (info) info->hierarchy_bytes = D.arena.bytes;
+  return 0;
+}
+
 // pressure.rs:55-97: the cached factor, or the hierarchy checked against its signature.
 int prepare_preconditioner(cfdg_grid* G, const Poller& poll, cfdg_info* info) {
-  if (G->preconditioner == CFDG_PRECOND_MULTIGRID) return prepare_mg_impl(G, poll, info);
+  if (G->preconditioner == CFDG_PRECOND_MULTIGRID) {
+    if (int e = prepare_mg_impl(G, poll, info)) return e;
+    return ensure_sweeps(G, info);
+  }
   if (!G->ic0) {
     reset_chunk(G);
     const auto t0 = std::chrono::steady_clock::now();

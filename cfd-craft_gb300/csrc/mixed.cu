@@ -112,11 +112,11 @@ struct FineCase {
   int bin1, nbh1, h1, pad_bin1;
   int nb1[3], pad_nb1;
   const int *goff, *gmem;
-  // transfers level 0 <-> 1
+  // transfers level 0 <-> 1 (null where bin1 gives them)
   int n1;
   const int *r_off, *r_child;  // level-1 rows gather level-0 children
   const float* r_w;
-  const int *p_off, *p_col;    // level-0 rows (full layout) from level-1
+  const int *p_off, *p_col;    // level-0 rows (full layout) from level-1, where it isn't by injection
   const float* p_w;
   const int* pinj;             // injection prolongation (aggregation): level-1 parent per slot, -1 none
   float pscale;                // the coarse-correction scale of the injection path
@@ -143,7 +143,7 @@ struct CLev {
   int jacobi, res0;
   const float* il1;  // l1-Jacobi: 1 / (diag + sum |a_ij|), 0 where diag is 0
   float* x2;         // l1-Jacobi: the second iterate of a sweep pair
-  const int *off, *col;
+  const int *off, *col;  // the rows, for the residual of levels without res0 (null elsewhere)
   const float *val, *diag;
   const int* coff;  // colour c owns rows coff[c] .. coff[c+1]-1
   const int *ell_off, *ell_w;  // per colour: start of its ELL block and its width
@@ -2511,6 +2511,14 @@ std::vector<float> to_f32(const std::vector<T>& v) {
   return std::vector<float>(v.begin(), v.end());
 }
 
+// A bin level of the hierarchy for plan_cluster: its bins per axis and the types of its rows
+// (coarse_cluster.cuh ClRow), one per row of the bin layout.
+struct BinMatrix {
+  int nb[3] = {0, 0, 0}, nbh = 0, h = 0;
+  std::vector<uint16_t> type;                  // [2h]
+  std::vector<std::array<uint32_t, 12>> tab;
+};
+
 struct CaseState {
   cfdg_grid* G = nullptr;
   uint64_t version = 0;  // the grid's faces_version this state was built from
@@ -2518,9 +2526,15 @@ struct CaseState {
   FineCase F{};
   CCase C{};
   // on: the coarse levels from cl.lc run on a cluster of their own, those above grid-wide (over
-  // their row types, where all are bin levels: up).
+  // their row types, where all are bin levels: up). The row types (bins, by level) go to the
+  // device with the first batch that has room for them (upload_plan), last in the arena.
   ClCase cl{};
   ClUp up{};
+  std::vector<BinMatrix> bins;
+  std::mutex plan_mu;
+  bool plan_ready = false;
+  size_t plan_ptrs = 0;  // the arena without them
+  uint64_t plan_bytes = 0;
   std::vector<std::vector<int32_t>> colors;  // per coarse level: colour offsets (host copy)
   struct LevelStats {
     long long rows, nnz, ell, groups, blocks;
@@ -2602,13 +2616,6 @@ bool encode_split(CUtensorMap& m, const void* base, bool u16, int nxh, int rows,
              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// A bin level of the hierarchy for plan_cluster: its bins per axis and the types of its rows
-// (coarse_cluster.cuh ClRow), one per row of the bin layout.
-struct BinMatrix {
-  int nb[3] = {0, 0, 0}, nbh = 0, h = 0;
-  std::vector<uint16_t> type;                  // [2h]
-  std::vector<std::array<uint32_t, 12>> tab;
-};
 constexpr int CL_TYPES = 2048;  // more types than this: the level is not planned as a bin level
 
 ClBin bin_shape(const BinMatrix& M, const CLev& L) {
@@ -2631,20 +2638,20 @@ int upload_types(Arena& A, cudaStream_t s, const BinMatrix& M, ClBin& B) {
 }
 
 // Plans k_coarse_cluster for a case whose coarse levels allow it (aggregation levels of at
-// most two colours without closed groups) and uploads what it needs; bins[l] holds the bin
-// levels among levels 1.. (h == 0: not a bin level). Levels are split over the cluster's
+// most two colours without closed groups), but for the row types on the device (upload_plan);
+// bins[l] holds the bin levels among levels 1.. (h == 0: not a bin level). Levels are split over the cluster's
 // blocks while their layers fill at least three quarters of them and a split phase beats one
 // block's (about 1,200 rows), or while one block would be slow (above 2,500 rows); levels
 // without a bin layout are split above 1,500 rows. The cluster starts at the first level
 // whose slabs fit the blocks' registers and shared memory; a level split by rows is taken up
 // to 32,768 of them (four a thread).
 // Where the levels above are bin levels, too, U describes them.
-int plan_cluster(Arena& A, cudaStream_t s, const CCase& C, const std::vector<int>& jacobi, const std::vector<BinMatrix>& bins,
-                 float alpha, ClCase& K, ClUp& U) {
+void plan_cluster(const CCase& C, const std::vector<int>& jacobi, const std::vector<BinMatrix>& bins, float alpha,
+                  ClCase& K, ClUp& U) {
   K = ClCase{};
   U = ClUp{};
   for (int l = 1; l <= C.nl; ++l)
-    if (C.lv[l - 1].ngroups || jacobi[l] || C.lv[l - 1].ncolors > 2) return 0;
+    if (C.lv[l - 1].ngroups || jacobi[l] || C.lv[l - 1].ncolors > 2) return;
   for (int lc = 1; lc <= C.nl; ++lc) {
     ClCase T{};
     T.lc = lc - 1;
@@ -2696,25 +2703,44 @@ int plan_cluster(Arena& A, cudaStream_t s, const CCase& C, const std::vector<int
     if (!ok || at > (size_t)CL_SMEM) continue;
     T.smem = (int)at;
     T.on = 1;
-    for (int t = 0; t < T.nb; ++t)
-      if (int e = upload_types(A, s, bins[lc + t], T.b[t])) return e;
     bool up = T.lc > 0 && T.lc <= CLUP && T.nb > 0;
     for (int l = 1; l < lc; ++l)
       up = up && bins[l].h > 0 && (uint64_t)bins[l].h * bins[l].nbh < ((uint64_t)1 << 32);  // cl_div
     if (up) {
       U.n = T.lc;
       U.alpha = alpha;
-      for (int l = 1; l < lc; ++l) {
-        U.lv[l - 1] = bin_shape(bins[l], C.lv[l - 1]);
-        if (int e = upload_types(A, s, bins[l], U.lv[l - 1])) return e;
-      }
+      for (int l = 1; l < lc; ++l) U.lv[l - 1] = bin_shape(bins[l], C.lv[l - 1]);
       U.lv[T.lc] = T.b[0];
       for (int l = 0; l <= T.lc; ++l) U.rhs[l] = C.lv[l].rhs;
     }
     K = T;
-    return 0;
+    return;
   }
-  return 0;
+}
+
+// The row types of a case's plan to the device, once; CFDG_ERR_ADMISSION where the context's
+// budget has no room for them. *now: done by this call.
+int upload_plan(CaseState& K, cudaStream_t s, bool* now) {
+  std::lock_guard<std::mutex> lk(K.plan_mu);
+  *now = false;
+  if (K.plan_ready) return 0;
+  K.plan_ptrs = K.arena.ptrs.size();
+  K.plan_bytes = K.arena.bytes;
+  int e = 0;
+  for (int t = 0; t < K.cl.nb && !e; ++t) e = upload_types(K.arena, s, K.bins[K.cl.lc + 1 + t], K.cl.b[t]);
+  for (int l = 0; l < K.up.n && !e; ++l) e = upload_types(K.arena, s, K.bins[l + 1], K.up.lv[l]);
+  if (K.up.n) K.up.lv[K.up.n] = K.cl.b[0];
+  const cudaError_t c = cudaStreamSynchronize(s);
+  if (!e && c != cudaSuccess) e = fail(CFDG_ERR_CUDA, cudaGetErrorString(c));
+  if (e) K.arena.rollback(K.plan_ptrs, K.plan_bytes);
+  *now = K.plan_ready = e == 0;
+  return e;
+}
+// Takes back what an upload_plan of the same caller put there.
+void drop_plan(CaseState& K) {
+  std::lock_guard<std::mutex> lk(K.plan_mu);
+  K.arena.rollback(K.plan_ptrs, K.plan_bytes);
+  K.plan_ready = false;
 }
 
 // Builds the FP32 device copy of a grid's hierarchy for the mixed form (cached on the grid).
@@ -3034,7 +3060,7 @@ int build_case(cfdg_grid* G, CaseState& cs) {
     }
     F.pscale = alpha;
     for (auto& w : pw32) w *= alpha;
-    if (inj) {
+    if (inj && !F.bin1) {
       std::vector<int32_t> par(F.N2, -1);
       for (int sl = 0; sl < F.N2; ++sl)
         if (poff[sl + 1] > poff[sl]) par[sl] = pcol[poff[sl]];
@@ -3042,15 +3068,22 @@ int build_case(cfdg_grid* G, CaseState& cs) {
       if (int e = A.upload(&pp, par, s)) return e;
       F.pinj = pp;
     }
-    int *o, *c, *po, *pc;
-    float *w, *pw;
-    if (int e = A.upload(&o, R0.off, s)) return e;
-    if (int e = A.upload(&c, child, s)) return e;
-    if (int e = A.upload(&w, to_f32(R0.val), s)) return e;
-    if (int e = A.upload(&po, poff, s)) return e;
-    if (int e = A.upload(&pc, pcol, s)) return e;
-    if (int e = A.upload(&pw, pw32, s)) return e;
-    F.r_off = o, F.r_child = c, F.r_w = w, F.p_off = po, F.p_col = pc, F.p_w = pw;
+    if (!F.bin1) {
+      int *o, *c;
+      float* w;
+      if (int e = A.upload(&o, R0.off, s)) return e;
+      if (int e = A.upload(&c, child, s)) return e;
+      if (int e = A.upload(&w, to_f32(R0.val), s)) return e;
+      F.r_off = o, F.r_child = c, F.r_w = w;
+    }
+    if (!inj) {
+      int *po, *pc;
+      float* pw;
+      if (int e = A.upload(&po, poff, s)) return e;
+      if (int e = A.upload(&pc, pcol, s)) return e;
+      if (int e = A.upload(&pw, pw32, s)) return e;
+      F.p_off = po, F.p_col = pc, F.p_w = pw;
+    }
   }
   int maxg = 1;
   for (int l = 1; l <= C.nl; ++l) {
@@ -3060,19 +3093,24 @@ int build_case(cfdg_grid* G, CaseState& cs) {
     L.terminal = l == C.nl;
     L.ngroups = M.groups.rows();
     maxg = std::max(maxg, L.ngroups);
-    int *o, *c;
-    float *v, *d;
-    if (int e = A.upload(&o, M.a.off, s)) return e;
-    if (int e = A.upload(&c, M.a.col, s)) return e;
-    if (int e = A.upload(&v, to_f32(M.a.val), s)) return e;
-    if (int e = A.upload(&d, to_f32(M.diag), s)) return e;
-    L.off = o, L.col = c, L.val = v, L.diag = d;
     std::vector<int32_t> coff = lcoff[l], rows(M.n);
     for (int i = 0; i < M.n; ++i) rows[i] = i;  // colour c owns rows coff[c] .. coff[c+1]-1
     L.ncolors = lcolors[l];
     // A level whose graph needs many colours (the wide stencils of linear-interpolation
     // coarse operators) is smoothed by l1-Jacobi instead: one phase per sweep.
     L.jacobi = ljacobi[l];
+    L.res0 = !L.terminal && !L.jacobi && L.ncolors == 2 && L.ngroups == 0 ? 1 : 0;
+    float* d;
+    if (int e = A.upload(&d, to_f32(M.diag), s)) return e;
+    L.diag = d;
+    if (!L.terminal && !L.res0) {
+      int *o, *c;
+      float* v;
+      if (int e = A.upload(&o, M.a.off, s)) return e;
+      if (int e = A.upload(&c, M.a.col, s)) return e;
+      if (int e = A.upload(&v, to_f32(M.a.val), s)) return e;
+      L.off = o, L.col = c, L.val = v;
+    }
     if (L.jacobi) {
       std::vector<float> il1(M.n, 0.0f);
       for (int i = 0; i < M.n; ++i) {
@@ -3189,7 +3227,6 @@ int build_case(cfdg_grid* G, CaseState& cs) {
     CU(cudaMemsetAsync(x, 0, sizeof(float) * L.n, s));
     CU(cudaMemsetAsync(res, 0, sizeof(float) * L.n, s));  // colour-1 rows of res0 levels stay zero
     L.rhs = rhs, L.x = x, L.res = res;
-    L.res0 = !L.terminal && !L.jacobi && L.ncolors == 2 && L.ngroups == 0 ? 1 : 0;
     if (L.terminal) {
       L.nblocks = M.direct_idx.rows();
       int *io, *ix;
@@ -3324,7 +3361,8 @@ int build_case(cfdg_grid* G, CaseState& cs) {
       for (int a = 0; a < 3; ++a) M.nb[a] = B.nb[a];
       M.nbh = B.nbh, M.h = B.h;
     }
-    if (int e = plan_cluster(A, s, C, ljacobi, bins, alpha, cs.cl, cs.up)) return e;
+    plan_cluster(C, ljacobi, bins, alpha, cs.cl, cs.up);
+    if (cs.cl.on) cs.bins = std::move(bins);
   }
   F.n1 = C.lv[0].n;
   F.rhs1 = C.lv[0].rhs;
@@ -3859,6 +3897,73 @@ void fill_info(const MState& m, cfdg_info& I) {
   I.refinement_steps = (uint64_t)m.outer;
 }
 
+// Decides which cases of the batch run their coarse levels on clusters (with `plans`, else none)
+// and allocates the descriptors of the launches.
+// `fresh`: the cases whose row types it has put on the device.
+int choose_clusters(cfdg_batch* B, bool plans, std::vector<CaseState*>& fresh, cudaStream_t s) {
+  const int nc = (int)B->cases.size();
+  Arena& A = B->arena;
+  std::vector<ClCase>& cl = B->plan;
+  std::vector<ClUp>& up = B->ups;
+  B->cl_smem = 0;
+  cl.assign(nc, ClCase{});
+  up.assign(nc, ClUp{});
+  for (int i = 0; i < nc; ++i) {
+    CaseState& K = *B->cases[i];
+    if (!plans || !K.cl.on || (K.cl.lc > 0 && K.up.n == 0 && !B->coop)) continue;
+    bool now = false;
+    if (int e = upload_plan(K, s, &now)) {
+      if (e != CFDG_ERR_ADMISSION) return e;
+      continue;
+    }
+    if (now) fresh.push_back(&K);
+    cl[i] = K.cl, up[i] = K.up;
+    B->cl_smem = std::max(B->cl_smem, cl[i].smem);
+  }
+  int clusters = 0;
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute at[2];
+  cluster_config(cfg, at, 1, CLS, CLT, B->cl_smem, s);
+  cfg.numAttrs = 1;
+  if (cudaFuncSetAttribute(k_coarse_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+      cudaFuncSetAttribute(k_coarse_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, CL_SMEM) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&clusters, k_coarse_cluster, &cfg) != cudaSuccess || clusters < 1) {
+    cudaGetLastError();
+    cl.assign(nc, ClCase{});
+    up.assign(nc, ClUp{});
+  }
+  B->any_cl = B->any_tab[0] = B->any_tab[1] = false;
+  B->up_levels = 0;
+  std::fill(B->up_h, B->up_h + CLUP, 0);
+  std::fill(B->up_next, B->up_next + CLUP, 0);
+  for (int i = 0; i < nc; ++i) {
+    B->any_cl |= cl[i].on != 0;
+    B->any_tab[0] |= !cl[i].on;
+    B->any_tab[1] |= cl[i].on && cl[i].lc > 0 && up[i].n == 0;
+    B->up_levels = std::max(B->up_levels, up[i].n);
+    for (int l = 0; l < up[i].n; ++l) {
+      B->up_h[l] = std::max(B->up_h[l], up[i].lv[l].h);
+      B->up_next[l] = std::max(B->up_next[l], up[i].lv[l + 1].h);
+    }
+  }
+  B->d_cl = nullptr;
+  B->d_up = nullptr;
+  // Allocated before the first copy: what a refusal takes back has none in flight.
+  if (B->any_cl)
+    if (int e = A.alloc(&B->d_cl, nc)) return e;
+  if (B->up_levels)
+    if (int e = A.alloc(&B->d_up, nc)) return e;
+  for (int which = 0; which < 2; ++which) {
+    if (!B->any_tab[which]) continue;
+    if (int e = A.alloc(&B->tab_buf[which], (size_t)B->nlev_all * (nc + 1) * (6 + 2 * MAXC) + 1)) return e;
+    if (int e = A.alloc(&B->d_tab[which], 1)) return e;
+  }
+  if (B->any_cl) CU(cudaMemcpyAsync(B->d_cl, cl.data(), nc * sizeof(ClCase), cudaMemcpyHostToDevice, s));
+  if (B->up_levels) CU(cudaMemcpyAsync(B->d_up, up.data(), nc * sizeof(ClUp), cudaMemcpyHostToDevice, s));
+  CU(cudaStreamSynchronize(s));
+  return 0;
+}
+
 }  // namespace
 
 // (Re)packs a batch's device tables after its cases are known.
@@ -3990,52 +4095,20 @@ int cfdg_mixed_pack(cfdg_batch* B) {
     B->coop_blocks = sms * std::max(1, std::min(per, 4));
   }
   // Which cases run their coarse levels on clusters: all that have a plan, when such a cluster
-  // fits the device (and, for those with levels above it, the cooperative launch).
+  // fits the device (and, for those with levels above it, the cooperative launch) and the
+  // context's budget has room for its row types, after everything else; none of them where the
+  // launches' descriptors don't fit.
   {
-    std::vector<ClCase>& cl = B->plan;
-    std::vector<ClUp>& up = B->ups;
-    B->cl_smem = 0;
-    cl.assign(nc, ClCase{});
-    up.assign(nc, ClUp{});
-    for (int i = 0; i < nc; ++i) {
-      const CaseState& K = *B->cases[i];
-      if (K.cl.on && (K.cl.lc == 0 || K.up.n > 0 || B->coop)) cl[i] = K.cl, up[i] = K.up;
-      B->cl_smem = std::max(B->cl_smem, cl[i].smem);
+    const size_t held = A.ptrs.size();
+    const uint64_t held_bytes = A.bytes;
+    std::vector<CaseState*> fresh;
+    int e = choose_clusters(B, true, fresh, s);
+    if (e == CFDG_ERR_ADMISSION && B->any_cl) {
+      A.rollback(held, held_bytes);
+      for (CaseState* K : fresh) drop_plan(*K);
+      e = choose_clusters(B, false, fresh, s);
     }
-    int clusters = 0;
-    cudaLaunchConfig_t cfg;
-    cudaLaunchAttribute at[2];
-    cluster_config(cfg, at, 1, CLS, CLT, B->cl_smem, s);
-    cfg.numAttrs = 1;
-    if (cudaFuncSetAttribute(k_coarse_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-        cudaFuncSetAttribute(k_coarse_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, CL_SMEM) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&clusters, k_coarse_cluster, &cfg) != cudaSuccess || clusters < 1) {
-      cudaGetLastError();
-      cl.assign(nc, ClCase{});
-      up.assign(nc, ClUp{});
-    }
-    B->any_cl = B->any_tab[0] = B->any_tab[1] = false;
-    B->up_levels = 0;
-    std::fill(B->up_h, B->up_h + CLUP, 0);
-    std::fill(B->up_next, B->up_next + CLUP, 0);
-    for (int i = 0; i < nc; ++i) {
-      B->any_cl |= cl[i].on != 0;
-      B->any_tab[0] |= !cl[i].on;
-      B->any_tab[1] |= cl[i].on && cl[i].lc > 0 && up[i].n == 0;
-      B->up_levels = std::max(B->up_levels, up[i].n);
-      for (int l = 0; l < up[i].n; ++l) {
-        B->up_h[l] = std::max(B->up_h[l], up[i].lv[l].h);
-        B->up_next[l] = std::max(B->up_next[l], up[i].lv[l + 1].h);
-      }
-    }
-    if (int e = A.upload(&B->d_up, up, s)) return e;
-    if (int e = A.upload(&B->d_cl, cl, s)) return e;
-    CU(cudaStreamSynchronize(s));
-  }
-  for (int which = 0; which < 2; ++which) {
-    if (!B->any_tab[which]) continue;
-    if (int e = A.alloc(&B->tab_buf[which], (size_t)B->nlev_all * (nc + 1) * (6 + 2 * MAXC) + 1)) return e;
-    if (int e = A.alloc(&B->d_tab[which], 1)) return e;
+    if (e) return e;
   }
   B->active.assign(nc, 1);
   if (int e = set_active(B, s)) return e;

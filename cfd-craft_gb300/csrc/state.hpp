@@ -206,11 +206,11 @@ struct DevHierarchy {
   int pc_rest = 0, pc_smem = 0;
   std::vector<int> pc_chunk;  // rows per block of levels 1 .. pc_rest - 1
   bool lines = false;  // block-smoothed (anisotropic): level by level, sweeps on a cluster
-  // Where the arena ends without the plan, the records or the rows of the sweeps; lean: these were
-  // built for the fewest bytes.
+  // Where the arena ends without the plan, the records or the rows of the sweeps; ready: it holds
+  // them.
   size_t base_ptrs = 0;
   uint64_t base_bytes = 0;
-  bool lean = false;
+  bool ready = false;
 };
 
 // A launch whose blocks may be scheduled while the kernel before it is still running: every

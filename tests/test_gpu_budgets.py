@@ -13,8 +13,8 @@ def bits(a):
     return np.ascontiguousarray(a, np.float64).view(np.uint64)
 
 
-def iso(pkg, n, dx=2.0, nb=0, boundaries=("open", "slip", "slip"), inflow=5.0):
-    boxes = pkg.synth.random_boxes(np.random.default_rng(1), nb, [dx * v for v in n], side=(3 * dx, 8 * dx), dx=dx)
+def iso(pkg, n, dx=2.0, nb=0, boundaries=("open", "slip", "slip"), inflow=5.0, boxes=()):
+    boxes = boxes or pkg.synth.random_boxes(np.random.default_rng(1), nb, [dx * v for v in n], side=(3 * dx, 8 * dx), dx=dx)
     return pkg.synth.case(n, dx, boundaries=boundaries, inflow=inflow, preconditioner="multigrid", boxes=boxes)
 
 
@@ -88,3 +88,70 @@ def test_more_dependency_levels_than_shared_memory_holds(pkg, O):
     dg = pkg.pressure.DeviceGrid(g, preconditioner="multigrid")
     assert np.array_equal(bits(dg.precondition(r)), bits(oz))
     dg.close()
+
+
+MIXED = {  # cases of a batch, bytes
+    "smallest": ([dict(n=(4, 4, 4))], 45100),
+    "small": ([dict(n=(8, 8, 8))], 284888),
+    "odd rows": ([dict(n=(9, 7, 8))], 299703),
+    "no solid cell": ([dict(n=(60, 44, 24))], 40386560),
+    "mostly solid": ([dict(n=(45, 39, 21), boxes=[((8.0, 0.0, 0.0), (90.0, 70.0, 42.0))])], 11026432),
+    "buildings": ([dict(n=(37, 29, 33), dx=1.5, nb=3)], 12873728),
+    "closed": ([dict(n=(64, 48, 32), boundaries=WALLS, inflow=0.0, nb=3)], 37371904),
+    "five smallest": ([dict(n=(4, 4, 4))] * 5, 223148),
+    "two without solid cells": ([dict(n=(40, 44, 24)), dict(n=(33, 30, 17))], 37535744),
+}
+
+
+def mixed(pkg, grids, budget):
+    """Projections of the grids alone, or of several in a batch; also what ran the coarse levels."""
+    us = [pkg.synth.random_velocity(g, 70 + i) for i, g in enumerate(grids)]
+    ps = [np.zeros(g.count) for g in grids]
+    ctx = pkg.pressure.Context(0, hbm_budget_bytes=budget)
+    dgs, batch = [], None
+    try:
+        for g in grids:
+            dgs.append(pkg.pressure.DeviceGrid(g, ctx=ctx, preconditioner="multigrid", precision="mixed"))
+        batch = pkg.pressure.Batch(dgs, ctx=ctx)
+        kernel = batch.stats()["coarse_kernel"]
+        if len(dgs) > 1:
+            assert all(code == 0 for code, _ in batch.project(us, ps, [0.1] * len(grids), 1e-8, 10000))
+        else:
+            batch.close()
+            batch = None
+            dgs[0].project(us[0], ps[0], 0.1, 1e-8, 10000)
+    finally:
+        if batch:
+            batch.close()
+        for d in dgs:
+            d.close()
+        ctx.close()
+    return [bits(a) for a in us + ps], kernel
+
+
+@pytest.mark.parametrize("name", list(MIXED))
+def test_mixed_form_within_the_bytes(pkg, name):
+    cases, held = MIXED[name]
+    grids = [pkg.grid.Grid.build(iso(pkg, **kw)) for kw in cases]
+    ample, _ = mixed(pkg, grids, 1 << 36)
+    least, _ = mixed(pkg, grids, held)
+    assert all(np.array_equal(a, b) for a, b in zip(ample, least))
+
+
+def test_mixed_form_without_its_plans(pkg):
+    """Budgets from ample down to the least that admits the grid: some without room for the cluster's plan."""
+    grids = [pkg.grid.Grid.build(iso(pkg, n=(37, 29, 33), dx=1.5, nb=3))]
+    ample, kernel = mixed(pkg, grids, 1 << 36)
+    lo, hi, seen = 0, 1 << 24, {kernel}
+    while hi - lo > 1 << 8:
+        mid = (lo + hi) // 2
+        try:
+            out, kernel = mixed(pkg, grids, mid)
+        except pkg.pressure.PressureError as e:
+            assert "budget" in str(e)
+            lo = mid
+            continue
+        assert all(np.array_equal(a, b) for a, b in zip(ample, out))
+        seen.add(kernel)
+        hi = mid
+    assert seen == {"cluster", "cooperative"}
