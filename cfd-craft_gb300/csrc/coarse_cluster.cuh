@@ -44,7 +44,7 @@ constexpr int CL_SMEM = 224 * 1024;  // dynamic shared memory a case may ask for
 // memory, in bytes, the same in every block of the cluster.
 struct ClBin {
   int nby, nbz, nbh, plane, h;  // bins in y and z, slots per bin row, per layer, per colour
-  unsigned mh, my;              // 2^32 / nbh and 2^32 / nby, rounded up (cl_div)
+  unsigned mh, my;              // bin_magic of nbh and nby
   int layers;                   // layers per block at most
   int x;                        // iterate, [colour][(layers + 2) * plane]
   int rhs, type;                // right-hand side and row types, [colour][layers * plane]; -1: in registers
@@ -74,9 +74,6 @@ struct ClUp {
   ClBin lv[CLUP + 1];
 };
 static_assert(sizeof(ClCase) % 8 == 0, "ClCase is copied to shared memory in 8-byte words");
-
-// q / d for m = ceil(2^32 / d) and q d < 2^32.
-__device__ __forceinline__ int cl_div(int q, unsigned m, int d) { return d == 1 ? q : (int)__umulhi((unsigned)q, m); }
 
 // A block's view of a bin level.
 struct ClView {
@@ -246,7 +243,7 @@ __device__ __forceinline__ float cl_resid_smem(const ClView& V, int q, const uns
 template <class Res>
 __device__ __forceinline__ float cl_restrict(const ClView& W, int c, int q, int order, int fine_y, int fine_z, int fine_h,
                                              Res res) {
-  const int R = cl_div(q, W.B->mh, W.B->nbh), kk = cl_div(R, W.B->my, W.B->nby);
+  const int R = bin_div(q, W.B->mh, W.B->nbh), kk = bin_div(R, W.B->my, W.B->nby);
   const int J = R - kk * W.B->nby, K = W.k0 + kk, s = q - R * W.B->nbh;
   const int I = 2 * s + ((c + J + K) & 1);
   float acc = 0.0f;
@@ -262,14 +259,14 @@ __device__ __forceinline__ float cl_restrict(const ClView& W, int c, int q, int 
 
 // The iterate of the parent of colour-0 row q of V in the coarse view W (same block).
 __device__ __forceinline__ float cl_parent(const ClView& V, const ClView& W, int q) {
-  const int R = cl_div(q, V.B->mh, V.B->nbh), kk = cl_div(R, V.B->my, V.B->nby);
+  const int R = bin_div(q, V.B->mh, V.B->nbh), kk = bin_div(R, V.B->my, V.B->nby);
   const int J = R - kk * V.B->nby, K = V.k0 + kk, s = q - R * V.B->nbh;
   const int J1 = J >> 1, K1 = K >> 1, c1 = (s + J1 + K1) & 1;
   return W.x[c1 * W.ldx + W.B->plane + (K1 - W.k0) * W.B->plane + J1 * W.B->nbh + (s >> 1)];
 }
 // The same through the coarse level's iterate in global memory.
 __device__ __forceinline__ float cl_parent_global(const ClView& V, const ClBin& W, int q) {
-  const int R = cl_div(q, V.B->mh, V.B->nbh), kk = cl_div(R, V.B->my, V.B->nby);
+  const int R = bin_div(q, V.B->mh, V.B->nbh), kk = bin_div(R, V.B->my, V.B->nby);
   const int J = R - kk * V.B->nby, K = V.k0 + kk, s = q - R * V.B->nbh;
   const int J1 = J >> 1, K1 = K >> 1, c1 = (s + J1 + K1) & 1;
   return __ldcg(&W.gx[c1 * W.h + (K1 * W.nby + J1) * W.nbh + (s >> 1)]);

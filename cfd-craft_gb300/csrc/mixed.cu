@@ -42,6 +42,7 @@
 #include <vector>
 
 #include "state.hpp"
+#include "bin_div.hpp"
 
 namespace cg = cooperative_groups;
 
@@ -2621,8 +2622,7 @@ constexpr int CL_TYPES = 2048;  // more types than this: the level is not planne
 ClBin bin_shape(const BinMatrix& M, const CLev& L) {
   ClBin B{};
   B.nby = M.nb[1], B.nbz = M.nb[2], B.nbh = M.nbh, B.h = M.h, B.plane = M.nb[1] * M.nbh;
-  auto magic = [](int d) { return (unsigned)((((uint64_t)1 << 32) + d - 1) / d); };
-  B.mh = magic(B.nbh), B.my = magic(B.nby);
+  B.mh = bin_magic(B.nbh), B.my = bin_magic(B.nby);
   B.ntypes = (int)M.tab.size();
   B.grhs = L.rhs, B.gx = L.x, B.gres = L.res;
   return B;
@@ -2684,7 +2684,7 @@ void plan_cluster(const CCase& C, const std::vector<int>& jacobi, const std::vec
         }
       }
       const size_t rows = (size_t)B.layers * B.plane;
-      ok = (uint64_t)rows * B.nbh < ((uint64_t)1 << 32);  // cl_div
+      ok = bin_div_exact(rows, B.nbh, B.nby);
       B.x = take(2 * (rows + 2 * B.plane) * 4);
       B.tab = take(48 * M.tab.size());
       B.rhs = B.type = -1;
@@ -2704,8 +2704,7 @@ void plan_cluster(const CCase& C, const std::vector<int>& jacobi, const std::vec
     T.smem = (int)at;
     T.on = 1;
     bool up = T.lc > 0 && T.lc <= CLUP && T.nb > 0;
-    for (int l = 1; l < lc; ++l)
-      up = up && bins[l].h > 0 && (uint64_t)bins[l].h * bins[l].nbh < ((uint64_t)1 << 32);  // cl_div
+    for (int l = 1; l <= lc; ++l) up = up && bins[l].h > 0 && bin_div_exact(bins[l].h, bins[l].nbh, bins[l].nb[1]);
     if (up) {
       U.n = T.lc;
       U.alpha = alpha;
