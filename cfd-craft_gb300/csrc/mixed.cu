@@ -172,6 +172,7 @@ struct CLev {
 
 static_assert(sizeof(CLev) % 8 == 0, "CLev is copied to shared memory in 8-byte words");
 
+struct ClCase;  // coarse_cluster.cuh
 struct CCase {
   int nl;  // levels 1 .. nl (lv[0] is level 1)
   CLev lv[MAXL];
@@ -1863,14 +1864,16 @@ __device__ void c_sweep(const CLev& L, bool backward, int pass, bool gs_on) {
 }
 
 // nu: Gauss-Seidel sweeps before and after the coarse correction (l1-Jacobi levels run
-// the next even count, so their iterate ends in x).
-__global__ void __launch_bounds__(CT) k_coarse(const CCase* cases, const MState* ST, int nu) {
+// the next even count, so their iterate ends in x). cl: the plans of the cases that
+// k_coarse_cluster has done (null: none).
+__device__ bool on_cluster(const ClCase* cl, int ci);
+__global__ void __launch_bounds__(CT) k_coarse(const CCase* cases, const MState* ST, int nu, const ClCase* cl) {
   pdl_enter();
   __shared__ double sh[32];
   const int csz = (int)cg::this_cluster().num_blocks();
   const int ci = blockIdx.x / csz;
   const MState& S = ST[ci];
-  if (!(S.state == RUN || S.state == START)) return;  // uniform over the cluster
+  if (!(S.state == RUN || S.state == START) || on_cluster(cl, ci)) return;  // uniform over the cluster
   const CCase& C = cases[ci];
   const int rank = (int)cg::this_cluster().block_rank();
   const int tid = rank * blockDim.x + threadIdx.x, nth = csz * blockDim.x;
@@ -2145,6 +2148,8 @@ __device__ __forceinline__ void terminal_block(const CLev& L, int bk, int ln) {
 }
 
 #include "coarse_cluster.cuh"
+
+__device__ __forceinline__ bool on_cluster(const ClCase* cl, int ci) { return cl && cl[ci].on; }
 
 // Levels l0 .. of case C, down to the terminal level and back up to l0.
 __device__ void blk_cycle(const CCase& C, int l0, int nu, double* sh) {
@@ -3743,7 +3748,8 @@ void launch_coarse(cfdg_batch* B, cudaStream_t s) {
     return;
   }
   cluster_config(cfg, at, nc, B->csize, CT, 0, s);
-  cudaLaunchKernelEx(&cfg, k_coarse, (const CCase*)B->d_cc, (const MState*)B->d_st, B->nuc);
+  cudaLaunchKernelEx(&cfg, k_coarse, (const CCase*)B->d_cc, (const MState*)B->d_st, B->nuc,
+                     (const ClCase*)(B->any_cl ? B->d_cl : nullptr));
 }
 
 #define FINE(K, W, ...) \
