@@ -470,6 +470,35 @@ __global__ void k_ic0_bwd(const int* __restrict__ order, int begin, int end, con
   z[c] = v / diag[c];
 }
 
+// v -+ sum a_ik x_k over a row's entries in order, the loads of GATHER_AHEAD of them in flight: the
+// coarse levels' kernel waits for the L2 round trips of columns and then values at every dependency
+// level. How many the compiler has in flight by itself changed with the code around the loop (a
+// closed domain of 33x31x65, rows of up to 26 entries: 201 ms a solve, 245 once the line smoothers had
+// left the kernel; four ahead 183, eight 137). A row's end is a branch: a predicated FP64 operation
+// occupies the pipe for its 64 cycles as well (eight ahead 167). k_gs keeps the plain loop (gs_row):
+// its rows of level 0 have at most six entries (3x5x4 with a periodic axis 1.24 against 1.42 ms).
+constexpr int GATHER_AHEAD = 8;
+template <bool SUB>
+__device__ __forceinline__ double gather_row(double v, const int* __restrict__ col, const double* __restrict__ val,
+                                             int b, int e, const double* x) {
+  for (int k = b; k < e; k += GATHER_AHEAD) {
+    int c[GATHER_AHEAD];
+    double a[GATHER_AHEAD], xc[GATHER_AHEAD];
+#pragma unroll
+    for (int m = 0; m < GATHER_AHEAD; ++m)
+      if (k + m < e) c[m] = col[k + m], a[m] = val[k + m];
+#pragma unroll
+    for (int m = 0; m < GATHER_AHEAD; ++m)
+      if (k + m < e) xc[m] = __ldcg(&x[c[m]]);
+#pragma unroll
+    for (int m = 0; m < GATHER_AHEAD; ++m) {
+      if (k + m >= e) return v;
+      v = SUB ? v - a[m] * xc[m] : v + a[m] * xc[m];
+    }
+  }
+  return v;
+}
+
 // Row bodies shared by the level-by-level kernels and the cooperative coarse kernel
 // (same operations, same order; L2 loads for vectors another block may have written).
 __device__ __forceinline__ void gs_row(int i, const int* __restrict__ off, const int* __restrict__ col,
@@ -484,12 +513,20 @@ __device__ __forceinline__ void gs_row(int i, const int* __restrict__ off, const
   for (int k = off[i]; k < off[i + 1]; ++k) v = v - val[k] * __ldcg(&x[col[k]]);
   x[i] = v / d;
 }
+__device__ __forceinline__ void gs_row_ahead(int i, const int* __restrict__ off, const int* __restrict__ col,
+                                             const double* __restrict__ val, const double* __restrict__ diag,
+                                             const double* rhs, double* x) {
+  const double d = diag[i];
+  if (d == 0.0) {  // an isolated sealed cell: a null pressure space
+    x[i] = 0.0;
+    return;
+  }
+  x[i] = gather_row<true>(__ldcg(&rhs[i]), col, val, off[i], off[i + 1], x) / d;
+}
 __device__ __forceinline__ void residual_row(int i, const int* __restrict__ off, const int* __restrict__ col,
                                              const double* __restrict__ val, const double* __restrict__ diag,
                                              const double* rhs, const double* x, double* res) {
-  double v = diag[i] * __ldcg(&x[i]);
-  for (int k = off[i]; k < off[i + 1]; ++k) v = v + val[k] * __ldcg(&x[col[k]]);
-  res[i] = __ldcg(&rhs[i]) - v;
+  res[i] = __ldcg(&rhs[i]) - gather_row<false>(diag[i] * __ldcg(&x[i]), col, val, off[i], off[i + 1], x);
 }
 __device__ __forceinline__ void restrict_row(int j, const int* __restrict__ off, const int* __restrict__ child,
                                              const double* __restrict__ w, const double* res, double* rhs_c) {
@@ -688,7 +725,7 @@ __device__ void pc_sweep(const PLev& L, bool backward, Bar& grid) {
     if (blockIdx.x == 0)
       for (int dl = 0; dl < nlev; ++dl) {
         for (int t = start[dl] + threadIdx.x; t < start[dl + 1]; t += blockDim.x)
-          gs_row(order[t], L.off, L.col, L.val, L.diag, L.rhs, L.x);
+          gs_row_ahead(order[t], L.off, L.col, L.val, L.diag, L.rhs, L.x);
         __threadfence();
         __syncthreads();
       }
@@ -698,7 +735,7 @@ __device__ void pc_sweep(const PLev& L, bool backward, Bar& grid) {
   }
   const int gt = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
   for (int dl = 0; dl < nlev; ++dl) {
-    for (int t = start[dl] + gt; t < start[dl + 1]; t += nth) gs_row(order[t], L.off, L.col, L.val, L.diag, L.rhs, L.x);
+    for (int t = start[dl] + gt; t < start[dl + 1]; t += nth) gs_row_ahead(order[t], L.off, L.col, L.val, L.diag, L.rhs, L.x);
     __threadfence();
     grid.sync();
   }
