@@ -68,6 +68,36 @@ def test_scalar_steps_bit_identical(pkg, O, name, perturb):
     dg.close()
 
 
+@pytest.mark.parametrize("faces", ["uniform", "per face"])
+@pytest.mark.parametrize("per_sm,more", [(3, 0), (3, 1), (4, 0), (4, 1)])
+def test_scalar_steps_at_the_edges_of_the_shares(pkg, O, per_sm, more, faces):
+    """Slices of columns just up to and beyond the numbers per SM at which the blocks' shares change."""
+    torch = pytest.importorskip("torch")
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    case = pkg.synth.case((64, 48, per_sm * sms // 12 + more), 1.5, inflow=3.0, preconditioner="ic0",
+                          boxes=[((20.0, 5.0, 0.0), (31.0, 12.0, 30.0))])  # 2 x 6 columns
+    g = pkg.grid.Grid.build(case)
+    og = O.Grid(case)
+    dg = pkg.pressure.DeviceGrid(g, preconditioner="ic0")
+    rng = np.random.default_rng(17)
+    if faces == "per face":
+        area = np.asarray(g.face_area) * rng.uniform(0.8, 1.2, g.n_faces)
+        dist = np.asarray(g.face_distance) * rng.uniform(0.9, 1.1, g.n_faces)
+        og.set_faces(area, dist)
+        dg.update_faces(area, dist)
+    u = pkg.synth.random_velocity(g, 5)
+    fluid = g.fluid.astype(bool)
+    c, d = np.where(fluid, rng.uniform(0.0, 1e-3, g.count), 0.0), np.where(fluid, rng.uniform(0.01, 0.5, g.count), 0.0)
+    source = np.where(rng.random(g.count) < 0.01, 1e-4, 0.0)
+    d_u, d_c, d_d, d_s = (torch.from_numpy(a.copy()).to("cuda:0") for a in (u, c, d, source))
+    for _ in range(2):
+        c = og.scalar_step(c, u, d, source, 0.02)
+        dg.scalar_step_device(d_u.data_ptr(), d_c.data_ptr(), d_d.data_ptr(), d_s.data_ptr(), 0.02)
+    torch.cuda.synchronize()
+    assert np.array_equal(bits(d_c.cpu().numpy()), bits(c))
+    dg.close()
+
+
 @pytest.mark.parametrize("muscl", [False, True])
 @pytest.mark.parametrize("name,perturb", [("wide-tiles", False), ("buildings-open-wall", False),
                                           ("spacing-1.5m", False), ("wide-tiles", True)])
