@@ -231,7 +231,8 @@ __device__ __forceinline__ void cl_sweep_smem(const ClView& V, int c, bool skipx
 __device__ __forceinline__ float cl_resid_smem(const ClView& V, int q, const unsigned char* smem) {
   const ClBin& B = *V.B;
   const int P = B.plane;
-  const ClRow r = cl_row(reinterpret_cast<const float4*>(smem + B.tab), reinterpret_cast<const unsigned short*>(smem + B.type)[q]);
+  const unsigned short* ty = reinterpret_cast<const unsigned short*>(smem + B.type);
+  const ClRow r = cl_row(reinterpret_cast<const float4*>(smem + B.tab), ty[q]);
   const float v = cl_sum<false>(__fmul_rn(r.b.z, V.x[P + q]), V.x + V.ldx + P + q, r);
   return reinterpret_cast<const float*>(smem + B.rhs)[q] - v;
 }
@@ -297,7 +298,8 @@ __device__ __forceinline__ float cl_list_sum(float v, const int* ec, const float
 }
 // One colour's rows t0, t0 + step, ...
 template <bool GLOBAL>
-__device__ __forceinline__ void cl_sweep_list(const CLev& L, int color, bool skipx, float* x, const float* rhs, int t0, int step) {
+__device__ __forceinline__ void cl_sweep_list(const CLev& L, int color, bool skipx, float* x, const float* rhs, int t0,
+                                              int step) {
   const int c0 = L.coff[color], nrow = L.coff[color + 1] - c0, base = L.ell_off[color], w = L.ell_w[color];
   for (int t = t0; t < nrow; t += step) {
     float v = GLOBAL ? __ldcg(&rhs[c0 + t]) : rhs[c0 + t];
@@ -455,7 +457,8 @@ __device__ void cl_first_block(const ClCase& C, const CCase& D, int nu, unsigned
   }
 }
 
-__global__ void __launch_bounds__(CLT, 1) k_coarse_cluster(const ClCase* cases, const CCase* cc, const MState* ST, int nu) {
+__global__ void __launch_bounds__(CLT, 1)
+    k_coarse_cluster(const ClCase* cases, const CCase* cc, const MState* ST, int nu) {
   pdl_enter();
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ ClCase C;
@@ -548,8 +551,8 @@ __global__ void __launch_bounds__(CLT, 1) k_coarse_cluster(const ClCase* cases, 
       const int rows = N.layers * N.plane;
       for (int e = threadIdx.x; e < 2 * W.nl; e += CLT) {
         const int c = e >= W.nl ? 1 : 0, q = e - c * W.nl;
-        const int order = __float_as_int(
-            reinterpret_cast<const float4*>(smem + N.tab)[3 * reinterpret_cast<const unsigned short*>(smem + N.type)[c * rows + q] + 2].w);
+        const unsigned short* ty = reinterpret_cast<const unsigned short*>(smem + N.type);
+        const int order = __float_as_int(reinterpret_cast<const float4*>(smem + N.tab)[3 * ty[c * rows + q] + 2].w);
         rhs[c * rows + q] = cl_restrict(W, c, q, order, B.nby, B.nbz, B.nbh, [&](int k, int j, int s) {
           const int f = (k - V.k0) * B.plane + j * B.nbh + s;
           return r0 ? V.x[B.plane + f] : cl_resid_smem(V, f, smem);

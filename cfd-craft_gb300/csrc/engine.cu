@@ -19,8 +19,8 @@
 // Also here, on device arrays: laminar SSPRK2 time stepping (momentum right-hand side
 // and stage update, cfdg_step_device), linear-upwind scalar transport (k_scalar_pass,
 // cfdg_scalar_step_device), receptor sampling (cfdg_receptors_sample), and the
-// line/plane block smoothers of anisotropic multigrid hierarchies (line_cluster.cuh). All of it follows the reference's operation order
-// (bit-identical results) under -fmad=false.
+// line/plane block smoothers of anisotropic multigrid hierarchies (line_cluster.cuh). All of it
+// follows the reference's operation order (bit-identical results) under -fmad=false.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -1119,7 +1119,8 @@ void launch_vcycle(cfdg_grid* G, const double* r, double* z, const Scalars* S) {
       else k_residual_struct<false><<<grid_blocks(L.n), BLOCK, 0, s>>>(G->g, L.diag, L.rhs, L.x, L.res, L.n, S);
       tick(G);
     } else if (planned) {
-      k_plan_residual<<<grid_blocks((long long)PCS * H.pc_chunk[l - 1]), BLOCK, 0, s>>>((const PcPlan*)H.d_pc, l - 1, S); tick(G);
+      k_plan_residual<<<grid_blocks((long long)PCS * H.pc_chunk[l - 1]), BLOCK, 0, s>>>((const PcPlan*)H.d_pc, l - 1,
+                                                                                        S); tick(G);
     } else {
       k_residual<<<grid_blocks(L.n), BLOCK, 0, s>>>(L.n, L.a.off, L.a.col, L.a.val, L.diag, L.rhs, L.x, L.res, S); tick(G);
     }

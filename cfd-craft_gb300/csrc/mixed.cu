@@ -2622,7 +2622,9 @@ bool encode_split(CUtensorMap& m, const void* base, bool u16, int nxh, int rows,
              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-constexpr int CL_TYPES = 2048;  // more types than this: the level is not planned as a bin level
+// More types than this: the level is not planned as a bin level (its table would take more than 96 KB
+// of a block's shared memory; the first level of a site with 30 buildings has 261).
+constexpr int CL_TYPES = 2048;
 
 ClBin bin_shape(const BinMatrix& M, const CLev& L) {
   ClBin B{};
@@ -2644,13 +2646,19 @@ int upload_types(Arena& A, cudaStream_t s, const BinMatrix& M, ClBin& B) {
 
 // Plans k_coarse_cluster for a case whose coarse levels allow it (aggregation levels of at
 // most two colours without closed groups), but for the row types on the device (upload_plan);
-// bins[l] holds the bin levels among levels 1.. (h == 0: not a bin level). Levels are split over the cluster's
-// blocks while their layers fill at least three quarters of them and a split phase beats one
-// block's (about 1,200 rows), or while one block would be slow (above 2,500 rows); levels
-// without a bin layout are split above 1,500 rows. The cluster starts at the first level
-// whose slabs fit the blocks' registers and shared memory; a level split by rows is taken up
-// to 32,768 of them (four a thread).
-// Where the levels above are bin levels, too, U describes them.
+// bins[l] holds the bin levels among levels 1.. (h == 0: not a bin level).
+//
+// Levels are split over the cluster's blocks while their layers fill three quarters of them and a
+// split phase beats one block's (1,200 rows), or while one block would be slow (above 2,500 rows);
+// levels without a bin layout are split above 1,500 rows. us a cycle of all coarse levels: 48x48x48
+// 26.2 and, split from 2,400 rows or only with 16 layers, 28.8; 96x80x10 29.3 and, with few layers
+// split from 1,250 rows, 31.4; 75x61x37 32 and, from 5,000 rows, 40; lists from 750 rows 100x84x50
+// 77 -> 86, from 3,000 128x128x64 99 -> 110, never 179.
+//
+// The cluster starts at the first level whose slabs fit the blocks' registers and shared memory. A
+// level split by rows is taken up to 32,768 of them, four a thread (up to 8,192: 128x128x64 99 ->
+// 193, its first such level then runs grid-wide), one of the first block's to 4,096, whose iterate and
+// right-hand side take 32 KB. Where the levels above are bin levels, too, U describes them.
 void plan_cluster(const CCase& C, const std::vector<int>& jacobi, const std::vector<BinMatrix>& bins, float alpha,
                   ClCase& K, ClUp& U) {
   K = ClCase{};
@@ -3776,9 +3784,11 @@ void enqueue_vcycle(cfdg_batch* B, cudaStream_t s) {
     launch_rb(B, W, 0, sw == 0 ? 1 : 0, s);
     launch_rb(B, W, 1, 0, s);
   }
-  if (B->any_groups) launch_pdl(k_center0, grid_of(k_center0, 256, B->g_g), 256, 0, s, B->d_fc, B->d_st, W.gtab, W.counts + 3, 1);
+  if (B->any_groups)
+    launch_pdl(k_center0, grid_of(k_center0, 256, B->g_g), 256, 0, s, B->d_fc, B->d_st, W.gtab, W.counts + 3, 1);
   FINE(k_v_resid, W);
-  if (B->any_groups) launch_pdl(k_center0, grid_of(k_center0, 256, B->g_g), 256, 0, s, B->d_fc, B->d_st, W.gtab, W.counts + 3, 2);
+  if (B->any_groups)
+    launch_pdl(k_center0, grid_of(k_center0, 256, B->g_g), 256, 0, s, B->d_fc, B->d_st, W.gtab, W.counts + 3, 2);
   launch_pdl(k_v_restrict, grid_of(k_v_restrict, TILE, B->g_1), TILE, 0, s, B->d_fc, B->d_st, W.tiles1, W.counts + 1);
   launch_coarse(B, s);
   FINE(k_v_prolong, W);
@@ -3787,7 +3797,8 @@ void enqueue_vcycle(cfdg_batch* B, cudaStream_t s) {
     launch_rb(B, W, 1, 0, s);
     launch_rb(B, W, 0, 0, s);
   }
-  if (B->any_groups) launch_pdl(k_center0, grid_of(k_center0, 256, B->g_g), 256, 0, s, B->d_fc, B->d_st, W.gtab, W.counts + 3, 1);
+  if (B->any_groups)
+    launch_pdl(k_center0, grid_of(k_center0, 256, B->g_g), 256, 0, s, B->d_fc, B->d_st, W.gtab, W.counts + 3, 1);
 }
 
 // One iteration of the per-case state machine.
@@ -4499,31 +4510,50 @@ int64_t cfdg_batch_stats_json(cfdg_batch* B, char* buf, int64_t cap) {
   return (int64_t)out.size() + 1;
 }
 
-// Algorithmic bytes of one launch of the coarse levels of every case (each logical array
-// read or written once per phase): per non-terminal level of n rows, E ELL entries (8 bytes
-// each: value and column) and nnz CSR entries, the 2 nu sweeps read the ELL block, the
-// right-hand side and 1/diag and write x (8 E + 12 n each); x is zeroed (4 n); the residual
-// reads the ELL block of colour 0 with diag, x and rhs and writes res (a res0 level, about
-// half: 4 E + 8 n), or the CSR rows (8 nnz + 20 n); the restriction reads res, children and
-// weights (12 n) and writes the next level's right-hand side; the prolongation reads the
-// injection rows and updates x (20 n). The terminal blocks read their inverse (8 m^2 each).
+// Algorithmic bytes in global memory of one launch of the coarse levels of every case (each logical
+// array read or written once per phase), by how a level runs:
+// - Grid-wide over index lists, per non-terminal level of n rows, E ELL entries (8 bytes each: value
+//   and column) and nnz CSR entries: the 2 nu sweeps read the ELL block, the right-hand side and
+//   1/diag and write x (8 E + 12 n each); x is zeroed (4 n); the residual reads the ELL block of
+//   colour 0 with diag, x and rhs and writes res (a res0 level, about half: 4 E + 8 n), or the CSR
+//   rows (8 nnz + 20 n); the restriction reads res, children and weights (12 n) and writes the next
+//   level's right-hand side; the prolongation reads the injection rows and updates x (20 n).
+// - Grid-wide over row types (k_up_*), n rows: the sweeps read right-hand side, type and the other
+//   colour and write x (14 n each); residual and restriction read colour 0's right-hand side, type
+//   and x and colour 1's x (7 n) and the next level's types and write its right-hand side (6 each);
+//   the prolongation updates colour 0 (4 n) and reads the next level's x (4 each).
+// - On a cluster: a bin level's row types and table once (2 n + 48 per type) and, of the first one,
+//   right-hand side and x (8 n); levels by index lists the ELL block and 1/diag in each sweep (8 E +
+//   4 n), the residual's half of it, the children's lists and the injection rows (4 E + 16 n); the
+//   right-hand side and x that pass between the split levels and the first block's (8 n).
+// The terminal blocks read their inverse (at most 32 x 8 bytes a row).
 double coarse_bytes(const cfdg_batch* B) {
   double total = 0.0;
   const double nu = (double)B->nuc;
-  for (const auto& cs : B->cases) {
-    for (size_t l = 0; l < cs->stats.size(); ++l) {
+  for (size_t i = 0; i < B->cases.size(); ++i) {
+    const auto& cs = B->cases[i];
+    const ClCase& K = B->plan[i];
+    const ClUp& U = B->ups[i];
+    const int nl = (int)cs->stats.size();
+    for (int l = 0; l < nl; ++l) {
       const auto& v = cs->stats[l];
       const double n = (double)v.rows, E = (double)v.ell, nnz = (double)v.nnz;
-      const bool terminal = (int)l == cs->C.nl - 1;
-      if (terminal) {
-        total += 8.0 * n + 8.0 * n * 32.0;  // rhs in, x out, up to 32 x 32 inverse entries per row
-        continue;
+      const double n1 = l + 1 < nl ? (double)cs->stats[l + 1].rows : 0.0;
+      const int t = l - K.lc;  // the level in the cluster's plan
+      if (l == nl - 1) {
+        total += 8.0 * n + 8.0 * n * 32.0;  // rhs in, x out, the inverse
+      } else if (K.on && t >= 0) {
+        if (t < K.nb) total += 2.0 * n + 48.0 * K.b[t].ntypes + (t == 0 ? 8.0 * n : 0.0);
+        else total += 2.0 * nu * (8.0 * E + 4.0 * n) + 4.0 * E + 16.0 * n + (t == 0 ? 8.0 * n : 0.0);
+        if (t > 0 && t == K.nd + K.ndl) total += 8.0 * n;
+      } else if (l < U.n) {
+        total += 2.0 * nu * 14.0 * n + 11.0 * n + 10.0 * n1;
+      } else {
+        const bool res0 = cs->C.lv[l].res0 != 0;
+        total += 2.0 * nu * (8.0 * E + 12.0 * n) + 4.0 * n;
+        total += res0 ? 4.0 * E + 8.0 * n : 8.0 * nnz + 20.0 * n;
+        total += 12.0 * n + 4.0 * n1 + 20.0 * n;
       }
-      const bool res0 = cs->C.lv[l].res0 != 0;
-      total += 2.0 * nu * (8.0 * E + 12.0 * n) + 4.0 * n;
-      total += res0 ? 4.0 * E + 8.0 * n : 8.0 * nnz + 20.0 * n;
-      total += 12.0 * n + 4.0 * (l + 1 < cs->stats.size() ? (double)cs->stats[l + 1].rows : 0.0);
-      total += 20.0 * n;
     }
   }
   return total;
@@ -4581,7 +4611,7 @@ int cfdg_batch_time_kernel(cfdg_batch* B, int32_t which, int32_t reps, double* m
       case 7:  // level-0 residual and its restriction to level 1
         FINE(k_v_resid, B->run);
         launch_pdl(k_v_restrict, grid_of(k_v_restrict, TILE, B->g_1), TILE, 0, s, B->d_fc, B->d_st, B->run.tiles1,
-                                                                          B->run.counts + 1);
+                   B->run.counts + 1);
         break;
       case 9:  // e += alpha p, r -= alpha q with |r|^2
         FINE(k_update, B->run);

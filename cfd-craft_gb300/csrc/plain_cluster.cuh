@@ -27,10 +27,17 @@
 namespace {
 
 constexpr int PCS = 16;             // blocks per cluster (non-portable size)
-constexpr int PCT = 128;            // threads per block: one warp per sub-core, whose FP64 unit takes a warp's operation in 64 cycles
+constexpr int PCT = 128;            // threads per block: a warp per sub-core (its FP64 unit takes an operation in 64 cycles)
 constexpr int PC_SMEM = 208 * 1024;  // dynamic shared memory a plan may ask for
-constexpr int PC_GRID_ROWS = 40000;  // rows above which the transfers are grid-wide kernels
-constexpr int PC_SOLO_ROWS = 96;     // mean rows per dependency level up to which one block sweeps alone
+// Rows above which a level's transfers are grid-wide kernels. A cycle with them against the cluster's
+// own: 128x128x64 (131,000 rows) 3.70 / 3.81 ms, 100x84x50 (52,000) 2.43 / 2.47, 110x80x40 without
+// buildings (44,000) 42.6 / 42.7; from 30,000 rows down no difference.
+constexpr int PC_GRID_ROWS = 40000;
+// Mean rows per dependency level up to which one block sweeps alone. None alone, up to 48, 96, 144
+// (ms a cycle): 24x20x16 0.48, 0.43, 0.43, 0.43; 40x36x27 0.91, 0.86, 0.86, 0.97; 100x84x50 2.48,
+// 2.44, 2.43, 2.57; up to 400 128x128x64 6.2 instead of 3.7. Wide rows would take more: 110x80x40
+// without buildings 46.8, 42.6, 42.6, 37.0.
+constexpr int PC_SOLO_ROWS = 96;
 constexpr int PC_MAXLEV = 12;
 
 constexpr int PCW = 6;
@@ -290,8 +297,6 @@ __device__ __noinline__ void pc_direct(const int* ix, int n, const double* f, co
   if (on) x[ix[ln]] = xl;
 }
 
-// WHAT 0: two forward sweeps of level `from` from zero, its iterate to global memory. 1: two
-// backward sweeps of its iterate in global memory. 2: the whole cycle from level `from` on.
 // res = rhs - A x of a level whose transfers are grid-wide, from the plan's rows: the vectors in
 // row numbering, the neighbours through their owners' positions.
 __global__ void k_plan_residual(const PcPlan* plan, int l, const Scalars* S) {
@@ -324,6 +329,8 @@ __global__ void k_plan_residual(const PcPlan* plan, int l, const Scalars* S) {
   }
 }
 
+// what 0: two forward sweeps of level `from` from zero, its iterate to global memory. 1: two
+// backward sweeps of its iterate in global memory. 2: the whole cycle from level `from` on.
 __global__ void __launch_bounds__(PCT, 1) k_plain_cluster(const PcPlan* plan, int from, int what, const Scalars* S) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ PcLev sL, sN;

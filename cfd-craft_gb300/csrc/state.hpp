@@ -194,8 +194,8 @@ struct DevHierarchy {
   int* fluid_idx = nullptr;
   std::vector<DevLevel> levels;
   std::vector<uint64_t> level_cells, level_nonzeros;
-  // Without a cluster plan: levels 1 .. L-1 as one cooperative kernel's descriptors (engine.cu PLev), and its grid
-  // (0: not co-resident, the level-by-level launches are used instead).
+  // Without a cluster plan: levels 1 .. L-1 as one cooperative kernel's descriptors (engine.cu
+  // PLev), and its grid (0: not co-resident, the level-by-level launches are used instead).
   void* d_plev = nullptr;
   int coop_blocks = 0;
   bool cluster = false;  // the coarse kernel runs as one thread-block cluster (engine.cu)
