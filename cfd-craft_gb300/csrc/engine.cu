@@ -1994,7 +1994,9 @@ int ensure_sweeps(cfdg_grid* G, cfdg_info* info) {
     const auto t0 = std::chrono::steady_clock::now();
     cudaStream_t s = G->stream;
     for (DevLevel& L : D.levels) L.lean = false;
+    D.arena.spare = true;
     int e = plan_levels(D, *G->host_mg, s);
+    D.arena.spare = false;
     if (e == CFDG_ERR_ADMISSION) e = lean_levels(D, *G->host_mg, s);
     const cudaError_t c = cudaStreamSynchronize(s);
     if (!e && c != cudaSuccess) e = fail(CFDG_ERR_CUDA, cudaGetErrorString(c));
@@ -2010,6 +2012,29 @@ int ensure_sweeps(cfdg_grid* G, cfdg_info* info) {
   if (info) info->hierarchy_bytes = D.arena.bytes;
   return 0;
 }
+
+}  // namespace
+
+bool cfdg::release_sweeps(cfdg_context* ctx, uint64_t bytes) {
+  std::lock_guard<std::mutex> lk(ctx->mu);
+  for (cfdg_grid* G : ctx->open) {
+    if (ctx->used.load() + bytes <= ctx->budget) break;
+    std::unique_lock<GridMutex> grid(G->mu, std::try_to_lock);
+    if (!grid || !G->mg || !G->mg->ready) continue;
+    if (cudaDeviceSynchronize() != cudaSuccess) return false;
+    DevHierarchy& D = *G->mg;
+    reset_chunk(G);  // its graph may hold their addresses
+    D.arena.rollback(D.base_ptrs, D.base_bytes);
+    D.ready = false;
+    D.d_pc = D.d_plev = nullptr;
+    D.pc_rest = D.pc_smem = D.coop_blocks = 0;
+    D.cluster = false;
+    D.pc_chunk.clear();
+  }
+  return ctx->used.load() + bytes <= ctx->budget;
+}
+
+namespace {
 
 // pressure.rs:55-97: the cached factor, or the hierarchy checked against its signature.
 int prepare_preconditioner(cfdg_grid* G, const Poller& poll, cfdg_info* info) {
@@ -3076,6 +3101,7 @@ int cfdg_grid_open(cfdg_context* ctx, const cfdg_grid_desc* d, cfdg_grid** out) 
   {
     std::lock_guard<std::mutex> lk(ctx->mu);
     ctx->grids += 1;
+    ctx->open.push_back(G.get());
   }
   *out = G.release();
   return 0;
@@ -3085,7 +3111,11 @@ void cfdg_grid_close(cfdg_grid* G) {
   if (!G) return;
   cfdg_context* ctx = G->ctx;
   {
-    std::lock_guard<std::mutex> lk(G->mu);
+    std::lock_guard<std::mutex> lk(ctx->mu);
+    ctx->open.erase(std::remove(ctx->open.begin(), ctx->open.end(), G), ctx->open.end());
+  }
+  {
+    std::lock_guard<GridMutex> lk(G->mu);
     cudaSetDevice(G->ctx->device);
     if (G->stream) cudaStreamSynchronize(G->stream);
     G->solo.reset();  // before the streams go: the batch may hold the grid's stream
@@ -3120,7 +3150,7 @@ uint64_t cfdg_grid_device_bytes(const cfdg_grid* G) {
 
 int cfdg_grid_update_faces(cfdg_grid* G, const double* area, const double* distance) {
   if (int e = check_grid(G)) return e;
-  std::lock_guard<std::mutex> lk(G->mu);
+  std::lock_guard<GridMutex> lk(G->mu);
   CU(cudaSetDevice(G->ctx->device));
   if (area) G->h.face_area.assign(area, area + G->h.faces);
   if (distance) G->h.face_distance.assign(distance, distance + G->h.faces);
@@ -3135,7 +3165,7 @@ int cfdg_grid_update_faces(cfdg_grid* G, const double* area, const double* dista
 
 int cfdg_grid_configure(cfdg_grid* G, int32_t preconditioner, int32_t precision) {
   if (int e = check_grid(G)) return e;
-  std::lock_guard<std::mutex> lk(G->mu);
+  std::lock_guard<GridMutex> lk(G->mu);
   if (preconditioner != CFDG_PRECOND_IC0 && preconditioner != CFDG_PRECOND_MULTIGRID)
     return fail(CFDG_ERR_INVALID, "unknown preconditioner");
   if (preconditioner != G->preconditioner) reset_chunk(G);
@@ -3150,7 +3180,7 @@ int cfdg_grid_set_flow(cfdg_grid* G, const cfdg_flow_desc* flow) {
   for (int a = 0; a < 3; ++a)
     if (flow->boundary[a] == 0 || flow->boundary[a] == 4)
       return fail(CFDG_ERR_UNSUPPORTED, "laminar stepping supports open, wall and slip boundaries");
-  std::lock_guard<std::mutex> lk(G->mu);
+  std::lock_guard<GridMutex> lk(G->mu);
   CU(cudaSetDevice(G->ctx->device));
   if (!G->st_cu) {
     Arena& A = G->arena;
@@ -3174,7 +3204,7 @@ int cfdg_step_device(cfdg_grid* G, double* d_u, double* d_p, double dt, double t
                      cfdg_poll_fn poll, void* poll_ctx, cfdg_info* info) {
   if (int e = check_grid(G)) return e;
   if (!d_u || !d_p) return fail(CFDG_ERR_INVALID, "null u or p");
-  std::lock_guard<std::mutex> lk(G->mu);
+  std::lock_guard<GridMutex> lk(G->mu);
   if (!G->has_flow) return fail(CFDG_ERR_INVALID, "cfdg_grid_set_flow has not been called for this grid");
   CU(cudaSetDevice(G->ctx->device));
   cudaStream_t s = G->stream;
@@ -3226,7 +3256,7 @@ static int scalar_impl(cfdg_grid* G, const double* d_u, double* d_c, const doubl
   if (int e = check_grid(G)) return e;
   if (!d_u || !d_c || !d_diff || !d_source) return fail(CFDG_ERR_INVALID, "null array");
   if ((mode == 1 && !d_budget) || (mode == 2 && !rates)) return fail(CFDG_ERR_INVALID, "null budget or rates");
-  std::lock_guard<std::mutex> lk(G->mu);
+  std::lock_guard<GridMutex> lk(G->mu);
   CU(cudaSetDevice(G->ctx->device));
   for (int a = 0; a < 3; ++a)
     if (G->h.periodic[a]) return fail(CFDG_ERR_UNSUPPORTED, "scalar transport on the device: periodic axes");
@@ -3331,7 +3361,7 @@ int cfdg_scalar_step_device(cfdg_grid* G, const double* d_u, double* d_c, const 
 int cfdg_grid_set_advection(cfdg_grid* G, int32_t muscl) {
   if (int e = check_grid(G)) return e;
   if (muscl != 0 && muscl != 1) return fail(CFDG_ERR_INVALID, "advection is 0 (linear upwind) or 1 (MUSCL)");
-  std::lock_guard<std::mutex> lk(G->mu);
+  std::lock_guard<GridMutex> lk(G->mu);
   G->sc_muscl = muscl;
   return 0;
 }
@@ -3368,7 +3398,7 @@ int cfdg_receptors_set(cfdg_grid* G, int32_t n, const int64_t* offsets, const in
   const int64_t m = n > 0 ? offsets[n] : 0;
   for (int64_t k = 0; k < m; ++k)
     if (cells[k] < 0 || cells[k] >= G->h.cells) return fail(CFDG_ERR_INVALID, "a receptor cell is outside the grid");
-  std::lock_guard<std::mutex> lk(G->mu);
+  std::lock_guard<GridMutex> lk(G->mu);
   CU(cudaSetDevice(G->ctx->device));
   // Grown arrays come from the grid's arena (released with the grid); smaller sets reuse them.
   if (n + 1 > G->rc_cap_n) {
@@ -3394,7 +3424,7 @@ int cfdg_receptors_set(cfdg_grid* G, int32_t n, const int64_t* offsets, const in
 
 int cfdg_receptors_sample(cfdg_grid* G, const double* d_c, double* d_out) {
   if (int e = check_grid(G)) return e;
-  std::lock_guard<std::mutex> lk(G->mu);
+  std::lock_guard<GridMutex> lk(G->mu);
   if (G->rc_n == 0) return 0;
   if (!d_c || !d_out) return fail(CFDG_ERR_INVALID, "null array");
   CU(cudaSetDevice(G->ctx->device));
@@ -3407,7 +3437,7 @@ int cfdg_receptors_sample(cfdg_grid* G, const double* d_c, double* d_out) {
 int cfdg_debug_momentum_update(cfdg_grid* G, const double* u, const double* p, double dt, double* out) {
   if (int e = check_grid(G)) return e;
   if (!u || !p || !out) return fail(CFDG_ERR_INVALID, "null array");
-  std::lock_guard<std::mutex> lk(G->mu);
+  std::lock_guard<GridMutex> lk(G->mu);
   if (!G->has_flow) return fail(CFDG_ERR_INVALID, "cfdg_grid_set_flow has not been called for this grid");
   CU(cudaSetDevice(G->ctx->device));
   cudaStream_t s = G->stream;
@@ -3428,7 +3458,7 @@ int cfdg_grid_set_cycle(cfdg_grid* G, int32_t nu_fine, int32_t nu_coarse) {
   if (int e = check_grid(G)) return e;
   if (nu_fine < 1 || nu_fine > 4 || nu_coarse < 1 || nu_coarse > 4)
     return fail(CFDG_ERR_INVALID, "sweep counts must be 1..4");
-  std::lock_guard<std::mutex> lk(G->mu);
+  std::lock_guard<GridMutex> lk(G->mu);
   if (G->mx_nu0 != nu_fine || G->mx_nuc != nu_coarse) G->solo.reset();
   G->mx_nu0 = nu_fine;
   G->mx_nuc = nu_coarse;
@@ -3440,7 +3470,7 @@ int cfdg_grid_set_sweep_tile(cfdg_grid* G, int32_t rows, int32_t stages) {
   const bool automatic = rows == 0 && stages == 0;
   if (!automatic && (!(rows == 8 || rows == 16 || rows == 32) || stages < 2 || stages > 8))
     return fail(CFDG_ERR_INVALID, "sweep tile: rows must be 8, 16 or 32 and stages 2..8 (or both 0)");
-  std::lock_guard<std::mutex> lk(G->mu);
+  std::lock_guard<GridMutex> lk(G->mu);
   if (G->mx_sweep_rows != rows || G->mx_sweep_stages != stages) G->solo.reset();
   G->mx_sweep_rows = rows;
   G->mx_sweep_stages = stages;
@@ -3450,7 +3480,7 @@ int cfdg_grid_set_sweep_tile(cfdg_grid* G, int32_t rows, int32_t stages) {
 int cfdg_grid_set_coarse_scale(cfdg_grid* G, double alpha) {
   if (int e = check_grid(G)) return e;
   if (!(alpha > 0.0 && alpha < 2.0)) return fail(CFDG_ERR_INVALID, "the coarse-correction scale must lie in (0, 2)");
-  std::lock_guard<std::mutex> lk(G->mu);
+  std::lock_guard<GridMutex> lk(G->mu);
   if (G->mx_alpha != (float)alpha) {
     G->mixed.reset();  // the case state holds the scaled prolongation
     G->solo.reset();
@@ -3462,7 +3492,7 @@ int cfdg_grid_set_coarse_scale(cfdg_grid* G, double alpha) {
 int cfdg_grid_set_coarse_layout(cfdg_grid* G, int32_t bins) {
   if (int e = check_grid(G)) return e;
   if (bins != 0 && bins != 1) return fail(CFDG_ERR_INVALID, "the coarse layout is 0 (aggregate order) or 1 (bin grid)");
-  std::lock_guard<std::mutex> lk(G->mu);
+  std::lock_guard<GridMutex> lk(G->mu);
   if (G->mx_bins != bins) {
     G->mixed.reset();  // the case state holds the first coarse level's numbering
     G->solo.reset();
@@ -3474,7 +3504,7 @@ int cfdg_grid_set_coarse_layout(cfdg_grid* G, int32_t bins) {
 int cfdg_project_device(cfdg_grid* G, double* d_u, double* d_p, double dt, double tol, uint64_t max_iter,
                         cfdg_poll_fn poll, void* poll_ctx, cfdg_info* info) {
   if (int e = check_grid(G)) return e;
-  std::lock_guard<std::mutex> lk(G->mu);
+  std::lock_guard<GridMutex> lk(G->mu);
   CU(cudaSetDevice(G->ctx->device));
   Poller P;
   P.fn = poll;
@@ -3486,7 +3516,7 @@ int cfdg_project(cfdg_grid* G, double* u, double* p, double dt, double tol, uint
                  void* poll_ctx, cfdg_info* info) {
   if (int e = check_grid(G)) return e;
   if (!u || !p) return fail(CFDG_ERR_INVALID, "null u or p");
-  std::lock_guard<std::mutex> lk(G->mu);
+  std::lock_guard<GridMutex> lk(G->mu);
   CU(cudaSetDevice(G->ctx->device));
   cudaStream_t s = G->stream;
   CU(cudaMemcpyAsync(G->u, u, G->h.faces * 8, cudaMemcpyHostToDevice, s));
@@ -3505,7 +3535,7 @@ int cfdg_solve_scaled(cfdg_grid* G, const double* b, const double* roundoff_scal
                       cfdg_poll_fn poll, void* poll_ctx, double* x, cfdg_info* info) {
   if (int e = check_grid(G)) return e;
   if (!b || !x) return fail(CFDG_ERR_INVALID, "null b or x");
-  std::lock_guard<std::mutex> lk(G->mu);
+  std::lock_guard<GridMutex> lk(G->mu);
   CU(cudaSetDevice(G->ctx->device));
   cudaStream_t s = G->stream;
   CU(cudaMemcpyAsync(G->b, b, G->h.cells * 8, cudaMemcpyHostToDevice, s));
@@ -3521,7 +3551,7 @@ int cfdg_solve_scaled(cfdg_grid* G, const double* b, const double* roundoff_scal
 
 int cfdg_apply(cfdg_grid* G, const double* x, double* y) {
   if (int e = check_grid(G)) return e;
-  std::lock_guard<std::mutex> lk(G->mu);
+  std::lock_guard<GridMutex> lk(G->mu);
   CU(cudaSetDevice(G->ctx->device));
   cudaStream_t s = G->stream;
   CU(cudaMemcpyAsync(G->p, x, G->h.cells * 8, cudaMemcpyHostToDevice, s));
@@ -3534,7 +3564,7 @@ int cfdg_apply(cfdg_grid* G, const double* x, double* y) {
 
 int cfdg_center_nullspaces(cfdg_grid* G, double* x) {
   if (int e = check_grid(G)) return e;
-  std::lock_guard<std::mutex> lk(G->mu);
+  std::lock_guard<GridMutex> lk(G->mu);
   CU(cudaSetDevice(G->ctx->device));
   cudaStream_t s = G->stream;
   CU(cudaMemcpyAsync(G->z, x, G->h.cells * 8, cudaMemcpyHostToDevice, s));
@@ -3556,7 +3586,7 @@ int cfdg_multigrid_stats_json(cfdg_grid* G, char* buf, size_t cap) {
 
 int cfdg_debug_precondition(cfdg_grid* G, const double* r, double* z) {
   if (int e = check_grid(G)) return e;
-  std::lock_guard<std::mutex> lk(G->mu);
+  std::lock_guard<GridMutex> lk(G->mu);
   CU(cudaSetDevice(G->ctx->device));
   Poller P;
   if (int e = prepare_preconditioner(G, P, nullptr)) return e;
@@ -3572,7 +3602,7 @@ int cfdg_debug_precondition(cfdg_grid* G, const double* r, double* z) {
 
 int cfdg_debug_wave_stall(cfdg_grid* G, int32_t hold_tile, int64_t spin_limit) {
   if (int e = check_grid(G)) return e;
-  std::lock_guard<std::mutex> lk(G->mu);
+  std::lock_guard<GridMutex> lk(G->mu);
   if (!G->structured) return fail(CFDG_ERR_UNSUPPORTED, "the grid has no wavefront sweeps (a periodic axis)");
   if (hold_tile < -1 || hold_tile >= G->tiles_j * G->tiles_k)
     return fail(CFDG_ERR_INVALID, "hold_tile must be -1 or a tile of the grid's wavefront");
@@ -3592,7 +3622,7 @@ int cfdg_residual_norm_noalloc(cfdg_grid* G, const double* d_x, const double* d_
     return fail(CFDG_ERR_INVALID, "cfdg_residual_norm_noalloc: the grid has " + std::to_string(N) +
                                       " cells; the no-allocation scratch covers at most " +
                                       std::to_string((int64_t)NOALLOC_MAX_BLOCKS * NOALLOC_CHUNK));
-  std::lock_guard<std::mutex> lk(G->mu);
+  std::lock_guard<GridMutex> lk(G->mu);
   CU(cudaSetDevice(G->ctx->device));
   double* scratch = nullptr;
   if (int e = noalloc_scratch(G->ctx->device, &scratch)) return e;
@@ -3609,7 +3639,7 @@ int cfdg_residual_norm_noalloc(cfdg_grid* G, const double* d_x, const double* d_
 
 int cfdg_grid_set_stream(cfdg_grid* G, void* stream) {
   if (int e = check_grid(G)) return e;
-  std::lock_guard<std::mutex> lk(G->mu);
+  std::lock_guard<GridMutex> lk(G->mu);
   CU(cudaSetDevice(G->ctx->device));
   CU(cudaStreamSynchronize(G->stream));
   G->stream = stream ? (cudaStream_t)stream : G->own;
@@ -3622,7 +3652,7 @@ int cfdg_debug_time_kernel(cfdg_grid* G, int32_t which, int32_t reps, double* ms
                            double* algorithmic_bytes) {
   if (int e = check_grid(G)) return e;
   if (reps < 1) return fail(CFDG_ERR_INVALID, "reps must be positive");
-  std::lock_guard<std::mutex> lk(G->mu);
+  std::lock_guard<GridMutex> lk(G->mu);
   CU(cudaSetDevice(G->ctx->device));
   Poller P;
   const double N = (double)G->h.cells;
@@ -3673,7 +3703,7 @@ int cfdg_debug_time_kernel(cfdg_grid* G, int32_t which, int32_t reps, double* ms
 
 int cfdg_debug_projection_rhs(cfdg_grid* G, const double* u, double dt, double* b, double* terms) {
   if (int e = check_grid(G)) return e;
-  std::lock_guard<std::mutex> lk(G->mu);
+  std::lock_guard<GridMutex> lk(G->mu);
   CU(cudaSetDevice(G->ctx->device));
   cudaStream_t s = G->stream;
   CU(cudaMemcpyAsync(G->u, u, G->h.faces * 8, cudaMemcpyHostToDevice, s));

@@ -2739,8 +2739,10 @@ int upload_plan(CaseState& K, cudaStream_t s, bool* now) {
   K.plan_ptrs = K.arena.ptrs.size();
   K.plan_bytes = K.arena.bytes;
   int e = 0;
+  K.arena.spare = true;
   for (int t = 0; t < K.cl.nb && !e; ++t) e = upload_types(K.arena, s, K.bins[K.cl.lc + 1 + t], K.cl.b[t]);
   for (int l = 0; l < K.up.n && !e; ++l) e = upload_types(K.arena, s, K.bins[l + 1], K.up.lv[l]);
+  K.arena.spare = false;
   if (K.up.n) K.up.lv[K.up.n] = K.cl.b[0];
   const cudaError_t c = cudaStreamSynchronize(s);
   if (!e && c != cudaSuccess) e = fail(CFDG_ERR_CUDA, cudaGetErrorString(c));
@@ -4118,8 +4120,10 @@ int cfdg_mixed_pack(cfdg_batch* B) {
     const size_t held = A.ptrs.size();
     const uint64_t held_bytes = A.bytes;
     std::vector<CaseState*> fresh;
+    A.spare = true;
     int e = choose_clusters(B, true, fresh, s);
-    if (e == CFDG_ERR_ADMISSION && B->any_cl) {
+    A.spare = false;
+    if (e == CFDG_ERR_ADMISSION) {
       A.rollback(held, held_bytes);
       for (CaseState* K : fresh) drop_plan(*K);
       e = choose_clusters(B, false, fresh, s);
@@ -4266,7 +4270,7 @@ std::vector<cfdg_grid*> lock_order(const std::vector<cfdg_grid*>& g) {
 }
 
 struct Locks {
-  std::vector<std::unique_lock<std::mutex>> held;
+  std::vector<std::unique_lock<GridMutex>> held;
   explicit Locks(const std::vector<cfdg_grid*>& grids) {
     for (auto* G : lock_order(grids)) held.emplace_back(G->mu);
   }
@@ -4442,7 +4446,7 @@ int cfdg_batch_create(cfdg_context* ctx, cfdg_grid* const* grids, int32_t n, cfd
         cfdg_mixed_delete(B);
         return fail(CFDG_ERR_INVALID, "a grid can appear once in a batch");
       }
-    std::lock_guard<std::mutex> lk(G->mu);
+    std::lock_guard<GridMutex> lk(G->mu);
     if (int e = prepare_multigrid(G)) {
       cfdg_mixed_delete(B);
       return e;

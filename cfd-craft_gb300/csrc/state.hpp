@@ -9,6 +9,7 @@
 #include <cstring>
 #include <memory>
 #include <mutex>
+#include <thread>
 #include <string>
 #include <vector>
 
@@ -52,19 +53,49 @@ struct cfdg_context {
   std::mutex mu;
   int grids = 0;
   bool destroyed = false;
+  std::vector<cfdg_grid*> open;  // guarded by mu
 };
 
 namespace cfdg {
 
-// Device allocation owned by a grid, counted against the context's budget.
+// A grid's lock. It knows its owner, so that a thread may try any grid's.
+class GridMutex {
+ public:
+  void lock() {
+    m_.lock();
+    owner_ = std::this_thread::get_id();
+  }
+  bool try_lock() {
+    if (owner_ == std::this_thread::get_id() || !m_.try_lock()) return false;
+    owner_ = std::this_thread::get_id();
+    return true;
+  }
+  void unlock() {
+    owner_ = std::thread::id();
+    m_.unlock();
+  }
+
+ private:
+  std::mutex m_;
+  std::atomic<std::thread::id> owner_{std::thread::id()};
+};
+
+// Makes room for `bytes` in the context's budget: gives back what the plain cycle's sweeps of grids
+// that no call is using hold (ensure_sweeps builds it again, for the fewest bytes where it has to).
+bool release_sweeps(cfdg_context* ctx, uint64_t bytes);
+
+// Device allocation owned by a grid, counted against the context's budget. spare: what is allocated
+// can be done without, so nothing is released for it.
 struct Arena {
   cfdg_context* ctx = nullptr;
+  bool spare = false;
   std::vector<void*> ptrs;
   uint64_t bytes = 0;
   template <class T>
   int alloc(T** p, size_t n) {
     size_t b = std::max<size_t>(n, 1) * sizeof(T);
-    if (ctx->used.load() + b > ctx->budget) return fail(CFDG_ERR_ADMISSION, "the grid does not fit the context's HBM budget");
+    if (ctx->used.load() + b > ctx->budget && (spare || !release_sweeps(ctx, b)))
+      return fail(CFDG_ERR_ADMISSION, "the grid does not fit the context's HBM budget");
     CU(cudaMalloc((void**)p, b));
     ptrs.push_back(*p);
     bytes += b;
@@ -236,7 +267,7 @@ using namespace cfdg;
 
 struct cfdg_grid {
   cfdg_context* ctx = nullptr;
-  std::mutex mu;        // serialises solves on this grid
+  cfdg::GridMutex mu;   // serialises solves on this grid
   std::mutex stats_mu;  // guards the stats copy (readable from a poll callback)
   std::string stats_json;
   HostGrid h;

@@ -155,3 +155,43 @@ def test_mixed_form_without_its_plans(pkg):
         seen.add(kernel)
         hi = mid
     assert seen == {"cluster", "cooperative"}
+
+
+@pytest.mark.parametrize("form", ["plain", "lines", "mixed beside plain"])
+def test_several_grids_within_the_bytes(pkg, form):
+    """Three grids in a context of three times the bytes of one: what an earlier grid holds beyond them
+    gives way to a later one, whichever is used, and in turns."""
+    if form == "lines":
+        cells, size, boundaries, held = THIN["long lines"]
+        case = pkg.synth.case(cells, 1.0, boundaries=boundaries, inflow=1.0, preconditioner="multigrid")
+        case["domain"]["size_m"] = list(size)
+        total = 3 * held
+    else:
+        case = iso(pkg, n=(60, 44, 24))
+        total = 3 * PLAIN["open"][2]
+    if form == "mixed beside plain":
+        total = 2 * PLAIN["open"][2] + MIXED["no solid cell"][1]
+    g = pkg.grid.Grid.build(case)
+    rs = [np.random.default_rng(s).uniform(-1.0, 1.0, g.count) for s in range(3)]
+    u = pkg.synth.random_velocity(g, 70)
+    out = []
+    for budget in (1 << 36, total):
+        ctx = pkg.pressure.Context(0, hbm_budget_bytes=budget)
+        dgs, got = [], []
+        for i in range(3):
+            mixed_one = form == "mixed beside plain" and i == 2
+            dgs.append(pkg.pressure.DeviceGrid(g, ctx=ctx, preconditioner="multigrid",
+                                               precision="mixed" if mixed_one else "plain"))
+            if mixed_one:
+                uu, pp = u.copy(), np.zeros(g.count)
+                dgs[i].project(uu, pp, 0.1, 1e-8, 1000)
+                got += [uu, pp]
+            else:
+                got.append(dgs[i].precondition(rs[i]))
+        for _ in range(2):
+            got += [d.precondition(r) for d, r in list(zip(dgs, rs))[:2]]
+        for d in dgs:
+            d.close()
+        ctx.close()
+        out.append([bits(a) for a in got])
+    assert all(np.array_equal(a, b) for a, b in zip(*out))
